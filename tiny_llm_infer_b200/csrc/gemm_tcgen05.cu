@@ -187,24 +187,11 @@ __device__ __forceinline__ void store_row32(bf16* row_ptr, int col0, int cols, c
 // owns 256 rows, both accumulators belong to one tile, every slab of W fetched from L2 feeds
 // twice as many MMAs (32 KB of shared-memory fill per 128 x 256 x 64 instead of 48 KB), three
 // stages of 64 KB; the epilogue is not overlapped.
-// Grouped form (a mixture of experts): x holds the rows of every expert one after the other, w the
-// experts' matrices stacked ([experts * w_rows, K]), and a row tile is an entry of device-side lists made
-// by the step's plan: its expert and its first row, wherever that falls; rows at and past the expert's
-// last (`offsets[expert + 1]`) are computed along and not written.  How many entries there are is read
-// from the device too (`n_tiles`); `tile_row0 == nullptr` means the plain form.
-struct GroupedTiles {
-    const int* tile_expert;
-    const int* tile_row0;
-    const int* n_tiles;
-    const int* offsets;
-    int w_rows;
-};
-
 template <bool SWIGLU, int MT, int ACT>
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                     bf16* __restrict__ y, int M, int N, int K, int half_n, int interleaved, int tiles_m,
-                    int tiles_n, int* __restrict__ error_word, const GroupedTiles grouped, const GateConst gc) {
+                    int tiles_n, int* __restrict__ error_word, const GateConst gc) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[4], empty_bar[4], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_slot;
@@ -219,7 +206,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     unsigned char* stage_out = tiles + (size_t)kStages * kStageBytes + (size_t)(warp & 3) * 32 * kOutRowBytes;
     const int k_blocks = (K + kBK - 1) / kBK;
-    if (grouped.tile_row0 != nullptr) tiles_m = *grouped.n_tiles;
     const int total_tiles = tiles_m * tiles_n;
     const int out_cols = SWIGLU ? half_n : N;
     constexpr int kColTile = SWIGLU ? 128 : kBN;
@@ -255,11 +241,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             int it = 0;                               // k-blocks issued so far, over all tiles
             for (int t = blockIdx.x; t < total_tiles && !*aborted; t += gridDim.x) {
                 const int tile_m = t % tiles_m, tile_n = t / tiles_m;
-                int a_row = tile_m * kRows, w_row = 0;
-                if (grouped.tile_row0 != nullptr) {
-                    a_row = grouped.tile_row0[tile_m];
-                    w_row = grouped.tile_expert[tile_m] * grouped.w_rows;
-                }
+                const int a_row = tile_m * kRows;
                 for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % kStages;
                     if (it >= kStages && !mbar_wait(&empty_bar[s], ((it / kStages) - 1) & 1)) {
@@ -272,11 +254,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                     mbar_expect_tx(&full_bar[s], kStageBytes);
                     tma_load_2d(a_dst, &map_x, kb * kBK, a_row, &full_bar[s]);
                     if (SWIGLU && !interleaved) {
-                        tma_load_2d(b_dst, &map_w, kb * kBK, w_row + tile_n * 128, &full_bar[s]);
-                        tma_load_2d(b_dst + kStageBBytes / 2, &map_w, kb * kBK, w_row + half_n + tile_n * 128, &full_bar[s]);
+                        tma_load_2d(b_dst, &map_w, kb * kBK, tile_n * 128, &full_bar[s]);
+                        tma_load_2d(b_dst + kStageBBytes / 2, &map_w, kb * kBK, half_n + tile_n * 128, &full_bar[s]);
                     } else {
-                        tma_load_2d(b_dst, &map_w, kb * kBK, w_row + tile_n * kBN, &full_bar[s]);
-                        tma_load_2d(b_dst + kStageBBytes / 2, &map_w, kb * kBK, w_row + tile_n * kBN + 128, &full_bar[s]);
+                        tma_load_2d(b_dst, &map_w, kb * kBK, tile_n * kBN, &full_bar[s]);
+                        tma_load_2d(b_dst + kStageBBytes / 2, &map_w, kb * kBK, tile_n * kBN + 128, &full_bar[s]);
                     }
                 }
             }
@@ -331,11 +313,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         for (int t = blockIdx.x; t < total_tiles; t += gridDim.x, ++local) {
             const int buf = local % kNumBuf;
             const int tile_m = t % tiles_m, tile_n = t / tiles_m;
-            int row_base = tile_m * kRows, row_end = M;
-            if (grouped.tile_row0 != nullptr) {
-                row_base = grouped.tile_row0[tile_m];
-                row_end = grouped.offsets[grouped.tile_expert[tile_m] + 1];
-            }
+            const int row_base = tile_m * kRows;
             const bool ready = mbar_wait(&acc_full[buf], (local / kNumBuf) & 1);
             if (!ready) {
                 if (lane == 0) atomicExch(error_word, 3);
@@ -400,7 +378,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                     for (int j = 0; j < 8; ++j) {
                         const int piece = lane + 32 * j, r = piece >> 3, p16 = piece & 7;
                         const int row = row0 + r, col = col0 + p16 * 8;
-                        if (row < row_end && col < out_cols) {
+                        if (row < M && col < out_cols) {
                             const uint4 val = *reinterpret_cast<const uint4*>(stage_out + r * kOutRowBytes + p16 * 16);
                             bf16* dst = y + (size_t)row * out_cols + col;
                             if (col + 8 <= out_cols && (out_cols % 8) == 0) {
@@ -426,6 +404,222 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols)
                      : "memory");
     }
+}
+
+// ---------------------------------------------------------------- the experts of a mixture
+// y[r] = x[r] . W_e^T for the rows r of every expert e, x the plan's rows one after the other, w the experts' matrices
+// stacked ([experts * w_rows, K]).  The weights are the MMA's A operand (128 weight rows: the M of the instruction) and an
+// expert's rows its B operand, so the instruction's N follows the expert's rows in steps of sixteen: an accumulator is
+// [128 weight rows x n rows], a tile of few rows costs little, and every weight comes from HBM once as long as its expert
+// has no more rows than a tile of the plan.
+//
+// What bounds it: with few rows per expert the weights' way from HBM (64 experts of 2048 x 4096, gate|up + down: 138 + 69 us
+// for 8 tokens that reach 25 experts, 6.0 TB/s; 330 + 165 us for 256 tokens, 6.5 TB/s), with many what the blocks fetch
+// from L2 (425 + 224 us for 8192 rows, 0.97 PFLOP/s).  Two weight slabs per block halve the fetches of the rows: 441 instead of
+// 530 us with 8192 rows, 140 instead of 155 with 32.  Tiles of 256 rows leave no second accumulator beside the first (450 us),
+// boxes of 16 and 32 rows instead of 64 cost the copy engine more than they save (567, 501 us).  Issued from a branch for
+// one lane, the MMAs of a stage took longer than HBM takes to deliver it (180 instead of 155 us with 32 rows).
+// The form with the rows as A operand, padded to 128 per tile, took 465 + 233 us for 8192 rows; few rows ran on
+// mma.sync tiles (336 + 162 us for 8 tokens), and on mma.sync fragments straight from HBM they take 146 + 95 us.
+//
+// Warps as in the dense kernel: one producer thread, one MMA warp, four epilogue warps.  An epilogue thread owns one
+// weight row (an output column) and reads sixteen rows' sums at a time; for gated units, whose gate and up rows are
+// interleaved by eight, the lanes eight apart exchange sums, each then making the outputs of every second row.
+struct MoeTiles {
+    const int *tile_expert, *tile_row0, *n_tiles, *offsets;
+};
+constexpr int kMoeStages = 9, kMoeBoxRows = 64;
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+// The MMA warp runs its loop whole: the descriptors are made by all its lanes (in uniform registers) and one lane issues.
+__device__ __forceinline__ void umma_bf16_if(uint32_t issue, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(issue)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_if(uint32_t issue, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(cvta_shared(bar)),
+        "r"(issue)
+        : "memory");
+}
+
+// SLABS: weight tiles of 128 rows per block.  MODE 0: the product, as TOut.  1: act(gate) * up.  2: act(product).
+// ACT: a GateAct code.
+template <int SLABS, int MODE, int ACT, typename TOut>
+__global__ void __launch_bounds__(kGemmThreads)
+moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, TOut* __restrict__ y,
+                   int w_rows, int K, int tiles_n, int tile_rows, int stages, int* __restrict__ error_word,
+                   const MoeTiles lists, const GateConst gc) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t full_bar[kMoeStages], empty_bar[kMoeStages], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+    unsigned char* tiles = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    constexpr int kSlab = kBM * kBK * 2, kABytes = SLABS * kSlab;
+    const int stage_bytes = kABytes + tile_rows * kBK * 2;
+    constexpr int kAccCols = 128, kAccTile = SLABS * kAccCols;       // of tensor memory; two tiles' accumulators take turns
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int k_blocks = (K + kBK - 1) / kBK;
+    const int total = *lists.n_tiles * tiles_n;             // an expert's weight tiles one after the other
+    const int out_cols = MODE == 1 ? w_rows / 2 : w_rows;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kMoeStages; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 4);
+        }
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(cvta_shared(&tmem_base_slot)),
+                     "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem_base = tmem_base_slot;
+    volatile int* aborted = &abort_flag;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0, issued = 0;
+            uint32_t phase = 1;                              // of empty_bar: the first round of the ring waits for nothing
+            for (int t = blockIdx.x; t < total && !*aborted; t += gridDim.x) {
+                const int tile = t / tiles_n, e = lists.tile_expert[tile], row0 = lists.tile_row0[tile];
+                const int rows = min(tile_rows, lists.offsets[e + 1] - row0), boxes = (rows + kMoeBoxRows - 1) / kMoeBoxRows;
+                const int w_row = e * w_rows + (t - tile * tiles_n) * SLABS * kBM;
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (issued >= stages && !mbar_wait(&empty_bar[s], phase)) {
+                        atomicExch(error_word, 1);
+                        *aborted = 1;
+                    }
+                    if (*aborted) break;
+                    unsigned char* a_dst = tiles + (size_t)s * stage_bytes;
+                    mbar_expect_tx(&full_bar[s], kABytes + boxes * kMoeBoxRows * kBK * 2);
+                    tma_load_2d(a_dst, &map_w, kb * kBK, w_row, &full_bar[s]);
+                    for (int b = 0; b < boxes; ++b)
+                        tma_load_2d(a_dst + kABytes + b * kMoeBoxRows * kBK * 2, &map_x, kb * kBK, row0 + b * kMoeBoxRows, &full_bar[s]);
+                    ++issued;
+                    if (++s == stages) { s = 0; phase ^= 1; }
+                }
+            }
+            // on an abort: do not leave the block while copies into its shared memory are in flight
+            if (*aborted) {
+                const int first = issued > stages ? issued - stages : 0;
+                for (int i = first; i < issued; ++i) mbar_wait(&full_bar[i % stages], (i / stages) & 1);
+            }
+        }
+    } else if (warp == 1) {
+        const uint32_t issue = lane == 0;
+        const uint64_t desc0 = smem_desc_sw128(cvta_shared(tiles));     // a stage and a step inside it only add to its address
+        int s = 0, local = 0;
+        uint32_t phase = 0;
+        for (int t = blockIdx.x; t < total && !*aborted; t += gridDim.x, ++local) {
+            const int tile = t / tiles_n;
+            const int rows = min(tile_rows, lists.offsets[lists.tile_expert[tile] + 1] - lists.tile_row0[tile]);
+            const uint32_t idesc = instr_desc_bf16(kBM, (rows + 15) & ~15);
+            const int buf = local & 1;
+            if (local >= 2 && !mbar_wait(&acc_empty[buf], ((local >> 1) - 1) & 1)) {
+                if (issue) atomicExch(error_word, 4);
+                *aborted = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t tmem_acc = tmem_base + buf * kAccTile;
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!mbar_wait(&full_bar[s], phase)) {
+                    if (issue) atomicExch(error_word, 2);
+                    *aborted = 1;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const uint64_t a_desc = desc0 + (uint32_t)(s * stage_bytes >> 4), b_desc = a_desc + (kABytes >> 4);
+#pragma unroll
+                for (int k = 0; k < kBK / 16; ++k)
+#pragma unroll
+                    for (int m = 0; m < SLABS; ++m)
+                        umma_bf16_if(issue, tmem_acc + m * kAccCols, a_desc + (m * kSlab + k * 32) / 16, b_desc + k * 2, idesc,
+                                     (kb > 0 || k > 0) ? 1u : 0u);
+                umma_commit_if(issue, &empty_bar[s]);
+                if (++s == stages) { s = 0; phase ^= 1; }
+            }
+            umma_commit_if(issue, &acc_full[buf]);
+        }
+    } else {
+        const int quad = warp & 3;
+        int local = 0;
+        for (int t = blockIdx.x; t < total; t += gridDim.x, ++local) {
+            const int tile = t / tiles_n, row0 = lists.tile_row0[tile];
+            const int rows = min(tile_rows, lists.offsets[lists.tile_expert[tile] + 1] - row0);
+            const int buf = local & 1;
+            if (!mbar_wait(&acc_full[buf], (local >> 1) & 1)) {
+                if (lane == 0) atomicExch(error_word, 3);
+                *aborted = 1;
+            }
+            if (*aborted) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll 1
+            for (int m = 0; m < SLABS; ++m) {
+                const int w0 = ((t - tile * tiles_n) * SLABS + m) * kBM + quad * 32;       // first weight row of this warp
+                const uint32_t lane_addr = tmem_base + buf * kAccTile + m * kAccCols + ((uint32_t)(quad * 32) << 16);
+                const int col = MODE == 1 ? w0 / 2 + (lane >> 4) * 8 + (lane & 7) : w0 + lane;
+                const bool is_up = MODE == 1 && (lane & 8);
+#pragma unroll 1
+                for (int c = 0; c < rows; c += 16) {
+                    uint32_t r[16];
+                    tmem_ld16(lane_addr + c, r);
+                    tmem_ld_wait();
+                    TOut* dst = y + (size_t)(row0 + c) * out_cols + col;
+                    if (MODE == 1) {
+#pragma unroll
+                        for (int i = 0; i < 16; i += 2) {
+                            const float mine = __uint_as_float(is_up ? r[i + 1] : r[i]);
+                            const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(is_up ? r[i] : r[i + 1]), 8);
+                            const float v = gated_unit(is_up ? other : mine, is_up ? mine : other, ACT, gc);
+                            const int row = i + (is_up ? 1 : 0);
+                            if (c + row < rows && col < out_cols) dst[(size_t)row * out_cols] = from_f32<TOut>(v);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float v = MODE == 2 ? gate_act(__uint_as_float(r[i]), ACT) : __uint_as_float(r[i]);
+                            if (c + i < rows && col < out_cols) dst[(size_t)i * out_cols] = from_f32<TOut>(v);
+                        }
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
 }
 
 // ---------------------------------------------------------------------------------- host side
@@ -471,9 +665,7 @@ static int sm_count() {
 
 template <bool SWIGLU, int MT, int ACT = (SWIGLU ? (int)kActSilu : kActNone)>
 static int launch_tcgen05(const CUtensorMap& mx, const CUtensorMap& mw, void* y, int M, int N, int K, int half_n,
-                          int interleaved, int* error_word, cudaStream_t stream,
-                          const GroupedTiles grouped = GroupedTiles{nullptr, nullptr, nullptr, nullptr, 0},
-                          int grouped_max_tiles = 0, const GateConst gc = GateConst{0.0f, 0.0f}) {
+                          int interleaved, int* error_word, cudaStream_t stream, const GateConst gc = GateConst{0.0f, 0.0f}) {
     const size_t smem = (size_t)(MT == 1 ? 4 : 3) * (kBM * MT * kBK * 2 + kStageBBytes) + 1024 + 4 * 32 * (64 * 2 + 16);
     static OncePerDevice configured;
     if (configured.first()) {
@@ -485,12 +677,33 @@ static int launch_tcgen05(const CUtensorMap& mx, const CUtensorMap& mw, void* y,
     const int out_cols = SWIGLU ? half_n : N;
     const int col_tile = SWIGLU ? 128 : kBN;
     const int tiles_n = (out_cols + col_tile - 1) / col_tile;
-    const int tiles_m = grouped.tile_row0 != nullptr ? grouped_max_tiles : (M + kBM * MT - 1) / (kBM * MT);
+    const int tiles_m = (M + kBM * MT - 1) / (kBM * MT);
     const int total = tiles_m * tiles_n;
     const int grid = total < sm_count() ? total : sm_count();
     gemm_tcgen05_kernel<SWIGLU, MT, ACT><<<grid, kGemmThreads, smem, stream>>>(mx, mw, (bf16*)y, M, N, K, half_n, interleaved,
-                                                                      tiles_m, tiles_n, error_word, grouped, gc);
+                                                                      tiles_m, tiles_n, error_word, gc);
     return finish_launch("gemm_tcgen05");
+}
+
+template <int SLABS, int MODE, int ACT, typename TOut>
+static int launch_moe_tcgen05(const CUtensorMap& mx, const CUtensorMap& mw, void* y, int w_rows, int K, int tile_rows,
+                              int max_tiles, const MoeTiles& lists, GateConst gc, int* error_word, cudaStream_t stream) {
+    constexpr size_t kMost = 226 * 1024 - 512;              // of 227 KB; the barriers and the alignment of the ring take the rest
+    const size_t stage = (size_t)(SLABS * kBM + tile_rows) * kBK * 2;
+    int stages = (int)((kMost - 1024) / stage);
+    if (stages > kMoeStages) stages = kMoeStages;
+    static OncePerDevice configured;
+    if (configured.first()) {
+        cudaError_t e = cudaFuncSetAttribute(moe_tcgen05_kernel<SLABS, MODE, ACT, TOut>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost);
+        if (e != cudaSuccess) { set_error("moe_tcgen05: %s", cudaGetErrorString(e)); return (int)e; }
+        configured.done();
+    }
+    const int tiles_n = (w_rows + SLABS * kBM - 1) / (SLABS * kBM);
+    const long long most = (long long)max_tiles * tiles_n;
+    const int grid = most < sm_count() ? (int)most : sm_count();
+    moe_tcgen05_kernel<SLABS, MODE, ACT, TOut><<<grid, kGemmThreads, stages * stage + 1024, stream>>>(
+        mx, mw, (TOut*)y, w_rows, K, tiles_n, tile_rows, stages, error_word, lists, gc);
+    return finish_launch("moe_tcgen05");
 }
 
 }  // namespace tllm
@@ -534,9 +747,8 @@ extern "C" int tllm_gemm_tcgen05(const void* x, const void* w, void* y, int M, i
     TLLM_REQUIRE(gated_act_ok(act, limit), "gemm_tcgen05: unknown activation %d", act);
     if ((swiglu & 1) && act == kActClampedSwish) {
         const GateConst gc{limit, slope};
-        const GroupedTiles plain{nullptr, nullptr, nullptr, nullptr, 0};
-        return tall ? launch_tcgen05<true, 2, kActClampedSwish>(mx, mw, y, M, N, K, N / 2, interleaved, error_word, stream, plain, 0, gc)
-                    : launch_tcgen05<true, 1, kActClampedSwish>(mx, mw, y, M, N, K, N / 2, interleaved, error_word, stream, plain, 0, gc);
+        return tall ? launch_tcgen05<true, 2, kActClampedSwish>(mx, mw, y, M, N, K, N / 2, interleaved, error_word, stream, gc)
+                    : launch_tcgen05<true, 1, kActClampedSwish>(mx, mw, y, M, N, K, N / 2, interleaved, error_word, stream, gc);
     }
     if ((swiglu & 1) && act == kActRelu)
         return tall ? launch_tcgen05<true, 2, kActRelu>(mx, mw, y, M, N, K, N / 2, interleaved, error_word, stream)
@@ -551,45 +763,51 @@ extern "C" int tllm_gemm_tcgen05(const void* x, const void* w, void* y, int M, i
                 : launch_tcgen05<false, 1>(mx, mw, y, M, N, K, 0, 0, error_word, stream);
 }
 
-// The grouped form: x [rows, K] holds the experts' rows one after the other, w is [experts][n][K], and
-// the row tiles of 128 are the plan's lists (device memory; at most max_tiles entries).  flags as in
-// tllm_gemm_tcgen05 (bit 1 with bit 4: gate and up rows interleaved by eight, y is [rows, n / 2]).
-extern "C" int tllm_gemm_tcgen05_grouped(const void* x, const void* w, void* y, int rows, int n, int K, int experts,
-                                         int flags, const int* tile_expert, const int* tile_row0, const int* n_tiles,
-                                         const int* offsets, int max_tiles, float limit, float slope, int* error_word,
-                                         cudaStream_t stream) {
-    TLLM_REQUIRE(rows > 0 && n > 0 && K > 0 && experts > 0 && max_tiles > 0, "gemm_tcgen05_grouped: bad sizes");
-    TLLM_REQUIRE(K % 8 == 0, "gemm_tcgen05_grouped: K = %d is no multiple of 8", K);
+// The experts' products: x [rows, K] holds the experts' rows one after the other, w is [experts][n][K], and the plan's
+// lists (device memory; at most max_tiles entries) cut every expert's rows into tiles of at most tile_rows (64 or 128).  flags: 1 gated (with 4: gate and up rows interleaved by eight, y is [rows, n / 2] bfloat16); 16 an activation on
+// every output (y bfloat16); else the plain product, bfloat16 or with 32 float32.  Bits 8 and up: the activation
+// (GateAct).
+extern "C" int tllm_moe_tcgen05(const void* x, const void* w, void* y, int rows, int n, int K, int experts, int flags, int tile_rows,
+                                const int* tile_expert, const int* tile_row0, const int* n_tiles, const int* offsets, int max_tiles,
+                                float limit, float slope, int* error_word, cudaStream_t stream) {
+    TLLM_REQUIRE(rows > 0 && n > 0 && K > 0 && experts > 0 && max_tiles > 0, "moe_tcgen05: bad sizes");
+    TLLM_REQUIRE((long long)experts * n <= 0x7fffffff - 2 * kBM, "moe_tcgen05: %d experts of %d weight rows", experts, n);
+    TLLM_REQUIRE(K % 8 == 0, "moe_tcgen05: K = %d is no multiple of 8", K);
+    TLLM_REQUIRE(tile_rows == 64 || tile_rows == 128, "moe_tcgen05: tiles of %d rows", tile_rows);
     const bool gated = flags & 1;
-    TLLM_REQUIRE(!gated || ((flags & 4) && n % 16 == 0), "gemm_tcgen05_grouped: gate and up rows interleaved by eight, n = %d", n);
-    TLLM_REQUIRE((gated ? n / 2 : n) % 8 == 0, "gemm_tcgen05_grouped: rows of y must be whole 16-byte pieces");
+    // One weight slab per block while that still gives every multiprocessor at most one block (4 rows of 64 experts:
+    // 36 + 17 us instead of 40 + 19; 8 rows, 59 + 30 instead of 57 + 29, already take two).
+    const int reached = rows < experts ? rows : experts;
+    const bool two = (long long)reached * ((n + kBM - 1) / kBM) > sm_count();
+    TLLM_REQUIRE(!gated || ((flags & 4) && n % 16 == 0), "moe_tcgen05: gate and up rows interleaved by eight, n = %d", n);
+    TLLM_REQUIRE((long long)max_tiles * ((n + kBM - 1) / kBM) <= 0x7fffffff, "moe_tcgen05: too many tiles");
     TLLM_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0,
-                 "gemm_tcgen05_grouped: operands must be 16-byte aligned");
-    TLLM_REQUIRE(error_word && tile_expert && tile_row0 && n_tiles && offsets, "gemm_tcgen05_grouped: missing list");
+                 "moe_tcgen05: operands must be 16-byte aligned");
+    TLLM_REQUIRE(error_word && tile_expert && tile_row0 && n_tiles && offsets, "moe_tcgen05: missing list");
     CUtensorMap mx, mw;
-    TLLM_REQUIRE(make_map(&mx, x, rows, K, kBM) && make_map(&mw, w, (long long)experts * n, K, 128),
-                 "gemm_tcgen05_grouped: cuTensorMapEncodeTiled failed or is not available");
-    const GroupedTiles grouped{tile_expert, tile_row0, n_tiles, offsets, n};
+    TLLM_REQUIRE(make_map(&mx, x, rows, K, kMoeBoxRows) && make_map(&mw, w, (long long)experts * n, K, two ? 2 * kBM : kBM),
+                 "moe_tcgen05: cuTensorMapEncodeTiled failed or is not available");
+    const MoeTiles lists{tile_expert, tile_row0, n_tiles, offsets};
+    const GateConst gc{limit, slope};
     const int act = flags >> 8;
-    if (flags & 16) {                                       // a plain product with an activation on every output
-        TLLM_REQUIRE(!gated, "gemm_tcgen05_grouped: either a gated or a plain activation");
-#define UNARY(A) launch_tcgen05<false, 1, A>(mx, mw, y, rows, n, K, 0, 0, error_word, stream, grouped, max_tiles)
-        if (act == kActRelu2) return UNARY(kActRelu2);
-        if (act == kActTanh) return UNARY(kActTanh);
-        if (act == kActSilu) return UNARY(kActSilu);
-        if (act == kActGeluTanh) return UNARY(kActGeluTanh);
-        if (act == kActGeluErf) return UNARY(kActGeluErf);
-#undef UNARY
-        TLLM_REQUIRE(false, "gemm_tcgen05_grouped: unknown activation %d", act);
+#define MOE(M, A, T)                                                                                                            \
+    return two ? launch_moe_tcgen05<2, M, A, T>(mx, mw, y, n, K, tile_rows, max_tiles, lists, gc, error_word, stream)  \
+               : launch_moe_tcgen05<1, M, A, T>(mx, mw, y, n, K, tile_rows, max_tiles, lists, gc, error_word, stream)
+    if (flags & 16) {
+        TLLM_REQUIRE(!gated, "moe_tcgen05: either a gated or a plain activation");
+        if (act == kActRelu2) MOE(2, kActRelu2, bf16);
+        if (act == kActTanh) MOE(2, kActTanh, bf16);
+        if (act == kActSilu) MOE(2, kActSilu, bf16);
+        if (act == kActGeluTanh) MOE(2, kActGeluTanh, bf16);
+        if (act == kActGeluErf) MOE(2, kActGeluErf, bf16);
+        TLLM_REQUIRE(false, "moe_tcgen05: unknown activation %d", act);
     }
-    TLLM_REQUIRE(gated_act_ok(act, limit), "gemm_tcgen05_grouped: unknown activation %d", act);
-    if (gated && act == kActClampedSwish)
-        return launch_tcgen05<true, 1, kActClampedSwish>(mx, mw, y, rows, n, K, n / 2, 1, error_word, stream, grouped, max_tiles,
-                                                         GateConst{limit, slope});
-    if (gated && act == kActRelu)
-        return launch_tcgen05<true, 1, kActRelu>(mx, mw, y, rows, n, K, n / 2, 1, error_word, stream, grouped, max_tiles);
-    if (gated && act == kActGeluTanh)
-        return launch_tcgen05<true, 1, kActGeluTanh>(mx, mw, y, rows, n, K, n / 2, 1, error_word, stream, grouped, max_tiles);
-    if (gated) return launch_tcgen05<true, 1>(mx, mw, y, rows, n, K, n / 2, 1, error_word, stream, grouped, max_tiles);
-    return launch_tcgen05<false, 1>(mx, mw, y, rows, n, K, 0, 0, error_word, stream, grouped, max_tiles);
+    TLLM_REQUIRE(!gated || gated_act_ok(act, limit), "moe_tcgen05: unknown activation %d", act);
+    if (gated && act == kActClampedSwish) MOE(1, kActClampedSwish, bf16);
+    if (gated && act == kActRelu) MOE(1, kActRelu, bf16);
+    if (gated && act == kActGeluTanh) MOE(1, kActGeluTanh, bf16);
+    if (gated) MOE(1, kActSilu, bf16);
+    if (flags & 32) MOE(0, kActSilu, float);
+    MOE(0, kActSilu, bf16);
+#undef MOE
 }

@@ -103,7 +103,7 @@ def _declare(h) -> None:
         "tllm_ssd_prepare": [vp, i32, i32, vp, vp, vp, i32, vp, vp, vp, vp, i64, i64, i32, i32, i32, i32, vp, vp, vp,
                              vp, vp, i32, vp],
         "tllm_ssd_finish": [vp, vp, vp, i32, vp, i32, i32, vp, f32, i32, vp, i32, i32, i32, i32, vp, i64, i64, vp, vp],
-        "tllm_gemm_tcgen05_grouped": [vp, vp, vp, i32, i32, i32, i32, i32, vp, vp, vp, vp, i32, f32, f32, vp, vp],
+        "tllm_moe_tcgen05": [vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, vp, vp, i32, f32, f32, vp, vp],
         "tllm_add_rmsnorm": [vp, vp, vp, i32, f32, vp, i32, vp, i32, i32, vp],
         "tllm_swiglu": [vp, vp, i32, i32, i32, i32, i32, f32, f32, vp],
         "tllm_cast": [vp, i32, vp, i32, i64, vp],
@@ -1317,13 +1317,16 @@ def moe_route_grouped(z: torch.Tensor, top: int, scores: str = "softmax", correc
 class MoePlan:
     """Device-side lists that sort a step's (token, choice) assignments by expert, with the rows cut
     into tiles of ``tile_rows`` per expert.  ``real``: experts that have matrices; assignments to later ones
-    (identity experts) get rows and no tiles."""
+    (identity experts) get rows and no tiles.  ``tensor_memory``: the products over this plan take the tcgen05 kernel
+    (None: tiles of 128 rows say so)."""
 
-    def __init__(self, ids: torch.Tensor, experts: int, tile_rows: Optional[int] = None, real: Optional[int] = None):
+    def __init__(self, ids: torch.Tensor, experts: int, tile_rows: Optional[int] = None, real: Optional[int] = None,
+                 tensor_memory: Optional[bool] = None):
         n = ids.numel()
         self.n, self.experts = n, experts
         self.real = experts if real is None else int(real)
         self.tile_rows = tile_rows or moe_tile_rows()
+        self.tensor_memory = self.tile_rows == MOE_TCGEN05_TILE if tensor_memory is None else bool(tensor_memory)
         self.max_tiles = n // self.tile_rows + experts
         ints = torch.empty(experts + 2 + 3 * n + 2 * self.max_tiles, dtype=torch.int32, device=ids.device)
         at = 0
@@ -1341,15 +1344,27 @@ class MoePlan:
                                    _p(self.tile_row0), _stream()), "moe_plan")
 
 
-MOE_TCGEN05_ROWS = 1024     # from this many (token, choice) rows on the experts' products run on tcgen05
+MOE_TCGEN05_ROWS = 1        # from this many (token, choice) rows on the experts' products run on tcgen05
 MOE_TCGEN05_TILE = 128
+MOE_NARROW_ROWS = 1024      # from this many rows on (and 32 per expert) their results are kept in the storage type
 
 
 def moe_tcgen05_pays(rows: int, experts: int, n: int, k: int, dtype) -> bool:
-    """Whether the experts' products of a step take the grouped tcgen05 kernel: bfloat16, whole 16-byte
-    pieces, and enough rows that an expert's tile of 128 is on average at least a quarter full."""
-    return (dtype == torch.bfloat16 and rows >= MOE_TCGEN05_ROWS and rows >= 32 * experts
-            and k % 8 == 0 and n % 8 == 0)
+    """Whether the experts' products of a step take the tcgen05 kernel: bfloat16 and whole 16-byte pieces."""
+    return dtype == torch.bfloat16 and rows >= MOE_TCGEN05_ROWS and k % 8 == 0 and n % 8 == 0
+
+
+def moe_row_box(rows: int, experts: int) -> int:
+    """Rows per tile of a plan for the tcgen05 kernel.  Tiles of 64 leave room for more stages, tiles of 128 read an expert's
+    weights once where it has more than 64 rows: with 64 experts of 2048 x 4096 (gate|up + down) 16 rows per expert take 329 + 167
+    us with 64 and 331 + 165 with 128, 32 rows 348 + 172 and 345 + 169, 64 rows 364 + 187 and 342 + 179."""
+    return 64 if rows <= 24 * experts else MOE_TCGEN05_TILE
+
+
+def moe_result_dtype(rows: int, experts: int, dtype) -> torch.dtype:
+    """How the rows of the experts' last product are kept until they are summed per token: float32 in steps of few rows,
+    the storage type where many rows make them a sizeable share of a step's memory traffic."""
+    return dtype if rows >= MOE_NARROW_ROWS and rows >= 32 * experts else torch.float32
 
 
 def moe_grouped(a: torch.Tensor, w: torch.Tensor, plan: MoePlan, top: int, gated: bool, gather: bool,
@@ -1359,30 +1374,31 @@ def moe_grouped(a: torch.Tensor, w: torch.Tensor, plan: MoePlan, top: int, gated
     ``interleaved`` by eight), K].  ``gather``: ``a`` is [tokens, K] and a row reads its token, times ``weights``
     [tokens, top] if given.  ``gated``: the result is act(gate) * up [rows, N] in the storage type, else
     [rows, N] float32 (``consts``: constants of ``act``, see ``ACTIVATIONS``), or with ``unary`` act(.) [rows, N] in the storage type (``act`` then one of
-    ``ELEMENTWISE_ACTIVATIONS``).  A plan cut into tiles of 128 rows goes to the grouped tcgen05 product (bfloat16
-    in and out; the gathered rows are laid out by a kernel of their own first).  Rows of experts without matrices
-    (``plan.real``) are left unwritten."""
+    ``ELEMENTWISE_ACTIVATIONS``).  A plan made for it (``plan.tensor_memory``) goes to the tcgen05 product (bfloat16
+    in; the gathered rows are laid out by a kernel of their own first; a plain product leaves bfloat16, or float32 with
+    ``out_dtype``).  Rows of experts without matrices (``plan.real``) are left unwritten."""
     _cuda(a, w, weights)
     experts, n_total, k = w.shape
     assert a.shape[1] == k and a.dtype == w.dtype and experts == plan.real and not (gated and unary)
     act_code = ELEMENTWISE_ACTIVATIONS[act] if unary else ACTIVATIONS[act] if gated else 0
     limit, slope = _consts(act, consts) if gated else NO_CONSTS
     n = n_total // 2 if gated else n_total
-    if plan.tile_rows == MOE_TCGEN05_TILE:
+    if plan.tensor_memory:
         assert a.dtype == torch.bfloat16 and (interleaved or not gated)
         if gather:
             xs = torch.empty((plan.n, k), dtype=a.dtype, device=a.device)
             _check(lib().tllm_moe_gather(_p(a), _p(plan.src_of), _p(weights), top, _p(xs), plan.n, k, _stream()),
                    "moe_gather")
             a = xs
-        out = torch.empty((plan.n, n), dtype=torch.bfloat16, device=a.device)
+        wide = not gated and not unary and out_dtype == torch.float32
+        out = torch.empty((plan.n, n), dtype=torch.float32 if wide else torch.bfloat16, device=a.device)
         global tcgen05_calls
         tcgen05_calls += 1
-        flags = (1 | 4 | (act_code << 8)) if gated else ((16 | (act_code << 8)) if unary else 0)
-        _check(lib().tllm_gemm_tcgen05_grouped(
-            _p(a), _p(w), _p(out), plan.n, n_total, k, experts, flags, _p(plan.tile_expert), _p(plan.tile_row0),
+        flags = (1 | 4 | (act_code << 8)) if gated else ((16 | (act_code << 8)) if unary else 32 if wide else 0)
+        _check(lib().tllm_moe_tcgen05(
+            _p(a), _p(w), _p(out), plan.n, n_total, k, experts, flags, plan.tile_rows, _p(plan.tile_expert), _p(plan.tile_row0),
             _p(plan.n_tiles), _p(plan.offsets), plan.max_tiles, limit, slope, _p(error_word(a.device)), _stream()),
-            "gemm_tcgen05_grouped")
+            "moe_tcgen05")
         return out
     out = torch.empty((plan.n, n), dtype=a.dtype if (gated or unary) else torch.float32, device=a.device)
     _check(lib().tllm_moe_grouped(

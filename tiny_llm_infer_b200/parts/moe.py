@@ -23,9 +23,8 @@ Options that other routers use, each a parameter:
 
 The step's rows are sorted by expert on the device (``ops.MoePlan``); the experts' gate|up product
 gathers its rows from the tokens and applies the activation in its epilogue, the down product leaves
-rows that one kernel sums per token, in float32, with the shared unit's output.  Steps with many rows run
-both products on the grouped tcgen05 kernel (row tiles of 128 per expert), steps with few on mma.sync
-tiles of 64 rows that read the chosen experts' weights once.  Nothing is read by the host,
+rows that one kernel sums per token, in float32, with the shared unit's output.  In bfloat16
+both products run on the tcgen05 kernel, which reads the chosen experts' weights once.  Nothing is read by the host,
 so steps with this part are captured as CUDA graphs like the others.
 """
 from __future__ import annotations
@@ -155,13 +154,14 @@ class MixtureOfExperts:
         w_first = self.w_gate_up if self.gated else self.w_up
         tensor_cores = (self.interleaved or not self.gated) and x.dtype == w_first.dtype \
             and ops.moe_tcgen05_pays(rows, self.experts, self.inter, self.hidden, x.dtype)
-        plan = ops.MoePlan(ids, self.experts + self.identity, ops.MOE_TCGEN05_TILE if tensor_cores else None,
-                           real=self.experts)
+        plan = ops.MoePlan(ids, self.experts + self.identity, ops.moe_row_box(rows, self.experts) if tensor_cores else None,
+                           real=self.experts, tensor_memory=tensor_cores)
         on_input = self.weight_on == "input"
         act = ops.moe_grouped(x, w_first, plan, self.top, gated=self.gated, gather=True,
                               weights=weights if on_input else None, act=self.activation,
                               interleaved=self.interleaved, unary=not self.gated, consts=self.act_consts)
-        y = ops.moe_grouped(act, self.w_down, plan, self.top, gated=False, gather=False)
+        y = ops.moe_grouped(act, self.w_down, plan, self.top, gated=False, gather=False,
+                            out_dtype=ops.moe_result_dtype(rows, self.experts, self.dtype))
         shared = self.shared.forward(x, ctx) if self.shared is not None else None
         return ops.moe_combine(y, plan, self.top, shared, self.dtype, weights=None if on_input else weights,
                                identity_input=x if self.identity else None,
