@@ -1,0 +1,73 @@
+"""Prompt portions through the tcgen05 kernel with a changed score or output, against the general kernel (one block per row
+and head over all keys, float32 throughout), for every change alone and for mixtures of them."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV, D, PAGE = "cuda:0", 128, 16
+FORMS = {
+    "cap": dict(softcap=5.0), "slopes": dict(slopes=True), "chunk": dict(chunk=96), "chunk past a window": dict(chunk=256, window=70),
+    "sink of one": dict(sink=True), "gate": dict(gate="elements"), "gate, rows of odd length": dict(gate="odd"),
+    "gate per head": dict(gate="heads"), "cap, window, learned sink, gate per head": dict(softcap=2.0, window=150, sink=True, learned=True, gate="heads"),
+    "cap, slopes, chunk, sink, gate": dict(softcap=9.0, slopes=True, chunk=200, sink=True, gate="elements"),
+}
+
+
+def context(lengths, befores):
+    from tiny_llm_infer_b200.engine.batch import StepContext
+    seg, tiles, row = [], [], 0
+    for s, (n, p0) in enumerate(zip(lengths, befores)):
+        seg.append([s, row, n, p0])
+        tiles += [(s, off) for off in range(0, n, 64)]
+        row += n
+    tiles.sort(key=lambda t: (t[1] % 256 != 0, t[1] % 128 != 0))
+
+    def ints(v):
+        return torch.tensor(v, dtype=torch.int32, device=DEV)
+    return StepContext(tokens=row, token_ids=None, positions=ints([p0 + i for _, _, n, p0 in seg for i in range(n)]),
+                       token_slot=ints([s for s, _, n, _ in seg for _ in range(n)]), want_rows=None, segments=[], seg_info=ints(seg),
+                       dec_rows=ints([]), n_dec=0, pf_tiles=ints(tiles), n_tiles=len(tiles),
+                       n_tiles128=sum(t[1] % 128 == 0 for t in tiles), n_tiles256=sum(t[1] % 256 == 0 for t in tiles),
+                       max_context=max(n + p for n, p in zip(lengths, befores)), max_segment=max(lengths))
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+@pytest.mark.parametrize("heads,kv_heads,lengths,befores", [
+    (4, 2, (130, 2, 257), (0, 333, 61)),          # two heads of a group per block; a row past a tile, two rows, two tiles and one
+    (3, 3, (300,), (17,)),                        # two blocks of positions per block
+    (2, 1, (65,), (1500,)),                       # few rows and many keys: their keys cut into runs
+])
+def test_changes_of_the_score_and_the_output(form, heads, kv_heads, lengths, befores):
+    from tiny_llm_infer_b200 import ops
+    f = dict(FORMS[form])
+    g = torch.Generator(device=DEV).manual_seed(5)
+
+    def randn(*shape):
+        return torch.randn(*shape, generator=g, device=DEV)
+    ctx = context(lengths, befores)
+    pages = -(-ctx.max_context // PAGE)
+    order = torch.randperm(len(lengths) * pages, generator=g, device=DEV).to(torch.int32).view(len(lengths), pages)
+    planes = [randn(len(lengths) * pages, kv_heads, PAGE, D).bfloat16() for _ in range(2)]
+    q = randn(ctx.tokens, heads * D).bfloat16()
+    gate = None
+    if f.get("gate") == "heads":
+        gate = randn(ctx.tokens, heads + 3).bfloat16()[:, 2:2 + heads]
+    elif f.get("gate"):
+        at = 2 if f["gate"] == "odd" else 8
+        gate = randn(ctx.tokens, heads * D + (10 if f["gate"] == "odd" else 16)).bfloat16()[:, at:at + heads * D]
+    kw = dict(softcap=f.get("softcap", 0.0), chunk=f.get("chunk", 0), window=f.get("window", 0), sink=f.get("sink", False),
+              slopes=torch.rand(heads, generator=g, device=DEV) * 0.05 if f.get("slopes") else None, gate=gate,
+              gate_per_head=f.get("gate") == "heads", sink_logits=randn(heads) if f.get("learned") else None)
+    out = []
+    for c in (ctx, None):
+        o, before = torch.empty_like(q), ops.tcgen05_calls
+        ops.attention_biased(q, *planes, ctx.positions, ctx.token_slot, order, PAGE, heads, kv_heads, D, D, D ** -0.5, o, ctx=c, **kw)
+        assert (ops.tcgen05_calls > before) == (c is not None)
+        out.append(o.double())
+    ops.check_error_word(q.device)
+    # weights rounded to bfloat16 (2^-8 each, of weights that sum to at most one) times values of at most |v|; both results
+    # rounded to bfloat16 (2^-8 of values of at most |v| each)
+    bound = 3 * 2.0 ** -8 * planes[1].abs().max().item()
+    assert (out[0] - out[1]).abs().max().item() <= bound
+    assert ((out[0] - out[1]).norm() / out[1].norm()).item() <= 2.0 ** -7       # roundings are not all of one sign

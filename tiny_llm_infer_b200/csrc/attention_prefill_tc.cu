@@ -183,12 +183,38 @@ struct QTile {
     int head, q_off, rows, first_pos, last_pos, kt_first, n;
 };
 
+// What else the score and the output can be changed by (kChanged).  cap_in > 0: s <- cap tanh(s scale / cap) with cap_in =
+// 2 scale / cap and cap_out = cap, both times log2(e); else s scale.  slopes [q_heads] (or null): s - slope * distance.
+// chunk > 0: keys of the query's own chunk of positions only.  sink: exp(sink_logit[head]), one without logits, joins the
+// denominator.  gate (or null): the output times sigmoid of it, [tokens] rows `gate_stride` apart with a number per element
+// or, `gate_per_head`, per query head; gate_vec: its rows allow 16-byte accesses.
+struct Changes {
+    float cap_in, cap_out;
+    int chunk, sink;
+    const float* slopes;
+    const bf16* gate;
+    int gate_stride, gate_per_head, gate_vec;
+};
+constexpr Changes kNoChanges{0.0f, 0.0f, 0, 0, nullptr, nullptr, 0, 0, 0};
+enum ScoreForm : int { kPlain = 0, kBiased = 1, kChanged = 2 };
+
+__device__ __forceinline__ float rcp(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float sigmoid_of(bf16 g) { return 1.0f / (1.0f + expf(-__bfloat162float(g))); }
+
 // Keys and values lie in planes of their own: row (page * rows_per_page + head * page_size + place in the
 // page) of 128 elements from `k_base` and from `v_base` (the two halves of a page of the plain cache, or two
-// views into pages that hold more).  kBias: `dist_bias` [q_heads][dist_len] float32 is added to the scaled
+// views into pages that hold more).  kBiased: `dist_bias` [q_heads][dist_len] float32 is added to the scaled
 // score by the distance from the query to the key (distances from dist_len - 1 on share the last entry).
 // `sink_logit` (or null): exp(sink_logit[head]) joins the softmax's denominator, once, with no value.
-template <bool kBias>
+// kChanged: the changes above, but no table.  A capped score costs two exponential-unit instructions more (e^2x and the
+// reciprocal of tanh x = 1 - 2 / (e^2x + 1)); with them that unit sets the pace: 3 x 128 x 128 instructions on 16 a cycle are
+// 3070 cycles per pair of query tiles and 64 keys, where the plain form takes 1950.  One prompt of 2048 tokens, 32 heads
+// on 8, cap, window, learned sink and a gate per head: 85.5 us (363 on the mma.sync tiles of attention_biased.cu).
+template <int kForm>
 __global__ void __launch_bounds__(kThreads, 1)
 paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const bf16* __restrict__ k_base,
                                   const bf16* __restrict__ v_base, int rows_per_page,
@@ -196,10 +222,17 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                                   const int* __restrict__ block_table, int max_pages, int page_size, int q_heads,
                                   int kv_heads, int window, float scale_log2e, int pair_heads,
                                   const float* __restrict__ dist_bias, int dist_len,
-                                  const float* __restrict__ sink_logit,
+                                  const float* __restrict__ sink_logit, const Changes ch,
                                   bf16* __restrict__ out, int splits, float* __restrict__ part_o,
                                   float* __restrict__ part_ml, int* __restrict__ error_word) {
     extern __shared__ __align__(1024) unsigned char smem[];
+    constexpr bool kBias = kForm == kBiased, kChange = kForm == kChanged;
+    constexpr bool kLog2 = kForm != kPlain;                    // the scores are scaled and in base 2 before the maximum
+    auto first_key = [&](int pos) -> int {
+        int lo = window > 0 && pos - window + 1 > 0 ? pos - window + 1 : 0;
+        if (kChange && ch.chunk > 0) lo = max(lo, pos / ch.chunk * ch.chunk);
+        return lo;
+    };
     Barriers* bars = reinterpret_cast<Barriers*>(smem + kTilesBytes);
     volatile int* aborted = &bars->abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -218,8 +251,7 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
         t.rows = min(kBM, len - t.q_off);
         t.first_pos = pos0 + t.q_off;
         t.last_pos = t.first_pos + t.rows - 1;
-        const int lo = (window > 0 && t.first_pos - window + 1 > 0) ? t.first_pos - window + 1 : 0;
-        t.kt_first = lo / kBN;
+        t.kt_first = first_key(t.first_pos) / kBN;
         t.n = t.rows > 0 ? t.last_pos / kBN - t.kt_first + 1 : 0;
     }
     const int g = qt[0].head / (q_heads / kv_heads);           // both tiles read this key/value head
@@ -458,7 +490,7 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
         const int x = (warp - 4) >> 2, quad = warp & 3, r = quad * 32 + lane;
         const QTile t = x ? qt[1] : qt[0];
         const int pos = t.first_pos + r;
-        const int min_key = window > 0 ? pos - window + 1 : 0;
+        const int min_key = first_key(pos), last_first = first_key(t.last_pos);
         const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
         const uint32_t tmem_sx = tmem + lane_sel + x * 128, tmem_ox = tmem + lane_sel + 256 + x * 128;
         uint64_t* const o_full = &bars->o_full[x];
@@ -466,6 +498,7 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
         bool alive = t.n > 0 && !*aborted;
         const float* bias_row = nullptr;                      // this head's biases by distance
         float bias_far = 0.0f;                                // the last one, times log2(e)
+        const float slope2 = kChange && ch.slopes != nullptr ? ch.slopes[t.head] * kLog2e : 0.0f;
         if constexpr (kBias) {
             bias_row = dist_bias + (size_t)t.head * dist_len;
             bias_far = bias_row[dist_len - 1] * kLog2e;
@@ -505,8 +538,24 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                     }
                 }
             }
+            if constexpr (kChange) {
+                if (ch.cap_in > 0.0f) {
+                    // e overflows to infinity (tanh 1) and underflows to zero (tanh -1) where it should
+#pragma unroll
+                    for (int i = 0; i < kBN; ++i)
+                        sv[i] = __float_as_uint(fmaf(-2.0f * ch.cap_out, rcp(ex2(__uint_as_float(sv[i]) * ch.cap_in) + 1.0f), ch.cap_out));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < kBN; ++i) sv[i] = __float_as_uint(__uint_as_float(sv[i]) * scale_log2e);
+                }
+                if (ch.slopes != nullptr) {
+                    const float d0 = (float)(pos - key0);     // the distance to key i of the tile is d0 - i
+#pragma unroll
+                    for (int i = 0; i < kBN; ++i) sv[i] = __float_as_uint(fmaf(-slope2, d0 - (float)i, __uint_as_float(sv[i])));
+                }
+            }
             // only tiles on the diagonal or at the window's far edge hold keys some row may not see
-            if (key0 + kBN - 1 > t.first_pos || (window > 0 && key0 < t.last_pos - window + 1)) {
+            if (key0 + kBN - 1 > t.first_pos || key0 < last_first) {
 #pragma unroll
                 for (int i = 0; i < kBN; ++i) {
                     const int key = key0 + i;
@@ -516,7 +565,7 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
             for (int i = 0; i < kBN; ++i) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(sv[i]));
-            const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * (kBias ? 1.0f : scale_log2e);
+            const float tile_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * (kLog2 ? 1.0f : scale_log2e);
             // raise the reference maximum only when this tile is far above it
             const bool raise = tile_max > m_ref + kRaise;
             float factor = 1.0f;
@@ -551,8 +600,8 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
             uint32_t pw[kBN / 2];
 #pragma unroll
             for (int i = 0; i < kBN; i += 2) {
-                const float a = ex2(kBias ? __uint_as_float(sv[i]) - m_use : fmaf(__uint_as_float(sv[i]), scale_log2e, -m_use));
-                const float b = ex2(kBias ? __uint_as_float(sv[i + 1]) - m_use
+                const float a = ex2(kLog2 ? __uint_as_float(sv[i]) - m_use : fmaf(__uint_as_float(sv[i]), scale_log2e, -m_use));
+                const float b = ex2(kLog2 ? __uint_as_float(sv[i + 1]) - m_use
                                           : fmaf(__uint_as_float(sv[i + 1]), scale_log2e, -m_use));
                 sum[(i >> 1) & 3] += a + b;
                 pw[i >> 1] = pack2(a, b);
@@ -598,13 +647,35 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
         } else if (finish) {
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             if (sink_logit != nullptr) l_run += ex2(sink_logit[t.head] * kLog2e - m_ref);   // every row has seen a key
-            const float inv = 1.0f / l_run;
+            else if (kChange && ch.sink) l_run += ex2(-m_ref);
+            float inv = 1.0f / l_run;
+            const bf16* gate_row = nullptr;                     // a gate per element
+            if (kChange && ch.gate != nullptr && r < t.rows) {
+                const bf16* row = ch.gate + (size_t)(start + t.q_off + r) * ch.gate_stride;
+                if (ch.gate_per_head) inv *= sigmoid_of(row[t.head]);
+                else gate_row = row + (size_t)t.head * kHD;
+            }
             const uint32_t stage = q_s + x * kQBytes, stage_row = stage + r * 256;
 #pragma unroll 1
             for (int c = 0; c < kHD; c += 32) {
                 uint32_t o[32];
                 tmem_ld32(tmem_ox + c, o);
                 tmem_ld_wait();
+                if (kChange && gate_row != nullptr) {
+                    if (ch.gate_vec) {
+#pragma unroll
+                        for (int q4 = 0; q4 < 4; ++q4) {
+                            const uint4 raw = *reinterpret_cast<const uint4*>(gate_row + c + q4 * 8);
+                            const bf16* g = reinterpret_cast<const bf16*>(&raw);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e)
+                                o[q4 * 8 + e] = __float_as_uint(__uint_as_float(o[q4 * 8 + e]) * sigmoid_of(g[e]));
+                        }
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * sigmoid_of(gate_row[c + e]));
+                    }
+                }
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) {
                     uint32_t w[4];
@@ -647,7 +718,7 @@ __global__ void paged_attention_prefill_combine_kernel(const float* part_o, cons
                                                        const int* __restrict__ seg_info,
                                                        const int* __restrict__ tiles, int rows_per_tile,
                                                        int q_heads, int splits, const float* __restrict__ sink_logit,
-                                                       bf16* __restrict__ out) {
+                                                       const Changes ch, bf16* __restrict__ out) {
     const int seg = tiles[2 * blockIdx.x], q_off = tiles[2 * blockIdx.x + 1], head = blockIdx.y, d = threadIdx.x;
     const int start = seg_info[4 * seg + 1], len = seg_info[4 * seg + 2];
     for (int i = 0; i < kCombineRows; ++i) {
@@ -665,7 +736,10 @@ __global__ void paged_attention_prefill_combine_kernel(const float* part_o, cons
             acc += part_o[(base + z) * kHD + d] * f;
         }
         if (sink_logit != nullptr) total += exp2f(sink_logit[head] * kLog2e - mm);
-        out[((size_t)(start + r) * q_heads + head) * kHD + d] = __float2bfloat16_rn(acc / total);
+        else if (ch.sink) total += exp2f(-mm);
+        float v = acc / total;
+        if (ch.gate != nullptr) v *= sigmoid_of(ch.gate[(size_t)(start + r) * ch.gate_stride + (ch.gate_per_head ? head : head * kHD + d)]);
+        out[((size_t)(start + r) * q_heads + head) * kHD + d] = __float2bfloat16_rn(v);
     }
 }
 
@@ -714,8 +788,8 @@ static int launch_prefill_tc(const char* name, const void* q, int tokens, const 
                              long long rows_per_page, long long kv_rows, const int* seg_info, const int* tiles,
                              int n_tiles, const int* block_table, int max_pages, int page_size, int q_heads,
                              int kv_heads, int window, float scale, const float* dist_bias, int dist_len,
-                             const float* sink_logit, void* out, int splits, float* part_o, float* part_ml,
-                             int* error_word, cudaStream_t stream) {
+                             const float* sink_logit, const pftc::Changes* changes, void* out, int splits, float* part_o,
+                             float* part_ml, int* error_word, cudaStream_t stream) {
     TLLM_REQUIRE(q_heads > 0 && kv_heads > 0 && q_heads % kv_heads == 0 && q_heads <= 65535,
                  "%s: %d query heads over %d key/value heads", name, q_heads, kv_heads);
     TLLM_REQUIRE(page_size > 0 && page_size % 16 == 0, "%s: page size %d is no multiple of 16", name, page_size);
@@ -735,10 +809,13 @@ static int launch_prefill_tc(const char* name, const void* q, int tokens, const 
                  "%s: cuTensorMapEncodeTiled failed or is not available", name);
     static OncePerDevice configured;
     if (configured.first()) {
-        cudaError_t e = cudaFuncSetAttribute(pftc::paged_attention_prefill_tc_kernel<false>,
+        cudaError_t e = cudaFuncSetAttribute(pftc::paged_attention_prefill_tc_kernel<pftc::kPlain>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, pftc::kSmemBytes);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(pftc::paged_attention_prefill_tc_kernel<true>,
+            e = cudaFuncSetAttribute(pftc::paged_attention_prefill_tc_kernel<pftc::kBiased>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, pftc::kSmemBytes);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(pftc::paged_attention_prefill_tc_kernel<pftc::kChanged>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, pftc::kSmemBytes);
         if (e != cudaSuccess) { set_error("%s: %s", name, cudaGetErrorString(e)); return (int)e; }
         configured.done();
@@ -746,18 +823,20 @@ static int launch_prefill_tc(const char* name, const void* q, int tokens, const 
     const int rows_per_tile = tllm_paged_attention_prefill_tc_rows(q_heads, kv_heads);
     const int pair_heads = rows_per_tile == 128;
     const dim3 grid(pair_heads ? q_heads / 2 : q_heads, n_tiles, splits);
-#define PFTC(BIAS)                                                                                                \
-    pftc::paged_attention_prefill_tc_kernel<BIAS><<<grid, pftc::kThreads, pftc::kSmemBytes, stream>>>(            \
+    const pftc::Changes ch = changes != nullptr ? *changes : pftc::kNoChanges;
+#define PFTC(FORM)                                                                                                \
+    pftc::paged_attention_prefill_tc_kernel<FORM><<<grid, pftc::kThreads, pftc::kSmemBytes, stream>>>(            \
         mq, (const bf16*)k_base, (const bf16*)v_base, (int)rows_per_page, seg_info, tiles, block_table, max_pages, \
-        page_size, q_heads, kv_heads, window, scale * pftc::kLog2e, pair_heads, dist_bias, dist_len, sink_logit,  \
+        page_size, q_heads, kv_heads, window, scale * pftc::kLog2e, pair_heads, dist_bias, dist_len, sink_logit, ch, \
         (bf16*)out, splits, part_o, part_ml, error_word)
-    if (dist_bias != nullptr) PFTC(true);
-    else PFTC(false);
+    if (changes != nullptr) PFTC(pftc::kChanged);
+    else if (dist_bias != nullptr) PFTC(pftc::kBiased);
+    else PFTC(pftc::kPlain);
 #undef PFTC
     int rc = finish_launch(name);
     if (rc != 0 || splits == 1) return rc;
     pftc::paged_attention_prefill_combine_kernel<<<dim3(n_tiles, q_heads, rows_per_tile / pftc::kCombineRows), 128, 0, stream>>>(
-        part_o, part_ml, seg_info, tiles, rows_per_tile, q_heads, splits, sink_logit, (bf16*)out);
+        part_o, part_ml, seg_info, tiles, rows_per_tile, q_heads, splits, sink_logit, ch, (bf16*)out);
     return finish_launch("paged_attention_prefill_combine");
 }
 
@@ -777,24 +856,32 @@ extern "C" int tllm_paged_attention_prefill_tc(
     return launch_prefill_tc("paged_attention_prefill_tc", q, tokens, cache,
                              (const bf16*)cache + (size_t)kv_heads * page_size * 128, rows_per_page,
                              (long long)num_pages * rows_per_page, seg_info, tiles, n_tiles, block_table, max_pages,
-                             page_size, q_heads, kv_heads, window, scale, nullptr, 0, nullptr, out, splits, part_o,
+                             page_size, q_heads, kv_heads, window, scale, nullptr, 0, nullptr, nullptr, out, splits, part_o,
                              part_ml, error_word, stream);
 }
 
 // The same kernel over keys and values in planes of their own, [pages, kv_heads, page_size, 128] views whose
-// pages lie `page_stride` elements apart (a multiple of 128), with the two changes of the score the kernel
-// knows: dist_bias [q_heads, dist_len] float32 added by distance (or null) and a learned sink per query head
-// (or null).  Widths of 128 for keys and values only.
+// pages lie `page_stride` elements apart (a multiple of 128), with the changes of the score and of the output the
+// kernel knows: dist_bias [q_heads, dist_len] float32 added by distance, alone; or softcap, slopes [q_heads], chunk, a gate
+// (see Changes); with either a sink per query head (learned, or one where sink_logit is null).  Widths of 128 for keys and
+// values only.
 extern "C" int tllm_attention_planes_prefill_tc(
     const void* q, int tokens, const void* k_plane, const void* v_plane, long long page_stride, int num_pages,
     const int* seg_info, const int* tiles, int n_tiles, const int* block_table, int max_pages, int page_size,
     int q_heads, int kv_heads, int window, float scale, const float* dist_bias, int dist_len,
-    const float* sink_logit, void* out, int splits, float* part_o, float* part_ml, int* error_word,
-    cudaStream_t stream) {
+    const float* sink_logit, float softcap, int chunk, int sink, const float* slopes, const void* gate, int gate_stride,
+    int gate_per_head, void* out, int splits, float* part_o, float* part_ml, int* error_word, cudaStream_t stream) {
     TLLM_REQUIRE(page_stride > 0 && page_stride % 128 == 0,
                  "attention_planes_prefill_tc: pages %lld elements apart (no multiple of 128)", page_stride);
+    TLLM_REQUIRE(chunk >= 0 && window >= 0 && softcap >= 0.0f, "attention_planes_prefill_tc: negative constant");
+    TLLM_REQUIRE((reinterpret_cast<uintptr_t>(gate) & 1u) == 0, "attention_planes_prefill_tc: the gate must be 2-byte aligned");
+    const bool changed = softcap > 0.0f || chunk > 0 || slopes != nullptr || gate != nullptr || (sink && sink_logit == nullptr);
+    TLLM_REQUIRE(!changed || dist_bias == nullptr, "attention_planes_prefill_tc: a table of biases comes alone");
+    const pftc::Changes ch{softcap > 0.0f ? 2.0f * scale / softcap * pftc::kLog2e : 0.0f, softcap * pftc::kLog2e, chunk, sink, slopes,
+                           (const bf16*)gate, gate_stride, gate_per_head,
+                           gate_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(gate) & 15u) == 0};
     return launch_prefill_tc("attention_planes_prefill_tc", q, tokens, k_plane, v_plane, page_stride / 128,
                              (long long)num_pages * (page_stride / 128), seg_info, tiles, n_tiles, block_table,
                              max_pages, page_size, q_heads, kv_heads, window, scale, dist_bias, dist_len, sink_logit,
-                             out, splits, part_o, part_ml, error_word, stream);
+                             changed ? &ch : nullptr, out, splits, part_o, part_ml, error_word, stream);
 }

@@ -126,7 +126,8 @@ def _declare(h) -> None:
         "tllm_paged_attention_prefill_tc": [vp, i32, vp, i32, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, f32,
                                             vp, i32, vp, vp, vp, vp],
         "tllm_attention_planes_prefill_tc": [vp, i32, vp, vp, ctypes.c_longlong, i32, vp, vp, i32, vp, i32, i32,
-                                             i32, i32, i32, f32, vp, i32, vp, vp, i32, vp, vp, vp, vp],
+                                             i32, i32, i32, f32, vp, i32, vp, f32, i32, i32, vp, vp, i32, i32, vp, i32, vp,
+                                             vp, vp, vp],
     }
     for name, args in sigs.items():
         fn = getattr(h, name)
@@ -806,11 +807,13 @@ def attention_biased(q: torch.Tensor, k_plane: torch.Tensor, v_plane: torch.Tens
             _p(sink_logits), _p(distance_bias), dist_len, v_row, gate_ptr, gate_stride, int(gate_per_head), maps,
             *((0.0, 0.0, 0.0) if difference is None else (float(v) for v in difference)))
     consts = mods + (_p(out), _stream())
-    # the plain score, or one changed only by a table of biases and a learned sink, at width 128 on both
-    # sides: prompt portions go to the tcgen05 kernel of the plain cache, which reads the two planes
-    tcgen05 = PREFILL_TCGEN05 and dk == 128 and dv == 128 and maps == 1 and not values_in_keys and not softcap and not chunk \
-        and slopes is None and gate is None and (sink_logits is not None or not sink) \
-        and page_size % 16 == 0 and stride % 128 == 0 and q_heads <= 65535
+    # width 128 on both sides, one map and not a table of biases beside other changes: prompt portions go to the
+    # tcgen05 kernel of the plain cache, which reads the two planes
+    changed = bool(softcap) or bool(chunk) or slopes is not None or gate is not None or (sink and sink_logits is None)
+    tcgen05 = PREFILL_TCGEN05 and dk == 128 and dv == 128 and maps == 1 and not values_in_keys \
+        and not (changed and distance_bias is not None) \
+        and page_size % 16 == 0 and stride % 128 == 0 and q_heads <= 65535 \
+        and (q.data_ptr() | out.data_ptr() | kp | vp) % 16 == 0
     if BIASED_FAST and ctx is not None and ctx.pf_tiles is not None and ctx.tokens == tokens \
             and q.dtype == torch.bfloat16 and (gate_stride % 2 == 0 or gate_per_head) and v_row % 8 == 0 \
             and lib().tllm_attention_maps_fast_ok(q_heads, kv_heads, dk, dv, maps):
@@ -828,7 +831,7 @@ def attention_biased(q: torch.Tensor, k_plane: torch.Tensor, v_plane: torch.Tens
         if ctx.n_tiles and tcgen05 and getattr(ctx, "n_tiles256", 0):
             pairs = prefill_tcgen05_block_rows(q_heads, kv_heads) == 128
             blocks = ctx.n_tiles128 if pairs else ctx.n_tiles256
-            keys = ctx.max_context if not window else min(ctx.max_context, window + 256)
+            keys = min([ctx.max_context] + [v + 256 for v in (window, chunk) if v])
             splits = prefill_splits(blocks * (q_heads // 2 if pairs else q_heads), keys)
             part_o = part_ml = None
             if splits > 1:
@@ -840,7 +843,8 @@ def attention_biased(q: torch.Tensor, k_plane: torch.Tensor, v_plane: torch.Tens
             _check(lib().tllm_attention_planes_prefill_tc(
                 _p(q), tokens, kp, vp, stride, k_plane.shape[0], _p(ctx.seg_info), _p(ctx.pf_tiles), blocks,
                 _p(block_table), block_table.shape[1], page_size, q_heads, kv_heads, int(window or 0), float(scale),
-                _p(distance_bias), dist_len, _p(sink_logits), _p(out), splits, _p(part_o), _p(part_ml),
+                _p(distance_bias), dist_len, _p(sink_logits), float(softcap or 0.0), int(chunk or 0), int(bool(sink)), _p(slopes),
+                gate_ptr, gate_stride, int(gate_per_head), _p(out), splits, _p(part_o), _p(part_ml),
                 _p(error_word(q.device)), _stream()), "attention_planes_prefill_tc", kernels=2 if splits > 1 else 1)
         elif ctx.n_tiles:
             _check(lib().tllm_attention_biased_prefill(
