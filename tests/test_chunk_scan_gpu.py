@@ -1,0 +1,100 @@
+"""The recurrences by chunks of sixteen tokens against float64 and against the token-by-token scan: portions at the edges of a
+chunk, portions in any order, rows of no request, every recurrence the chunks serve."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def lanes(dk):
+    return 4 if dk <= 64 else 8
+
+
+def pack(S):
+    """[slots, heads, dk, dv] in the layout of a request's state."""
+    n, heads, dk, dv = S.shape
+    return S.reshape(n, heads, lanes(dk), dk // lanes(dk), dv).permute(0, 1, 3, 4, 2).reshape(n, -1).contiguous()
+
+
+def unpack(flat, heads, dk, dv):
+    return flat.reshape(-1, heads, dk // lanes(dk), dv, lanes(dk)).permute(0, 1, 4, 2, 3).reshape(-1, heads, dk, dv)
+
+
+@pytest.mark.parametrize("mode", ["delta", "channel", "channel, no weights", "head", "fixed"])
+@pytest.mark.parametrize("heads,kv_heads,dk,dv", [(4, 2, 128, 128), (3, 3, 64, 48), (8, 8, 128, 16), (40, 40, 64, 64)])
+@pytest.mark.parametrize("lengths", [(1, 15, 16, 17, 33), (200,), (64, 0, 31, 47)])
+def test_chunks_are_the_recurrence(mode, heads, kv_heads, dk, dv, lengths, monkeypatch):
+    from tiny_llm_infer_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(7)
+    n = len(lengths)
+    starts, row = [0] * n, 3                                       # rows of no portion before, between and after
+    for s in reversed(range(n)):                                   # the portions' rows lie in the opposite order
+        starts[s], row = row, row + lengths[s] + (2 if s == 1 else 0)
+    tokens = row + 5
+    slots = [n - s for s in range(n)]
+    if n > 2:
+        slots[2] = -1                                              # a portion of no request: left alone
+    seg = torch.tensor([[slots[s], starts[s], lengths[s], 0] for s in range(n)], dtype=torch.int32, device=DEV)
+
+    def randn(*shape):
+        return torch.randn(*shape, generator=g, device=DEV)
+    q, k = (torch.nn.functional.normalize(randn(tokens, kv_heads, dk), dim=-1) for _ in range(2))
+    v = randn(tokens, heads, dv)
+    decay = beta = fgate = None
+    if mode in ("delta", "channel", "channel, no weights"):
+        decay = torch.rand(tokens, heads, dk, generator=g, device=DEV) ** 0.2          # many near one, some near zero
+        decay[::7, :, ::5] = 0.0
+    if mode in ("delta", "channel"):
+        beta = torch.rand(tokens, heads, generator=g, device=DEV)
+    if mode == "head":
+        beta, fgate = torch.rand(tokens, heads, generator=g, device=DEV) ** 0.3, torch.rand(tokens, heads, generator=g, device=DEV)
+    if mode == "fixed":
+        fgate = torch.rand(heads, generator=g, device=DEV) ** 0.1
+    code = {"delta": ops.SCAN_DELTA, "head": ops.SCAN_HEAD_DECAY, "fixed": ops.SCAN_FIXED_DECAY}.get(mode, ops.SCAN_PLAIN)
+    S0 = randn(n + 1, heads, dk, dv)
+
+    want_o, want_S = torch.zeros(tokens, heads, dv, dtype=torch.float64, device=DEV), S0.double()
+    rep = heads // kv_heads
+    for s in range(n):
+        if slots[s] < 0:
+            continue
+        S = want_S[slots[s]].clone()
+        for t in range(starts[s], starts[s] + lengths[s]):
+            kt, qt = (x[t].double().repeat_interleave(rep, 0) for x in (k, q))
+            if mode == "head":
+                S = S * beta[t].double()[:, None, None]
+            elif mode == "fixed":
+                S = S * fgate.double()[:, None, None]
+            else:
+                S = S * decay[t].double()[..., None]
+            u = v[t].double()
+            if mode == "delta":
+                u = beta[t].double()[:, None] * (u - torch.einsum("hkv,hk->hv", S, kt))
+            elif mode == "channel":
+                u = beta[t].double()[:, None] * u
+            elif mode == "head":
+                u = fgate[t].double()[:, None] * u
+            S = S + kt[..., None] * u[:, None]
+            want_o[t] = torch.einsum("hkv,hk->hv", S, qt)
+        want_S[slots[s]] = S
+
+    def run(by_chunks):
+        monkeypatch.setattr(ops, "CHUNK_TOKENS", 1 if by_chunks else 1 << 30)
+        state, o = pack(S0), torch.zeros(tokens, heads, dv, device=DEV)
+        before = ops.launches
+        ops._scan(code, seg, tokens, None, q, k, v, decay, beta, state, heads, kv_heads, dk, dv, o, fgate=fgate)
+        assert ops.launches - before == (2 if by_chunks else 1)
+        return o, unpack(state, heads, dk, dv)
+
+    (o, S), (o1, S1) = run(True), run(False)
+    for got, token, want in ((o, o1, want_o), (S, S1, want_S)):
+        error, token_error = ((x.double() - want).norm() / want.norm() for x in (got, token))
+        # both sum in float32 (2^-24 a step); the chunks' sums may not be further off than a few more roundings
+        assert error <= 1.5 * token_error + 2.0 ** -23, (float(error), float(token_error))
+    idle = torch.ones(tokens, dtype=torch.bool, device=DEV)
+    for s in range(n):
+        if slots[s] >= 0:
+            idle[starts[s]:starts[s] + lengths[s]] = False
+    assert (o[idle] == 0).all()                                    # nothing is written for the others

@@ -129,10 +129,14 @@ def _declare(h) -> None:
                                              i32, i32, i32, f32, vp, i32, vp, f32, i32, i32, vp, vp, i32, i32, vp, i32, vp,
                                              vp, vp, vp],
     }
+    sigs["tllm_chunk_scan"] = [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, vp, i32, vp]
+    sigs["tllm_chunk_scan_ok"] = [i32, i32]
     for name, args in sigs.items():
         fn = getattr(h, name)
         fn.argtypes = args
         fn.restype = i32
+    h.tllm_chunk_scan_floats.argtypes = [i32, i32, i32]
+    h.tllm_chunk_scan_floats.restype = i64
     h.tllm_delta_rule_lanes.argtypes = [i32]
     h.tllm_delta_rule_lanes.restype = i32
     h.tllm_delta_rule_state_floats.argtypes = [i32, i32, i32, i32, i32]
@@ -1001,6 +1005,26 @@ def delta_rule_state_floats(heads: int, kv_heads: int, dk: int, dv: int, taps: i
 
 
 SCAN_DELTA, SCAN_PLAIN, SCAN_MEMORY, SCAN_HEAD_DECAY, SCAN_ERASE, SCAN_FIXED_DECAY = 0, 1, 2, 3, 4, 5     # recurrences of the scan kernel (csrc/delta_rule.cu, ScanMode)
+CHUNK_MODES = (SCAN_DELTA, SCAN_PLAIN, SCAN_HEAD_DECAY, SCAN_FIXED_DECAY)      # that csrc/chunk_scan.cu knows
+CHUNK_TOKENS = 64         # tokens per portion, on average, from which on the recurrences run by chunks
+
+
+def _scan(mode, seg_info, tokens, token_slot, qn, kn, vv, decay, beta, state, heads, kv_heads, dk, cols, o_raw, fgate=None,
+          erase=None, aux_off=0, floor_eps=0.0, den=None) -> None:
+    """The recurrence itself: by chunks of sixteen tokens for prompt portions, else token by token."""
+    segments = tokens if seg_info is None else seg_info.shape[0]
+    if seg_info is not None and mode in CHUNK_MODES and 0 < segments <= 65535 and tokens >= CHUNK_TOKENS * segments \
+            and lib().tllm_chunk_scan_ok(dk, cols):
+        pairs = torch.empty(lib().tllm_chunk_scan_floats(tokens, segments, heads), dtype=torch.float32, device=qn.device)
+        _check(lib().tllm_chunk_scan(_p(seg_info), segments, tokens, _p(qn), _p(kn), _p(vv), _p(decay), _p(beta), _p(fgate),
+                                     _p(pairs), _p(state), state.stride(0), heads, kv_heads, dk, cols, _p(o_raw), mode, _stream()),
+               "chunk_scan", kernels=2)
+        return
+    _check(lib().tllm_delta_scan(_p(seg_info), segments, tokens, _p(token_slot), _p(qn), _p(kn), _p(vv), _p(decay), _p(beta),
+                                 _p(state), state.stride(0), heads, kv_heads, dk, cols, _p(o_raw), mode, _p(fgate), _p(erase),
+                                 aux_off, float(floor_eps), _p(den), _stream()), "delta_scan")
+
+
 INPUT_ACTS = {None: 0, "silu": 1}                     # of q, k and v before a recurrence without a correction
 GATE_ACTS = {"sigmoid": 0, "silu": 1}                # what the read-out is multiplied by: act(gate)
 
@@ -1053,10 +1077,7 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, taps: int, a: torch.Ten
                                     float(unit_eps), _p(qn), _p(kn), _p(vv), _p(decay), _p(beta), tokens,
                                     int(decay_per_head), -1 if beta_col is None else int(beta_col), _stream()),
            "delta_prepare")
-    segments = tokens if seg_info is None else seg_info.shape[0]
-    _check(lib().tllm_delta_scan(_p(seg_info), segments, tokens, _p(token_slot), _p(qn), _p(kn), _p(vv), _p(decay), _p(beta),
-                                 _p(state), state.stride(0), heads, kv_heads, dk, dv, _p(o_raw), SCAN_DELTA, None, None, 0, 0.0,
-                                 None, _stream()), "delta_scan")
+    _scan(SCAN_DELTA, seg_info, tokens, token_slot, qn, kn, vv, decay, beta, state, heads, kv_heads, dk, dv, o_raw)
     return _delta_finish(o_raw, gate, out_weight, False, eps, token_slot, tokens, heads, kv_heads, dk, dv, out_dtype,
                          proj, ld, taps, state, None, gate_act)
 
@@ -1090,10 +1111,7 @@ def erase_delta_rule(proj: torch.Tensor, a_col: int, z: torch.Tensor, z_bias: to
     _check(lib().tllm_erase_prepare(_p(proj), ld, _dt(proj), int(a_col), _p(z), z.stride(0), _p(z_bias), _p(a_bias), float(rate),
                                     _p(token_slot), heads, dk, dv, float(unit_eps), _p(qn), _p(kn), _p(vv), _p(decay),
                                     _p(erase), tokens, _stream()), "erase_prepare")
-    segments = tokens if seg_info is None else seg_info.shape[0]
-    _check(lib().tllm_delta_scan(_p(seg_info), segments, tokens, _p(token_slot), _p(qn), _p(kn), _p(vv), _p(decay), None,
-                                 _p(state), state.stride(0), heads, heads, dk, dv, _p(o_raw), SCAN_ERASE, None, _p(erase), 0,
-                                 0.0, None, _stream()), "delta_scan")
+    _scan(SCAN_ERASE, seg_info, tokens, token_slot, qn, kn, vv, decay, None, state, heads, heads, dk, dv, o_raw, erase=erase)
     return _delta_finish(o_raw, gate, out_weight, weight_per_head, eps, token_slot, tokens, heads, heads, dk, dv,
                          out_dtype, None, 0, 1, state, None, gate_act)
 
@@ -1154,13 +1172,9 @@ def linear_recurrence(proj: torch.Tensor, kind: str, z: Optional[torch.Tensor], 
     _check(lib().tllm_linear_prepare(_p(proj), ld, _dt(proj), None if fixed else z.data_ptr(), 0 if fixed else z.stride(0), _p(z_bias),
                                      LINEAR_KINDS[kind], INPUT_ACTS[input_act], float(p0), _p(token_slot), heads, dk, dv, float(q_scale), _p(qn), _p(kn), _p(vv),
                                      _p(decay), _p(wgate), _p(fgate), tokens, _stream()), "linear_prepare")
-    segments = tokens if seg_info is None else seg_info.shape[0]
     aux_off = delta_rule_state_floats(heads, heads, dk, cols, 1) if memory else 0
-    _check(lib().tllm_delta_scan(_p(seg_info), segments, tokens, _p(token_slot), _p(qn), _p(kn), _p(vv), _p(decay), _p(wgate),
-                                 _p(state), state.stride(0), heads, heads, dk, cols, _p(o_raw),
-                                 SCAN_MEMORY if memory else SCAN_FIXED_DECAY if fixed else SCAN_PLAIN,
-                                 _p(z_bias) if fixed else _p(fgate), None, aux_off, float(floor_eps), _p(den), _stream()),
-           "delta_scan")
+    _scan(SCAN_MEMORY if memory else SCAN_FIXED_DECAY if fixed else SCAN_PLAIN, seg_info, tokens, token_slot, qn, kn, vv, decay,
+          wgate, state, heads, heads, dk, cols, o_raw, fgate=z_bias if fixed else fgate, aux_off=aux_off, floor_eps=floor_eps, den=den)
     if norm_whole:
         assert weight_per_head and den is None and gate.stride(1) == 1 and gate.dtype in (torch.float32, out_dtype)
         assert out_weight.dtype == torch.float32 and out_weight.numel() == heads * dv == gate.shape[1]
@@ -1214,10 +1228,8 @@ def state_space(proj: torch.Tensor, conv_w: torch.Tensor, conv_b: Optional[torch
     _check(lib().tllm_ssd_prepare(_p(proj), ld, _dt(proj), _p(conv_w), _p(conv_t), _p(conv_b), taps, _p(dt_bias), _p(rate),
                                   _p(token_slot), _p(state), state.stride(0), tail_off, heads, groups, n_state, head_dim,
                                   _p(qn), _p(kn), _p(vv), _p(decay), _p(step), tokens, _stream()), "ssd_prepare")
-    segments = tokens if seg_info is None else seg_info.shape[0]
-    _check(lib().tllm_delta_scan(_p(seg_info), segments, tokens, _p(token_slot), _p(qn), _p(kn), _p(vv), None, _p(decay),
-                                 _p(state), state.stride(0), heads, groups, n_state, head_dim, _p(o_raw), SCAN_HEAD_DECAY,
-                                 _p(step), None, 0, 0.0, None, _stream()), "delta_scan")
+    _scan(SCAN_HEAD_DECAY, seg_info, tokens, token_slot, qn, kn, vv, None, decay, state, heads, groups, n_state, head_dim, o_raw,
+          fgate=step)
     out = torch.empty((tokens, inner), dtype=out_dtype, device=proj.device)
     _check(lib().tllm_ssd_finish(_p(o_raw), _p(vv), _p(skip), head_dim, _p(proj), ld, _dt(proj), _p(out_weight), float(eps),
                                  int(norm_groups), _p(token_slot), tokens, inner, channels, taps, _p(state),
