@@ -463,12 +463,15 @@ static int launch_chunks(const int* seg_info, int segments, int rows, const floa
     chunk_pairs_kernel<DK, KIND><<<dim3((heads + 3) / 4, segments, each < 65535 ? each : 65535), 128, 0, stream>>>(
         seg_info, segments, qn, kn, decay, beta, fgate, heads, kv_heads, pairs);
     if (int rc = finish_launch("chunk_pairs")) return rc;
-    // blocks of 32 columns read the tokens' rows least often; 16 where those would leave multiprocessors without a block
+    // Blocks of 32 columns, four per lane, read the tokens' rows from shared memory least often, which is what bounds a full grid
+    // (2048 tokens of 32 heads of 128 x 128, delta rule, with the pairs: 353 us; two per lane 378, blocks of 16 columns 485 and
+    // 404).  Where they would leave a quarter of the multiprocessors without a block, 16 columns, two per lane (16 heads: 227 us
+    // against 327; four per lane 338).
     const int sms = sm_count_cached() > 0 ? sm_count_cached() : 148;
 #define CHUNK_LAUNCH(COLS, NL) \
     return launch_chunk_scan<DK, KIND, COLS, NL>(seg_info, segments, qn, kn, vv, decay, pairs, state, state_stride, heads, kv_heads, dv, o_raw, stream)
     if (dv % 32 == 0 && (long long)segments * heads * (dv / 32) * 4 >= 3LL * sms) CHUNK_LAUNCH(32, 4);
-    CHUNK_LAUNCH(16, 4);
+    CHUNK_LAUNCH(16, 2);
 #undef CHUNK_LAUNCH
 }
 

@@ -1006,14 +1006,17 @@ def delta_rule_state_floats(heads: int, kv_heads: int, dk: int, dv: int, taps: i
 
 SCAN_DELTA, SCAN_PLAIN, SCAN_MEMORY, SCAN_HEAD_DECAY, SCAN_ERASE, SCAN_FIXED_DECAY = 0, 1, 2, 3, 4, 5     # recurrences of the scan kernel (csrc/delta_rule.cu, ScanMode)
 CHUNK_MODES = (SCAN_DELTA, SCAN_PLAIN, SCAN_HEAD_DECAY, SCAN_FIXED_DECAY)      # that csrc/chunk_scan.cu knows
-CHUNK_TOKENS = 64         # tokens per portion, on average, from which on the recurrences run by chunks
+CHUNK_TOKENS = 64         # tokens per portion, on average, from which on the recurrences run by chunks (and in a step of half as
+                          # many again: a second kernel and less work per token break even at 64 to 96 tokens of one portion;
+                          # the delta rule with 32 heads of 128 x 128: 64 tokens 26 us against 24, 128 tokens 36 against 42,
+                          # eight portions of 32 tokens 53 against 54, of 64 tokens 80 against 99)
 
 
 def _scan(mode, seg_info, tokens, token_slot, qn, kn, vv, decay, beta, state, heads, kv_heads, dk, cols, o_raw, fgate=None,
           erase=None, aux_off=0, floor_eps=0.0, den=None) -> None:
     """The recurrence itself: by chunks of sixteen tokens for prompt portions, else token by token."""
     segments = tokens if seg_info is None else seg_info.shape[0]
-    if seg_info is not None and mode in CHUNK_MODES and 0 < segments <= 65535 and tokens >= CHUNK_TOKENS * segments \
+    if seg_info is not None and mode in CHUNK_MODES and 0 < segments <= 65535 and 2 * tokens >= CHUNK_TOKENS * max(2 * segments, 3) \
             and lib().tllm_chunk_scan_ok(dk, cols):
         pairs = torch.empty(lib().tllm_chunk_scan_floats(tokens, segments, heads), dtype=torch.float32, device=qn.device)
         _check(lib().tllm_chunk_scan(_p(seg_info), segments, tokens, _p(qn), _p(kn), _p(vv), _p(decay), _p(beta), _p(fgate),
