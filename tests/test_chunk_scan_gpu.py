@@ -98,3 +98,57 @@ def test_chunks_are_the_recurrence(mode, heads, kv_heads, dk, dv, lengths, monke
         if slots[s] >= 0:
             idle[starts[s]:starts[s] + lengths[s]] = False
     assert (o[idle] == 0).all()                                    # nothing is written for the others
+
+
+@pytest.mark.parametrize("mode", ["delta", "channel", "head", "fixed", "erase"])
+@pytest.mark.parametrize("rows", [1, 5, 70])
+@pytest.mark.parametrize("heads,kv_heads,dk,dv", [(4, 2, 128, 128), (3, 3, 64, 24), (2, 2, 128, 200), (6, 6, 64, 128)])
+def test_rows_of_one_token(mode, rows, heads, kv_heads, dk, dv):
+    """One step of the recurrence for requests that each bring one token, some rows of no request among them."""
+    from tiny_llm_infer_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(9)
+    if mode == "erase":
+        kv_heads = heads
+
+    def randn(*shape):
+        return torch.randn(*shape, generator=g, device=DEV)
+
+    def rand(*shape):
+        return torch.rand(*shape, generator=g, device=DEV)
+    slot = torch.randperm(rows, generator=g, device=DEV).to(torch.int32)
+    slot[1::3] = -1
+    q, k = (torch.nn.functional.normalize(randn(rows, kv_heads, dk), dim=-1) for _ in range(2))
+    v, S0 = randn(rows, heads, dv), randn(rows, heads, dk, dv)
+    decay = rand(rows, heads, dk) if mode in ("delta", "channel", "erase") else None
+    beta = rand(rows, heads) if mode in ("delta", "channel", "head") else None
+    fgate = rand(rows, heads) if mode == "head" else rand(heads) if mode == "fixed" else None
+    erase = k * rand(rows, heads, dk) if mode == "erase" else None
+    code = {"delta": ops.SCAN_DELTA, "channel": ops.SCAN_PLAIN, "head": ops.SCAN_HEAD_DECAY, "fixed": ops.SCAN_FIXED_DECAY, "erase": ops.SCAN_ERASE}[mode]
+    state, o = pack(S0), torch.zeros(rows, heads, dv, device=DEV)
+    ops._scan(code, None, rows, slot, q, k, v, decay, beta, state, heads, kv_heads, dk, dv, o, fgate=fgate, erase=erase)
+    live = slot >= 0
+    S, kt, qt = S0.double()[slot.clamp(min=0).long()], *(x.double().repeat_interleave(heads // kv_heads, 1) for x in (k, q))
+    old = S
+    if mode == "head":
+        S = S * beta.double()[..., None, None]
+    elif mode == "fixed":
+        S = S * fgate.double()[:, None, None]
+    else:
+        S = S * decay.double()[..., None]
+    u = v.double()
+    if mode == "delta":
+        u = beta.double()[..., None] * (u - torch.einsum("rhkv,rhk->rhv", S, kt))
+    elif mode in ("channel", "head"):
+        u = (beta if mode == "channel" else fgate).double()[..., None] * u
+    elif mode == "erase":
+        S = S - erase.double()[..., None] * torch.einsum("rhkv,rhk->rhv", old, kt)[:, :, None]
+    S = S + kt[..., None] * u[:, :, None]
+    want = torch.einsum("rhkv,rhk->rhv", S, qt)
+    got = unpack(state, heads, dk, dv).double()
+    assert (o[~live] == 0).all()
+    untouched = torch.ones(rows, dtype=torch.bool, device=DEV)
+    untouched[slot[live].long()] = False
+    assert torch.equal(got[untouched], S0.double()[untouched])
+    # sums of up to dk float32 products, a few roundings of 2^-24 each on average
+    assert ((o.double() - want)[live].norm() / want[live].norm()) < 4e-7
+    assert ((got[slot[live].long()] - S[live]).norm() / S[live].norm()) < 4e-7

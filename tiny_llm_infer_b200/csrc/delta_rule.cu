@@ -14,6 +14,7 @@
 //                  to R neighbouring lanes, which add their partial dot products with shuffles) and walks
 //                  the portion's tokens, which come through two stages of shared memory sixteen at a time
 //                  (cp.async: the next sixteen are on their way while these are walked; eight for the widest keys).
+//   delta_step     the same for rows of one token: one block per (row, head) or less, the state read and written once.
 //   delta_finish   one block per token: o divided by its root mean square per head, times a weight, times
 //                  sigmoid(gate); the block of a portion's last token also moves the convolution's
 //                  window of the request's state on.
@@ -541,6 +542,81 @@ delta_scan_kernel(const int* __restrict__ seg_info, const int* __restrict__ toke
     }
 }
 
+// ---------------------------------------------------------------- rows of one token
+// A step of one token per request reads every state once and writes it once, and nothing else counts.  A thread keeps four
+// neighbouring lanes' shares of a column (64 rows; keys of 64 elements: the whole column), so that its sixteen loads of 16
+// bytes are all under way before the first is needed; R / 4 threads share a column.  The scan kernel above, with its sixteen
+// loads of four bytes per thread and stages for tokens that are not there, took 90 us for 64 rows of 32 heads of 128 x 128
+// (268 MB, 3.0 TB/s), this ONE_US.  Every mode but the matrix memory.
+template <int DK, int MODE>
+__global__ void __launch_bounds__(256, 2)
+delta_step_kernel(const int* __restrict__ token_slot, const float* qn, const float* kn, const float* vv, const float* decay,
+                  const float* beta, const float* fgate, const float* erase, float* state, long long state_stride, int heads,
+                  int kv_heads, int dv, float* o_raw) {
+    constexpr int kR = DK <= 64 ? 4 : 8, kG = kR / 4, kPer = DK / kR;
+    constexpr bool kDecayRows = MODE == kScanDelta || MODE == kScanPlain || MODE == kScanErase;
+    __shared__ __align__(16) float rows[4][DK];                 // k, q, g, e of the token: row r * per + il at [il][r]
+    TLLM_PDL_ENTER();
+    const int t = blockIdx.x, head = blockIdx.y, slot = token_slot[t];
+    if (slot < 0) return;
+    const int j = blockIdx.z * (blockDim.x / kG) + threadIdx.x / kG, g = threadIdx.x % kG;
+    const bool live = j < dv;
+    const int kvh = head / (heads / kv_heads);
+    float* at = state + (long long)slot * state_stride + (size_t)head * DK * dv + (size_t)j * kR + 4 * g;
+    float4 S[kPer];
+#pragma unroll
+    for (int il = 0; il < kPer; ++il)
+        S[il] = live ? *reinterpret_cast<const float4*>(at + (size_t)il * dv * kR) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int i = threadIdx.x; i < DK; i += blockDim.x) {
+        const int to = (i % kPer) * kR + i / kPer;
+        rows[0][to] = kn[((size_t)t * kv_heads + kvh) * DK + i];
+        rows[1][to] = qn[((size_t)t * kv_heads + kvh) * DK + i];
+        if (kDecayRows) rows[2][to] = decay[((size_t)t * heads + head) * DK + i];
+        if (MODE == kScanErase) rows[3][to] = erase[((size_t)t * heads + head) * DK + i];
+    }
+    const size_t th = (size_t)t * heads + head;
+    const float v = live ? vv[th * dv + j] : 0.0f;
+    float keep = 1.0f, write = 1.0f;
+    if (MODE == kScanDelta) write = beta[th];
+    if (MODE == kScanPlain && beta != nullptr) write = beta[th];
+    if (MODE == kScanHeadDecay) { keep = beta[th]; write = fgate[th]; }
+    if (MODE == kScanFixedDecay) keep = fgate[head];
+    __syncthreads();
+    auto row4 = [&](int which, int il) -> float4 { return *reinterpret_cast<const float4*>(&rows[which][il * kR + 4 * g]); };
+    auto share = [&](float x) -> float { return kG == 2 ? x + __shfl_xor_sync(0xffffffffu, x, 1) : x; };
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int il = 0; il < kPer; ++il) {
+        const float4 k = row4(0, il), gg = kDecayRows ? row4(2, il) : make_float4(keep, keep, keep, keep);
+        float4& x = S[il];
+        if (MODE == kScanErase) {                               // the removal reads the state before its decay
+            acc.x = fmaf(x.x, k.x, acc.x); acc.y = fmaf(x.y, k.y, acc.y); acc.z = fmaf(x.z, k.z, acc.z); acc.w = fmaf(x.w, k.w, acc.w);
+        }
+        x.x *= gg.x; x.y *= gg.y; x.z *= gg.z; x.w *= gg.w;
+        if (MODE == kScanDelta) {
+            acc.x = fmaf(x.x, k.x, acc.x); acc.y = fmaf(x.y, k.y, acc.y); acc.z = fmaf(x.z, k.z, acc.z); acc.w = fmaf(x.w, k.w, acc.w);
+        }
+    }
+    float dot = 0.0f;
+    if (MODE == kScanDelta || MODE == kScanErase) dot = share((acc.x + acc.y) + (acc.z + acc.w));
+    const float u = MODE == kScanDelta ? write * (v - dot) : write * v;
+    acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int il = 0; il < kPer; ++il) {
+        const float4 k = row4(0, il), q = row4(1, il);
+        float4& x = S[il];
+        if (MODE == kScanErase) {
+            const float4 e = row4(3, il);
+            x.x = fmaf(e.x, -dot, x.x); x.y = fmaf(e.y, -dot, x.y); x.z = fmaf(e.z, -dot, x.z); x.w = fmaf(e.w, -dot, x.w);
+        }
+        x.x = fmaf(k.x, u, x.x); x.y = fmaf(k.y, u, x.y); x.z = fmaf(k.z, u, x.z); x.w = fmaf(k.w, u, x.w);
+        acc.x = fmaf(x.x, q.x, acc.x); acc.y = fmaf(x.y, q.y, acc.y); acc.z = fmaf(x.z, q.z, acc.z); acc.w = fmaf(x.w, q.w, acc.w);
+        if (live) *reinterpret_cast<float4*>(at + (size_t)il * dv * kR) = x;
+    }
+    const float o = share((acc.x + acc.y) + (acc.z + acc.w));
+    if (live && g == 0) o_raw[th * dv + j] = o;
+}
+
 // ---------------------------------------------------------------- finish
 // gate_act: 0 sigmoid(gate), 1 SiLU(gate).  weight_stride: 0 where the heads share one weight of dv numbers, dv
 // where every head has its own.  den: a divisor per (token, head) applied before the root mean square, or null.
@@ -605,6 +681,14 @@ template <> __device__ __forceinline__ float4 load_gate4<bf16>(const bf16* p) {
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
+__device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void store4(bf16* p, float4 v) {
+    uint2 raw;
+    *reinterpret_cast<__nv_bfloat162*>(&raw.x) = __floats2bfloat162_rn(v.x, v.y);
+    *reinterpret_cast<__nv_bfloat162*>(&raw.y) = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = raw;
+}
+
 template <typename T, typename TG>
 __global__ void delta_finish_vec_kernel(const float* o_raw, const TG* gate, int ldg, const float* __restrict__ weight,
                                         float eps, const int* __restrict__ token_slot, int n_rows, int heads, int dv,
@@ -622,24 +706,24 @@ __global__ void delta_finish_vec_kernel(const float* o_raw, const TG* gate, int 
     const int Y = gridDim.y, yb = blockIdx.y;          // with few rows a token's heads and channels are dealt to gridDim.y blocks
     for (int h = heads * yb / Y + warp; h < heads * (yb + 1) / Y; h += warps) {
         const float* src = o_raw + ((size_t)t * heads + h) * dv;
-        const float dn = den != nullptr ? den[(size_t)t * heads + h] : 1.0f;
+        const bool divide = den != nullptr;
+        const float dn = divide ? den[(size_t)t * heads + h] : 1.0f;
         float sum = 0.0f;
         for (int e = lane * 4; e < dv; e += 128) {
             float4 v = *reinterpret_cast<const float4*>(src + e);
-            v.x /= dn; v.y /= dn; v.z /= dn; v.w /= dn;
+            if (divide) { v.x /= dn; v.y /= dn; v.z /= dn; v.w /= dn; }
             sum += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
         }
         sum = warp_sum(sum);
         const float sc = 1.0f / sqrtf(sum / (float)dv + eps);
         for (int e = lane * 4; e < dv; e += 128) {
-            const float4 v = *reinterpret_cast<const float4*>(src + e);
+            float4 v = *reinterpret_cast<const float4*>(src + e);
+            if (divide) { v.x /= dn; v.y /= dn; v.z /= dn; v.w /= dn; }
             const float4 g = load_gate4<TG>(gate + (size_t)t * ldg + (size_t)h * dv + e);
             const float4 w = *reinterpret_cast<const float4*>(weight + (size_t)h * weight_stride + e);
             T* dst = out + ((size_t)t * heads + h) * dv + e;
-            dst[0] = from_f32<T>(v.x / dn * sc * w.x * finish_gate(g.x, gate_act));
-            dst[1] = from_f32<T>(v.y / dn * sc * w.y * finish_gate(g.y, gate_act));
-            dst[2] = from_f32<T>(v.z / dn * sc * w.z * finish_gate(g.z, gate_act));
-            dst[3] = from_f32<T>(v.w / dn * sc * w.w * finish_gate(g.w, gate_act));
+            store4(dst, make_float4(v.x * sc * w.x * finish_gate(g.x, gate_act), v.y * sc * w.y * finish_gate(g.y, gate_act),
+                                    v.z * sc * w.z * finish_gate(g.z, gate_act), v.w * sc * w.w * finish_gate(g.w, gate_act)));
         }
     }
     if (taps > 1 && (t + 1 >= n_rows || token_slot[t + 1] != slot)) {
@@ -1046,6 +1130,30 @@ int tllm_delta_scan(const int* seg_info, int segments, int rows, const int* toke
     if (segments == 0) return 0;
     const int r = delta_lanes(dk), per = (dk + r - 1) / r;
     TLLM_REQUIRE(per <= kScanMaxPer, "delta_scan: keys of width %d are too wide", dk);
+    if (seg_info == nullptr && mode != kScanMemory && (dk == 64 || dk == 128) && state_stride % 4 == 0 &&
+        (reinterpret_cast<uintptr_t>(state) & 15u) == 0) {
+        const int share = dk == 64 ? 1 : 2;
+        int threads = 256;                              // whole warps; fewer columns per block where few rows leave the GPU empty
+        while (threads > 64 && ((long long)segments * heads * threads < 256LL * 2 * (sm_count_cached() > 0 ? sm_count_cached() : 148) ||
+                                threads / 2 >= dv * share)) threads /= 2;
+        const dim3 grid(segments, heads, (dv * share + threads - 1) / threads);
+#define STEP(DK, MM)                                                                                                          \
+    launch_pdl(kPdlOther, delta_step_kernel<DK, MM>, grid, dim3(threads), 0, stream, token_slot, qn, kn, vv, decay, beta, fgate, erase, \
+               state, state_stride, heads, kv_heads, dv, o_raw)
+#define STEP_MODE(MM)                        \
+    do {                                     \
+        if (dk == 64) STEP(64, MM);          \
+        else STEP(128, MM);                  \
+    } while (0)
+        if (mode == kScanDelta) STEP_MODE(kScanDelta);
+        else if (mode == kScanPlain) STEP_MODE(kScanPlain);
+        else if (mode == kScanHeadDecay) STEP_MODE(kScanHeadDecay);
+        else if (mode == kScanErase) STEP_MODE(kScanErase);
+        else STEP_MODE(kScanFixedDecay);
+#undef STEP_MODE
+#undef STEP
+        return finish_launch("delta_step");
+    }
     // columns per block: whole warps, at most 256 threads, not wider than the values, and at least a block per
     // multiprocessor in all where the value width allows it (a column does not depend on the others, so the
     // result is the same however they are dealt)
