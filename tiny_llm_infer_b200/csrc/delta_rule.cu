@@ -23,6 +23,7 @@
 // [taps - 1][channels] inputs of the convolution, the newest last.  R and per follow from dk alone
 // (`tllm_delta_rule_lanes`), so every step of a request finds the layout the last one left.
 #include "common.cuh"
+#include "conv_window.cuh"
 
 namespace tllm {
 
@@ -547,7 +548,7 @@ delta_scan_kernel(const int* __restrict__ seg_info, const int* __restrict__ toke
 // neighbouring lanes' shares of a column (64 rows; keys of 64 elements: the whole column), so that its sixteen loads of 16
 // bytes are all under way before the first is needed; R / 4 threads share a column.  The scan kernel above, with its sixteen
 // loads of four bytes per thread and stages for tokens that are not there, took 90 us for 64 rows of 32 heads of 128 x 128
-// (268 MB, 3.0 TB/s), this ONE_US.  Every mode but the matrix memory.
+// (268 MB, 3.0 TB/s), this 49 (5.5 TB/s).  Every mode but the matrix memory.
 template <int DK, int MODE>
 __global__ void __launch_bounds__(256, 2)
 delta_step_kernel(const int* __restrict__ token_slot, const float* qn, const float* kn, const float* vv, const float* decay,
@@ -689,24 +690,69 @@ __device__ __forceinline__ void store4(bf16* p, float4 v) {
     *reinterpret_cast<uint2*>(p) = raw;
 }
 
+// The first `windows` of a token's blocks move the convolution's window (channels dealt to them), the others share its heads.  A
+// warp has four heads of up to 128 elements on their way at once: one head after the other, each read twice, took 47 us for
+// 2048 tokens of 32 heads of 128 (67 MB), this FINISH_US.
 template <typename T, typename TG>
 __global__ void delta_finish_vec_kernel(const float* o_raw, const TG* gate, int ldg, const float* __restrict__ weight,
                                         float eps, const int* __restrict__ token_slot, int n_rows, int heads, int dv,
                                         T* out, const T* proj, int ld, int channels, int taps, float* state,
                                         long long state_stride, long long tail_off, const float* den, int gate_act,
-                                        int weight_stride) {
+                                        int weight_stride, int windows) {
     TLLM_PDL_ENTER();
     const int t = blockIdx.x;
     const int slot = token_slot[t];
+    if ((int)blockIdx.y < windows) {
+        if (slot < 0 || (t + 1 < n_rows && token_slot[t + 1] == slot)) return;
+        const int quads = channels / 4, y = blockIdx.y;
+        move_window<T>(proj + (size_t)t * ld, ld, window_rows(token_slot, t, slot, taps - 1), taps - 1,
+                       state + (long long)slot * state_stride + tail_off, channels, quads * y / windows * 4, quads * (y + 1) / windows * 4, true);
+        return;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     if (slot < 0) {
         for (int e = threadIdx.x; e < heads * dv; e += blockDim.x) out[(size_t)t * heads * dv + e] = from_f32<T>(0.0f);
         return;
     }
-    const int Y = gridDim.y, yb = blockIdx.y;          // with few rows a token's heads and channels are dealt to gridDim.y blocks
-    for (int h = heads * yb / Y + warp; h < heads * (yb + 1) / Y; h += warps) {
+    const int Y = gridDim.y - windows, yb = blockIdx.y - windows;    // with few rows a token's heads are dealt to several blocks
+    const int h_end = heads * (yb + 1) / Y;
+    const bool divide = den != nullptr;
+    if (dv <= 128) {
+        constexpr int kHeads = 4;
+        const int e = lane * 4;
+        const bool in = e < dv;
+        for (int h0 = heads * yb / Y + warp; h0 < h_end; h0 += kHeads * warps) {
+            float4 v[kHeads], g[kHeads], w[kHeads];
+            float dn[kHeads];
+#pragma unroll
+            for (int i = 0; i < kHeads; ++i) {
+                const int h = h0 + i * warps;
+                const bool live = in && h < h_end;
+                v[i] = g[i] = w[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                dn[i] = 1.0f;
+                if (live) {
+                    v[i] = *reinterpret_cast<const float4*>(o_raw + ((size_t)t * heads + h) * dv + e);
+                    g[i] = load_gate4<TG>(gate + (size_t)t * ldg + (size_t)h * dv + e);
+                    w[i] = *reinterpret_cast<const float4*>(weight + (size_t)h * weight_stride + e);
+                    if (divide) dn[i] = den[(size_t)t * heads + h];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kHeads; ++i) {
+                const int h = h0 + i * warps;
+                if (divide) { v[i].x /= dn[i]; v[i].y /= dn[i]; v[i].z /= dn[i]; v[i].w /= dn[i]; }
+                const float sum = warp_sum(v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w);
+                const float sc = 1.0f / sqrtf(sum / (float)dv + eps);
+                if (in && h < h_end)
+                    store4(out + ((size_t)t * heads + h) * dv + e,
+                           make_float4(v[i].x * sc * w[i].x * finish_gate(g[i].x, gate_act), v[i].y * sc * w[i].y * finish_gate(g[i].y, gate_act),
+                                       v[i].z * sc * w[i].z * finish_gate(g[i].z, gate_act), v[i].w * sc * w[i].w * finish_gate(g[i].w, gate_act)));
+            }
+        }
+        return;
+    }
+    for (int h = heads * yb / Y + warp; h < h_end; h += warps) {
         const float* src = o_raw + ((size_t)t * heads + h) * dv;
-        const bool divide = den != nullptr;
         const float dn = divide ? den[(size_t)t * heads + h] : 1.0f;
         float sum = 0.0f;
         for (int e = lane * 4; e < dv; e += 128) {
@@ -721,25 +767,9 @@ __global__ void delta_finish_vec_kernel(const float* o_raw, const TG* gate, int 
             if (divide) { v.x /= dn; v.y /= dn; v.z /= dn; v.w /= dn; }
             const float4 g = load_gate4<TG>(gate + (size_t)t * ldg + (size_t)h * dv + e);
             const float4 w = *reinterpret_cast<const float4*>(weight + (size_t)h * weight_stride + e);
-            T* dst = out + ((size_t)t * heads + h) * dv + e;
-            store4(dst, make_float4(v.x * sc * w.x * finish_gate(g.x, gate_act), v.y * sc * w.y * finish_gate(g.y, gate_act),
-                                    v.z * sc * w.z * finish_gate(g.z, gate_act), v.w * sc * w.w * finish_gate(g.w, gate_act)));
-        }
-    }
-    if (taps > 1 && (t + 1 >= n_rows || token_slot[t + 1] != slot)) {
-        int len = 1;
-        while (len < taps - 1 && t - len >= 0 && token_slot[t - len] == slot) ++len;
-        float* tail = state + (long long)slot * state_stride + tail_off;
-        const int keep = taps - 1;
-        const int cc = channels / 8;
-        for (int c = (cc * yb / Y) * 8 + threadIdx.x * 8; c < (cc * (yb + 1) / Y) * 8; c += blockDim.x * 8) {
-            for (int i = 0; i < keep; ++i) {         // ascending: an old entry is read before its place is written
-                const int from_end = keep - i;
-                float x[8];
-                if (from_end <= len) Ld8<T>::load(proj + (size_t)(t + 1 - from_end) * ld + c, x);
-                else Ld8<float>::load(tail + (size_t)(i + len) * channels + c, x);
-                Ld8<float>::store(tail + (size_t)i * channels + c, x);
-            }
+            store4(out + ((size_t)t * heads + h) * dv + e,
+                   make_float4(v.x * sc * w.x * finish_gate(g.x, gate_act), v.y * sc * w.y * finish_gate(g.y, gate_act),
+                               v.z * sc * w.z * finish_gate(g.z, gate_act), v.w * sc * w.w * finish_gate(g.w, gate_act)));
         }
     }
 }
@@ -1255,11 +1285,12 @@ int tllm_delta_finish(const float* o_raw, const void* gate, int gate_f32, int ld
     const int sms_f = sm_count_cached() > 0 ? sm_count_cached() : 148;
     int split = 1;
     while (vec && split * 2 <= heads && (long long)n_rows * split < 2LL * sms_f) split *= 2;
+    const int windows = taps > 1 ? (split > 1 ? split : 2) : 0;      // blocks of a token that may have a window to move
 #define FIN(T, TG)                                                                                                         \
     do {                                                                                                                   \
         if (vec)                                                                                                           \
-            launch_pdl(kPdlOther, delta_finish_vec_kernel<T, TG>, dim3(n_rows, split), dim3(split > 1 ? 128 : 256), 0, stream, o_raw, (const TG*)gate, ldg, weight, eps, \
-                       token_slot, n_rows, heads, dv, (T*)out, (const T*)proj, ld, channels, taps, state, state_stride, tail_off, den, gate_act, weight_stride); \
+            launch_pdl(kPdlOther, delta_finish_vec_kernel<T, TG>, dim3(n_rows, windows + split), dim3(split > 1 ? 128 : 256), 0, stream, o_raw, (const TG*)gate, ldg, weight, eps, \
+                       token_slot, n_rows, heads, dv, (T*)out, (const T*)proj, ld, channels, taps, state, state_stride, tail_off, den, gate_act, weight_stride, windows); \
         else                                                                                                               \
             launch_pdl(kPdlOther, delta_finish_kernel<T, TG>, dim3(n_rows), dim3(256), 0, stream, o_raw, (const TG*)gate, ldg, weight, eps, \
                        token_slot, n_rows, heads, dv, (T*)out, (const T*)proj, ld, channels, taps, state, state_stride, tail_off, den, gate_act, weight_stride); \

@@ -19,6 +19,7 @@
 // request: S of every head in the scan's layout, then [taps - 1][channels] float32 inputs of the convolution,
 // the newest last.  Everything behind the projection is float32 in both storage types.
 #include "common.cuh"
+#include "conv_window.cuh"
 
 namespace tllm {
 
@@ -147,14 +148,22 @@ template <typename T, bool VEC>
 __global__ void ssd_finish_kernel(const float* o_raw, const float* xs, const float* __restrict__ skip_d, int P, const T* proj, int ld,
                                   const float* __restrict__ weight, float eps, int norm_groups,
                                   const int* __restrict__ token_slot, int n_rows, int inner, int channels, int taps,
-                                  float* state, long long state_stride, long long tail_off, T* out) {
+                                  float* state, long long state_stride, long long tail_off, T* out, int windows, int window_vec) {
     extern __shared__ __align__(16) float g[];   // the gated read-out of one norm part, per warp or for the block
     __shared__ float scratch[32];
     TLLM_PDL_ENTER();
     const int t = blockIdx.x;
     const int slot = token_slot[t];
-    const int part = inner / norm_groups;
-    const int p0 = norm_groups * blockIdx.y / gridDim.y, p1 = norm_groups * (blockIdx.y + 1) / gridDim.y;
+    if ((int)blockIdx.y < windows) {             // the first of a token's blocks move the window after a portion's last row
+        if (slot < 0 || (t + 1 < n_rows && token_slot[t + 1] == slot)) return;
+        const int quads = channels / 4, y = blockIdx.y;
+        move_window<T>(proj + (size_t)t * ld + inner, ld, window_rows(token_slot, t, slot, taps - 1), taps - 1,
+                       state + (long long)slot * state_stride + tail_off, channels, quads * y / windows * 4,
+                       y + 1 == windows ? channels : quads * (y + 1) / windows * 4, window_vec);
+        return;
+    }
+    const int part = inner / norm_groups, Y = gridDim.y - windows, yb = blockIdx.y - windows;
+    const int p0 = norm_groups * yb / Y, p1 = norm_groups * (yb + 1) / Y;
     if (slot < 0) {
         for (int e = p0 * part + threadIdx.x; e < p1 * part; e += blockDim.x) out[(size_t)t * inner + e] = from_f32<T>(0.0f);
         return;
@@ -203,23 +212,6 @@ __global__ void ssd_finish_kernel(const float* o_raw, const float* xs, const flo
         }
         if (by_warp) __syncwarp();
         else __syncthreads();                    // g is written again for the next part
-    }
-    // the portion's last row moves the convolution's window on: its taps - 1 newest inputs
-    if (taps > 1 && (t + 1 >= n_rows || token_slot[t + 1] != slot)) {
-        int len = 1;                                 // rows of the portion, as far as the window reaches
-        while (len < taps - 1 && t - len >= 0 && token_slot[t - len] == slot) ++len;
-        float* tail = state + (long long)slot * state_stride + tail_off;
-        const int keep = taps - 1;
-        const int c0 = (int)((long long)channels * blockIdx.y / gridDim.y), c1 = (int)((long long)channels * (blockIdx.y + 1) / gridDim.y);
-        for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-            for (int i = 0; i < keep; ++i) {         // ascending: an old entry is read before its place is written
-                const int from_end = keep - i;       // this entry is the from_end-th newest input
-                float x;
-                if (from_end <= len) x = to_f32<T>(proj[(size_t)(t + 1 - from_end) * ld + inner + c]);
-                else x = tail[(size_t)(i + len) * channels + c];
-                tail[(size_t)i * channels + c] = x;
-            }
-        }
     }
 }
 
@@ -296,15 +288,17 @@ int tllm_ssd_finish(const float* o_raw, const float* xs, const float* skip_d, in
     TLLM_REQUIRE(smem <= 200 * 1024, "ssd_finish: parts of %d do not fit in shared memory", part);
     const auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const bool vec = part % 8 == 0 && P % 8 == 0 && ld % 8 == 0 && al(o_raw) && al(xs) && al(proj) && al(weight) && al(out);
+    const int windows = taps > 1 ? (split > 2 ? split : 2) : 0;      // blocks of a token that may have a window to move
+    const int window_vec = channels % 4 == 0 && ld % 4 == 0 && inner % 4 == 0 && tail_off % 4 == 0 && state_stride % 4 == 0 && al(state) && al(proj);
 #define FIN(T, V)                                                                                                   \
     do {                                                                                                            \
         if (smem > 48 * 1024) {                                                                                     \
             cudaError_t e = cudaFuncSetAttribute(ssd_finish_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             if (e != cudaSuccess) { set_error("ssd_finish: %s", cudaGetErrorString(e)); return (int)e; }            \
         }                                                                                                           \
-        launch_pdl(kPdlOther, ssd_finish_kernel<T, V>, dim3(n_rows, split), dim3(256), smem, stream, o_raw, xs,     \
+        launch_pdl(kPdlOther, ssd_finish_kernel<T, V>, dim3(n_rows, windows + split), dim3(256), smem, stream, o_raw, xs, \
                    skip_d, P, (const T*)proj, ld, weight, eps, norm_groups, token_slot, n_rows, inner, channels, taps, state,  \
-                   state_stride, tail_off, (T*)out);                                                                \
+                   state_stride, tail_off, (T*)out, windows, window_vec);                                           \
     } while (0)
     if (dtype == kBF16) { if (vec) FIN(bf16, true); else FIN(bf16, false); }
     else if (dtype == kF32) { if (vec) FIN(float, true); else FIN(float, false); }
