@@ -692,7 +692,7 @@ __device__ __forceinline__ void store4(bf16* p, float4 v) {
 
 // The first `windows` of a token's blocks move the convolution's window (channels dealt to them), the others share its heads.  A
 // warp has four heads of up to 128 elements on their way at once: one head after the other, each read twice, took 47 us for
-// 2048 tokens of 32 heads of 128 (67 MB), this FINISH_US.
+// 2048 tokens of 32 heads of 128 (67 MB), this 35 (64 rows of one token: 9.4 to 6.7).
 template <typename T, typename TG>
 __global__ void delta_finish_vec_kernel(const float* o_raw, const TG* gate, int ldg, const float* __restrict__ weight,
                                         float eps, const int* __restrict__ token_slot, int n_rows, int heads, int dv,
