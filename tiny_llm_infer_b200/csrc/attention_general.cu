@@ -23,7 +23,7 @@ __global__ void paged_attention_general_kernel(
     const T* q, const T* cache, const int* __restrict__ positions,
     const int* __restrict__ token_slot, const int* __restrict__ block_table, int max_pages,
     int page_size, int q_heads, int kv_heads, int head_dim, int window, float scale,
-    T* __restrict__ out) {
+    const int* __restrict__ rows, T* __restrict__ out) {
     extern __shared__ float smem[];
     TLLM_PDL_ENTER();
     float* qs = smem;                          // [head_dim]
@@ -31,7 +31,7 @@ __global__ void paged_attention_general_kernel(
     float* m_s = acc_s + kWarps * head_dim;    // [kWarps]
     float* l_s = m_s + kWarps;                 // [kWarps]
 
-    const int head = blockIdx.x, t = blockIdx.y;
+    const int head = blockIdx.x, t = rows != nullptr ? rows[blockIdx.y] : blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     T* dst = out + ((size_t)t * q_heads + head) * head_dim;
     const int slot = token_slot[t];
@@ -105,14 +105,14 @@ template <typename T>
 static int launch_general(const void* q, const void* cache, const int* positions,
                           const int* token_slot, const int* block_table, int max_pages,
                           int page_size, int tokens, int q_heads, int kv_heads, int head_dim,
-                          int window, float scale, void* out, cudaStream_t stream) {
+                          int window, float scale, const int* rows, void* out, cudaStream_t stream) {
     const dim3 grid(q_heads, tokens), block(kWarps * 32);
     const size_t smem = ((size_t)head_dim * (1 + kWarps) + 2 * kWarps) * sizeof(float);
     const int chunks = (head_dim + 31) / 32;
 #define LAUNCH(C)                                                                              \
     launch_pdl(kPdlAttention, paged_attention_general_kernel<T, C>, grid, block, smem, stream,                 \
         (const T*)q, (const T*)cache, positions, token_slot, block_table, max_pages, page_size, \
-        q_heads, kv_heads, head_dim, window, scale, (T*)out)
+        q_heads, kv_heads, head_dim, window, scale, rows, (T*)out)
     if (chunks <= 1) LAUNCH(1);
     else if (chunks <= 2) LAUNCH(2);
     else if (chunks <= 4) LAUNCH(4);
@@ -126,10 +126,11 @@ static int launch_general(const void* q, const void* cache, const int* positions
 
 using namespace tllm;
 
+// rows: the `tokens` rows to do (null: all, tokens of them).
 extern "C" int tllm_paged_attention_general(
     const void* q, const void* cache, const int* positions, const int* token_slot,
     const int* block_table, int max_pages, int page_size, int dtype, int tokens, int q_heads,
-    int kv_heads, int head_dim, int window, float scale, void* out, cudaStream_t stream) {
+    int kv_heads, int head_dim, int window, float scale, const int* rows, void* out, cudaStream_t stream) {
     TLLM_REQUIRE(tokens >= 0 && q_heads > 0 && kv_heads > 0 && q_heads % kv_heads == 0,
                  "paged_attention: %d query heads over %d key/value heads", q_heads, kv_heads);
     TLLM_REQUIRE(head_dim > 0 && head_dim <= 512, "paged_attention: head_dim %d outside 1..512", head_dim);
@@ -138,9 +139,9 @@ extern "C" int tllm_paged_attention_general(
     if (tokens == 0) return 0;
     if (dtype == kBF16)
         return launch_general<bf16>(q, cache, positions, token_slot, block_table, max_pages, page_size,
-                                    tokens, q_heads, kv_heads, head_dim, window, scale, out, stream);
+                                    tokens, q_heads, kv_heads, head_dim, window, scale, rows, out, stream);
     if (dtype == kF32)
         return launch_general<float>(q, cache, positions, token_slot, block_table, max_pages, page_size,
-                                     tokens, q_heads, kv_heads, head_dim, window, scale, out, stream);
+                                     tokens, q_heads, kv_heads, head_dim, window, scale, rows, out, stream);
     TLLM_REQUIRE(false, "paged_attention: unknown dtype %d", dtype);
 }

@@ -112,7 +112,8 @@ def _declare(h) -> None:
                                     i32, i32, i32, i32, i32, i32, vp, vp],
         "tllm_rope_table": [vp, vp, i32, i32, vp, vp],
         "tllm_paged_attention_general": [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32,
-                                         i32, f32, vp, vp],
+                                         i32, f32, vp, vp, vp],
+        "tllm_paged_attention_f32": [vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, f32, vp, vp],
         "tllm_sample": [vp, i32, i32, i64, vp, vp, vp, vp],
         "tllm_sample_split": [vp, i32, i32, i64, vp, vp, vp, vp, i32, vp, vp],
         "tllm_gemm_skinny": [vp, vp, vp, i32, i32, i32, i32, vp],
@@ -475,7 +476,8 @@ def paged_attention(q: torch.Tensor, cache: torch.Tensor, positions, token_slot,
     positions max(0, pos - window + 1) .. pos.  With the step's context and a shape the
     tensor-core kernels take (bfloat16, head width 64 or 128, pages of a multiple of 16),
     one-token rows go to the split-key decode kernel and longer segments to the tiled
-    prefill kernel; everything else runs the general kernel."""
+    prefill kernel; in float32 at those widths longer segments go to tiles on the float32 pipe;
+    everything else runs the general kernel."""
     _cuda(q, cache, positions, token_slot, block_table, out)
     tokens = q.shape[0]
     assert tuple(cache.shape[1:]) == (2, kv_heads, page_size, head_dim) and cache.dtype == q.dtype
@@ -498,10 +500,20 @@ def paged_attention(q: torch.Tensor, cache: torch.Tensor, positions, token_slot,
                 paged_attention_prefill(q, cache, ctx.seg_info, ctx.pf_tiles, ctx.n_tiles, block_table,
                                         page_size, q_heads, kv_heads, head_dim, window, scale, out)
         return out
-    _check(lib().tllm_paged_attention_general(
-        _p(q), _p(cache), _p(positions), _p(token_slot), _p(block_table), block_table.shape[1],
-        page_size, _dt(q), tokens, q_heads, kv_heads, head_dim, int(window or 0), float(scale),
-        _p(out), _stream()), "paged_attention")
+    rows, n = None, tokens
+    if ctx is not None and ctx.pf_tiles is not None and ctx.tokens == tokens and 0 < ctx.n_tiles <= 65535 \
+            and q.dtype == torch.float32 and head_dim in (64, 128) \
+            and (q.data_ptr() | cache.data_ptr() | out.data_ptr()) % 16 == 0:
+        # float32 portions: tiles of 64 rows; what is left are the one-token rows
+        _check(lib().tllm_paged_attention_f32(
+            _p(q), _p(cache), _p(ctx.seg_info), _p(ctx.pf_tiles), ctx.n_tiles, _p(block_table), block_table.shape[1], page_size,
+            q_heads, kv_heads, head_dim, int(window or 0), float(scale), _p(out), _stream()), "paged_attention_f32")
+        rows, n = ctx.dec_rows, ctx.n_dec
+    if n:
+        _check(lib().tllm_paged_attention_general(
+            _p(q), _p(cache), _p(positions), _p(token_slot), _p(block_table), block_table.shape[1],
+            page_size, _dt(q), n, q_heads, kv_heads, head_dim, int(window or 0), float(scale), _p(rows),
+            _p(out), _stream()), "paged_attention")
     return out
 
 
