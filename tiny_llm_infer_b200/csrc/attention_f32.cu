@@ -3,7 +3,7 @@
 //
 // The general kernel (attention_general.cu) gives every (token, head) a block that reads all its keys and values again, a dot
 // product per warp and key with a reduction for each: two prompts of 300 tokens with 16 heads on 8 of 128 took 250 us, this
-// F32_US.  Here a thread owns 8 rows x 4 keys of the scores and 8 rows x HD / 16 columns of the output, so that a value read
+// 76.  Here a thread owns 8 rows x 4 keys of the scores and 8 rows x HD / 16 columns of the output, so that a value read
 // from shared memory serves four to eight products (packed, two per instruction; a score's even and odd elements are summed
 // apart).  What bounds it is that pipe and the shared memory's reads, about equally, and with few tiles the longest block.
 //
