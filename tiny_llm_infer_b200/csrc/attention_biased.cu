@@ -876,11 +876,6 @@ static int launch_biased_prefill(const void* q, const void* kp, const void* vp, 
 // With two maps a tile's rows are the group's heads for the first map, then the same heads for the second; a row's
 // query is its map's half of a vector as wide as a row of keys (both maps' keys side by side), the other half zeros,
 // so that one product serves both maps and keys and values are still read once.
-// What bounds it is the keys' and values' way from HBM, so two blocks per multiprocessor (registers) hold three stages each:
-// 64 rows of 32 heads on 8 at contexts of 1300 to 2000 took 133 us with two stages, block-wide barriers and the block table
-// looked up in front of every copy (3.2 TB/s); now DECODE_US.
-__host__ __device__ constexpr int dec_stages(int maps) { return maps == 1 ? 3 : 2; }
-
 template <int DKP, int DVP, int MAPS>
 __global__ void __launch_bounds__(kPfWarps * 32, 2)
 attention_biased_decode_kernel(const bf16* q, const bf16* k_plane, const bf16* v_plane, long long page_stride,
@@ -952,59 +947,49 @@ attention_biased_decode_kernel(const bf16* q, const bf16* k_plane, const bf16* v
     }
     float l_lo = (first && (lane & 3) == 0) ? 1.0f : 0.0f, l_hi = l_lo;
 
-    // A warp copies and reads its own sixteen keys of a tile, so that no warp waits for another.  Lane l looks up the page of
-    // key l % 16 a tile ahead of its copies.
-    auto lookup = [&](int kt) -> int {
-        const int key = kt * kPfN + warp * 16 + (lane & 15);
-        int page_index, place;
-        page_of(key, page_size, page_shift, page_index, place);
-        return (kt <= kt_last && key <= pos && key >= lo) ? table[page_index] : -1;
-    };
-    auto issue = [&](int kt, int stage, int pages) {
+    auto issue = [&](int kt, int stage) {
         const uint32_t ks = smem_u32(pf_smem + (size_t)stage * (kKBytes + kVBytes));
         const uint32_t vs = ks + kKBytes;
         constexpr int kMC = DKP / 8, kKC = MAPS * kMC, kVC = DVP / 8;       // 16-byte pieces of a map's key, a row of keys, a value
-        constexpr int kKRows = 32 / kKC, kVRows = 32 / kVC;                 // rows per instruction
-#pragma unroll
-        for (int i = 0; i < 16 / kKRows; ++i) {
-            const int r = i * kKRows + lane / kKC, chunk = lane % kKC, row = warp * 16 + r;
-            const int page = __shfl_sync(0xffffffffu, pages, r);
+        for (int row = threadIdx.x / kKC, chunk = threadIdx.x % kKC; row < kPfN; row += kPfWarps * 32 / kKC) {
+            const int key = kt * kPfN + row;
             int page_index, place;
-            page_of(kt * kPfN + row, page_size, page_shift, page_index, place);
-            const int in_key = (chunk % kMC) * 8;                           // within its map's key
-            const bool k_ok = page >= 0 && in_key < dk;
-            cp_async_16(ks + (row * kKRow + chunk * 8) * 2,
-                        k_plane + (k_ok ? (long long)page * page_stride + ((long long)g * page_size + place) * kd + (chunk / kMC) * dk + in_key : 0), k_ok);
+            page_of(key, page_size, page_shift, page_index, place);
+            const int page = (key <= pos && key >= lo) ? table[page_index] : -1;
+            const bool ok = page >= 0;
+            const long long page_at = ok ? (long long)page * page_stride : 0;
+            const long long in_page = (long long)g * page_size + place;
+            const int in_key = (chunk % kMC) * 8;                       // within its map's key
+            const bool k_ok = ok && in_key < dk;
+            cp_async_16(ks + (row * kKRow + chunk * 8) * 2, k_plane + (k_ok ? page_at + in_page * kd + (chunk / kMC) * dk + in_key : 0), k_ok);
+            if (kKC == kVC) {
+                const bool v_ok = ok && chunk * 8 < dv;
+                cp_async_16(vs + (row * kVRow + chunk * 8) * 2, v_plane + (v_ok ? page_at + in_page * v_row + chunk * 8 : 0), v_ok);
+            }
         }
-#pragma unroll
-        for (int i = 0; i < 16 / kVRows; ++i) {
-            const int r = i * kVRows + lane / kVC, chunk = lane % kVC, row = warp * 16 + r;
-            const int page = __shfl_sync(0xffffffffu, pages, r);
-            int page_index, place;
-            page_of(kt * kPfN + row, page_size, page_shift, page_index, place);
-            const bool v_ok = page >= 0 && chunk * 8 < dv;
-            cp_async_16(vs + (row * kVRow + chunk * 8) * 2,
-                        v_plane + (v_ok ? (long long)page * page_stride + ((long long)g * page_size + place) * v_row + chunk * 8 : 0), v_ok);
+        if (kKC != kVC) {
+            for (int row = threadIdx.x / kVC, chunk = threadIdx.x % kVC; row < kPfN; row += kPfWarps * 32 / kVC) {
+                const int key = kt * kPfN + row;
+                int page_index, place;
+                page_of(key, page_size, page_shift, page_index, place);
+                const int page = (key <= pos && key >= lo) ? table[page_index] : -1;
+                const bool v_ok = page >= 0 && chunk * 8 < dv;
+                cp_async_16(vs + (row * kVRow + chunk * 8) * 2, v_plane + (v_ok ? (long long)page * page_stride + ((long long)g * page_size + place) * v_row + chunk * 8 : 0), v_ok);
+            }
         }
         cp_async_commit();
     };
 
-    constexpr int kAhead = dec_stages(MAPS) - 1;                        // tiles on their way while one is read
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i) {
-        if (kt_first + i <= kt_last) issue(kt_first + i, i, lookup(kt_first + i));
-        else cp_async_commit();
-    }
-    int pages = lookup(kt_first + kAhead);
-    for (int kt = kt_first, stage = 0; kt <= kt_last; ++kt, stage = stage == kAhead ? 0 : stage + 1) {
-        if (kt + kAhead <= kt_last) {
-            issue(kt + kAhead, stage == 0 ? kAhead : stage - 1, pages);
-            pages = lookup(kt + kAhead + 1);
+    if (kt_first <= kt_last) issue(kt_first, 0);
+    for (int kt = kt_first; kt <= kt_last; ++kt) {
+        const int stage = (kt - kt_first) & 1;
+        if (kt + 1 <= kt_last) {
+            issue(kt + 1, stage ^ 1);
+            cp_async_wait<1>();
         } else {
-            cp_async_commit();
+            cp_async_wait<0>();
         }
-        cp_async_wait<kAhead>();
-        __syncwarp();
+        __syncthreads();
         const int key0 = kt * kPfN + warp * 16;                          // this warp's 16 keys of the tile
         if (key0 <= pos && key0 + 15 >= lo) {
             const uint32_t ks_base = smem_u32(pf_smem + (size_t)stage * (kKBytes + kVBytes));
@@ -1077,9 +1062,8 @@ attention_biased_decode_kernel(const bf16* q, const bf16* k_plane, const bf16* v
                 mma_bf16_16816(o[c + 1], pa, b1);
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
-    __syncthreads();                                                   // the staging buffers are written over below
     l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
     l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
     l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
@@ -1223,7 +1207,7 @@ static int launch_biased_decode(const void* q, const void* kp, const void* vp, l
                                 const int* block_table, int max_pages, int page_size, int q_heads, int kv_heads,
                                 int dk, int dv, ScoreMod mod, DiffMod diff, const float* slopes, const float* sink_logit, int v_row,
                                 const void* gate, int gate_stride, int splits, float* part, void* out, cudaStream_t stream) {
-    const size_t smem = (size_t)dec_stages(MAPS) * kPfN * ((MAPS * DKP + kPfPad) + (DVP + kPfPad)) * 2;      // also holds the warps' meeting
+    const size_t smem = (size_t)2 * kPfN * ((MAPS * DKP + kPfPad) + (DVP + kPfPad)) * 2;      // also holds the warps' meeting
     static OncePerDevice configured;
     if (configured.first()) {
         cudaError_t e = cudaFuncSetAttribute(attention_biased_decode_kernel<DKP, DVP, MAPS>,
