@@ -479,21 +479,14 @@ static int launch_chunks(const int* seg_info, int segments, int rows, const floa
 
 using namespace tllm;
 
-// Floats of `pairs` for a step of `rows` tokens in `segments` portions.
-extern "C" long long tllm_chunk_scan_floats(int rows, int segments, int heads) {
-    return ((long long)rows / kC + segments) * heads * kPairFloats;
-}
-
-// Whether the kernels here take keys of width dk and values of width dv.
-extern "C" int tllm_chunk_scan_ok(int dk, int dv) { return (dk == 64 || dk == 128) && dv > 0 && dv % 16 == 0; }
-
 // The recurrences of tllm_delta_scan by chunks: modes 0 (delta rule), 1 (decay per channel), 3 (decay per token and head), 5
-// (constant decay per head), with that entry's operands.  qn, kn, vv, decay and pairs on 16-byte boundaries.
+// (constant decay per head), with that entry's operands.  pairs
+// float[(rows / 16 + segments) * heads * 512].  qn, kn, vv, decay and pairs on 16-byte boundaries.
 extern "C" int tllm_chunk_scan(const int* seg_info, int segments, int rows, const float* qn, const float* kn, const float* vv,
                                const float* decay, const float* beta, const float* fgate, float* pairs, float* state,
                                long long state_stride, int heads, int kv_heads, int dk, int dv, float* o_raw, int mode, cudaStream_t stream) {
     TLLM_REQUIRE(segments >= 0 && rows >= 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0, "chunk_scan: bad sizes");
-    TLLM_REQUIRE(tllm_chunk_scan_ok(dk, dv), "chunk_scan: keys of %d, values of %d", dk, dv);
+    TLLM_REQUIRE((dk == 64 || dk == 128) && dv > 0 && dv % 16 == 0, "chunk_scan: keys of %d, values of %d", dk, dv);
     TLLM_REQUIRE(segments <= 65535, "chunk_scan: %d portions", segments);
     const auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     TLLM_REQUIRE(al(qn) && al(kn) && al(vv) && al(decay) && al(pairs), "chunk_scan: operands must be 16-byte aligned");

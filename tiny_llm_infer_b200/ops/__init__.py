@@ -82,6 +82,7 @@ def _declare(h) -> None:
         "tllm_delta_prepare": [vp, i32, i32, vp, vp, i32, vp, i32, vp, vp, vp, vp, i64, i32, i32, i32, i32, f32, f32,
                                vp, vp, vp, vp, vp, i32, i32, i32, vp],
         "tllm_delta_scan": [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, vp, i32, vp, vp, i64, f32, vp, vp],
+        "tllm_chunk_scan": [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, vp, i32, vp],
         "tllm_erase_prepare": [vp, i32, i32, i32, vp, i32, vp, vp, f32, vp, i32, i32, i32, f32, vp, vp, vp, vp, vp, i32, vp],
         "tllm_stream_read": [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, f32, vp, i32, vp, vp, vp, i64, i32, vp, vp, i32, i32, i32, vp],
         "tllm_stream_tails": [vp, i32, vp, i32, vp, i64, i32, vp],
@@ -130,14 +131,10 @@ def _declare(h) -> None:
                                              i32, i32, i32, f32, vp, i32, vp, f32, i32, i32, vp, vp, i32, i32, vp, i32, vp,
                                              vp, vp, vp],
     }
-    sigs["tllm_chunk_scan"] = [vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, vp, i32, vp]
-    sigs["tllm_chunk_scan_ok"] = [i32, i32]
     for name, args in sigs.items():
         fn = getattr(h, name)
         fn.argtypes = args
         fn.restype = i32
-    h.tllm_chunk_scan_floats.argtypes = [i32, i32, i32]
-    h.tllm_chunk_scan_floats.restype = i64
     h.tllm_delta_rule_lanes.argtypes = [i32]
     h.tllm_delta_rule_lanes.restype = i32
     h.tllm_delta_rule_state_floats.argtypes = [i32, i32, i32, i32, i32]
@@ -1027,19 +1024,24 @@ def delta_rule_state_floats(heads: int, kv_heads: int, dk: int, dv: int, taps: i
 
 SCAN_DELTA, SCAN_PLAIN, SCAN_MEMORY, SCAN_HEAD_DECAY, SCAN_ERASE, SCAN_FIXED_DECAY = 0, 1, 2, 3, 4, 5     # recurrences of the scan kernel (csrc/delta_rule.cu, ScanMode)
 CHUNK_MODES = (SCAN_DELTA, SCAN_PLAIN, SCAN_HEAD_DECAY, SCAN_FIXED_DECAY)      # that csrc/chunk_scan.cu knows
-CHUNK_TOKENS = 64         # tokens per portion, on average, from which on the recurrences run by chunks (and in a step of half as
-                          # many again: a second kernel and less work per token break even at 64 to 96 tokens of one portion;
-                          # the delta rule with 32 heads of 128 x 128: 64 tokens 26 us against 24, 128 tokens 36 against 42,
-                          # eight portions of 32 tokens 53 against 54, of 64 tokens 80 against 99)
+# Tokens per portion, on average, from which on the recurrences run by chunks if the step is large (64 * 32768 tokens x heads x
+# key elements), and from two and a half times which on in any case.  Token by token a portion takes a quarter of a
+# microsecond per token whatever else there is, and a step of many portions or heads as long as its work; by chunks there
+# are two kernels and less work.  The delta rule with 32 heads of 128 x 128: one portion of 64 tokens 24 us against 26, of 256 77
+# against 56; eight of 32 tokens 54 against 53, of 64 99 against 80.  Between the lines both take some 40 us, and the second
+# launch costs more than it saves (four portions of 90 tokens, 16 heads of 64 x 128: the whole op 40 us against 48).
+CHUNK_TOKENS = 64
 
 
 def _scan(mode, seg_info, tokens, token_slot, qn, kn, vv, decay, beta, state, heads, kv_heads, dk, cols, o_raw, fgate=None,
           erase=None, aux_off=0, floor_eps=0.0, den=None) -> None:
     """The recurrence itself: by chunks of sixteen tokens for prompt portions, else token by token."""
     segments = tokens if seg_info is None else seg_info.shape[0]
-    if seg_info is not None and mode in CHUNK_MODES and 0 < segments <= 65535 and 2 * tokens >= CHUNK_TOKENS * max(2 * segments, 3) \
-            and lib().tllm_chunk_scan_ok(dk, cols):
-        pairs = torch.empty(lib().tllm_chunk_scan_floats(tokens, segments, heads), dtype=torch.float32, device=qn.device)
+    if seg_info is not None and mode in CHUNK_MODES and 0 < segments <= 65535 and tokens >= CHUNK_TOKENS * segments \
+            and (2 * tokens >= 5 * CHUNK_TOKENS * segments or tokens * heads * dk >= CHUNK_TOKENS << 15) \
+            and dk in (64, 128) and cols % 16 == 0:
+        # T and Q T of every chunk and head: a chunk of sixteen tokens at most per sixteen rows and one more per portion
+        pairs = torch.empty((tokens // 16 + segments) * heads * 512, dtype=torch.float32, device=qn.device)
         _check(lib().tllm_chunk_scan(_p(seg_info), segments, tokens, _p(qn), _p(kn), _p(vv), _p(decay), _p(beta), _p(fgate),
                                      _p(pairs), _p(state), state.stride(0), heads, kv_heads, dk, cols, _p(o_raw), mode, _stream()),
                "chunk_scan", kernels=2)
