@@ -164,13 +164,14 @@ def _check(code: int, what: str, kernels: int = 1) -> None:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream() -> int:
     """Handle of the current CUDA stream of the current device (the raw getter costs a fraction
     of a microsecond, the Stream object several)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_raw_device())             # (there are CUDA tensors: nothing is left to initialise)
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -1037,7 +1038,7 @@ def _scan(mode, seg_info, tokens, token_slot, qn, kn, vv, decay, beta, state, he
           erase=None, aux_off=0, floor_eps=0.0, den=None) -> None:
     """The recurrence itself: by chunks of sixteen tokens for prompt portions, else token by token."""
     segments = tokens if seg_info is None else seg_info.shape[0]
-    if seg_info is not None and mode in CHUNK_MODES and 0 < segments <= 65535 and tokens >= CHUNK_TOKENS * segments \
+    if seg_info is not None and tokens >= CHUNK_TOKENS * segments and mode in CHUNK_MODES and 0 < segments <= 65535 \
             and (2 * tokens >= 5 * CHUNK_TOKENS * segments or tokens * heads * dk >= CHUNK_TOKENS << 15) \
             and dk in (64, 128) and cols % 16 == 0:
         # T and Q T of every chunk and head: a chunk of sixteen tokens at most per sixteen rows and one more per portion
