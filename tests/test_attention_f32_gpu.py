@@ -53,3 +53,13 @@ def test_tiles_are_the_general_kernel(hd, heads, kv_heads, page, window, lengths
     tiled, general = ((o - want).norm() / want.norm() for o in out)
     # both sum in float32; the tiles may not be further off than the general kernel but for a few roundings of 2^-24
     assert tiled <= 1.5 * general + 2.0 ** -23, (float(tiled), float(general))
+    # a token's key and value reach no row before it, whatever they are
+    for s, first, n, p0 in seg:
+        if n > 1:
+            at = p0 + n - 1
+            cache[table[s, at // page].long(), :, :, at % page] = float("nan") if s else float("inf")
+    o = torch.empty_like(q)
+    ops.paged_attention(q, cache, ctx.positions, ctx.token_slot, table, page, heads, kv_heads, hd, window or None, hd ** -0.5, o, ctx=ctx)
+    last = torch.zeros(row, dtype=torch.bool, device=DEV)
+    last[[first + n - 1 for _, first, n, _ in seg if n > 1]] = True
+    assert torch.equal(o.double()[~last], out[0][~last])

@@ -98,6 +98,13 @@ def test_chunks_are_the_recurrence(mode, heads, kv_heads, dk, dv, lengths, monke
         if slots[s] >= 0:
             idle[starts[s]:starts[s] + lengths[s]] = False
     assert (o[idle] == 0).all()                                    # nothing is written for the others
+    # a token reaches no read-out before it, whatever its values are
+    last = [starts[s] + lengths[s] - 1 for s in range(n) if slots[s] >= 0 and lengths[s]]
+    v[last[::2]], v[last[1::2]] = float("nan"), float("inf")
+    o2, _ = run(True)
+    kept = torch.ones(tokens, dtype=torch.bool, device=DEV)
+    kept[last] = False
+    assert torch.equal(o2[kept], o[kept])
 
 
 @pytest.mark.parametrize("mode", ["delta", "channel", "head", "fixed", "erase"])

@@ -136,8 +136,7 @@ paged_attention_f32_kernel(const float* q, const float* cache, const int* __rest
                     make_float4(p[4 * h][i], p[4 * h + 1][i], p[4 * h + 2][i], p[4 * h + 3][i]);
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // the values; the next keys may still be coming
         __syncthreads();
-#pragma unroll 4
-        for (int j = 0; j < kTN; ++j) {
+        auto meet = [&](int j, int row0, int row1) {            // key j with the thread's rows that see it
             const float4 pa = *reinterpret_cast<const float4*>(p_s + j * L::kPRow + ty * 8);
             const float4 pb = *reinterpret_cast<const float4*>(p_s + j * L::kPRow + ty * 8 + 4);
             const float w[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
@@ -146,10 +145,22 @@ paged_attention_f32_kernel(const float* q, const float* cache, const int* __rest
                 const float4 v4 = *reinterpret_cast<const float4*>(v_s + j * HD + 64 * c + 4 * tx);
 #pragma unroll
                 for (int r = 0; r < 8; ++r) {
+                    if (r < row0 || r > row1) continue;
                     const float2 w2 = make_float2(w[r], w[r]);
                     o[r][2 * c] = __ffma2_rn(w2, make_float2(v4.x, v4.y), o[r][2 * c]);
                     o[r][2 * c + 1] = __ffma2_rn(w2, make_float2(v4.z, v4.w), o[r][2 * c + 1]);
                 }
+            }
+        };
+        if (whole) {
+#pragma unroll 4
+            for (int j = 0; j < kTN; ++j) meet(j, 0, 7);
+        } else {
+            // a key that a row does not see is left out, not weighted by zero: its value may be infinite or no number
+            const int pos = first_pos + ty * 8, lo = first_key(pos);
+            for (int j = max(0, lo - key0); j < kTN && key0 + j <= pos + 7; ++j) {
+                const int key = key0 + j;
+                meet(j, key - pos, window > 0 ? key + window - 1 - pos : 7);
             }
         }
         __syncthreads();                                        // values and weights have been read

@@ -342,6 +342,8 @@ chunk_scan_kernel(const int* __restrict__ seg_info, const float* qn, const float
         const float* T = s + L::kT;
         const float* Qm = s + L::kQm;
         const float* vcol = s + L::kV + warp * kWide + myc;
+        // token j's value as the lane's m-th token sees it: a later one not at all, be it infinite or no number
+        auto before = [&](float x, int j, int m) -> float { return j >= kGroup * m && j > kGroup * m + tr ? 0.0f : x; };
         float o[NL];
         if (kCorr) {
 #pragma unroll
@@ -358,8 +360,9 @@ chunk_scan_kernel(const int* __restrict__ seg_info, const float* qn, const float
                     if (kGroup * (m + 1) <= j) continue;        // T and Q T are zero above their diagonals
                     const float4 t4 = *reinterpret_cast<const float4*>(T + (kGroup * m + tr) * kPad + j);
                     const float4 q4 = *reinterpret_cast<const float4*>(Qm + (kGroup * m + tr) * kPad + j);
-                    u[m] = fmaf(t4.x, x0, fmaf(t4.y, x1, fmaf(t4.z, x2, fmaf(t4.w, x3, u[m]))));
-                    o[m] = fmaf(q4.x, x0, fmaf(q4.y, x1, fmaf(q4.z, x2, fmaf(q4.w, x3, o[m]))));
+                    const float y0 = before(x0, j, m), y1 = before(x1, j + 1, m), y2 = before(x2, j + 2, m), y3 = before(x3, j + 3, m);
+                    u[m] = fmaf(t4.x, y0, fmaf(t4.y, y1, fmaf(t4.z, y2, fmaf(t4.w, y3, u[m]))));
+                    o[m] = fmaf(q4.x, y0, fmaf(q4.y, y1, fmaf(q4.z, y2, fmaf(q4.w, y3, o[m]))));
                 }
             }
 #pragma unroll
@@ -380,7 +383,8 @@ chunk_scan_kernel(const int* __restrict__ seg_info, const float* qn, const float
                 for (int m = 0; m < NL; ++m) {
                     if (kGroup * (m + 1) <= j) continue;
                     const float4 q4 = *reinterpret_cast<const float4*>(Qm + (kGroup * m + tr) * kPad + j);
-                    o[m] = fmaf(q4.x, y[0], fmaf(q4.y, y[1], fmaf(q4.z, y[2], fmaf(q4.w, y[3], o[m]))));
+                    o[m] = fmaf(q4.x, before(y[0], j, m), fmaf(q4.y, before(y[1], j + 1, m),
+                           fmaf(q4.z, before(y[2], j + 2, m), fmaf(q4.w, before(y[3], j + 3, m), o[m]))));
                 }
             }
             __syncwarp();
