@@ -712,14 +712,14 @@ BIASED_FAST = True       # False: every row takes the general kernel (for compar
 def biased_decode_splits(rows: int, kv_heads: int, reach: int) -> int:
     """Runs of keys per (row, key/value head) of ``attention_biased``'s one-token kernel, by the time its grid takes: whole rounds
     of the blocks that are resident at once (two per multiprocessor), each as long as a run's tiles of 64 keys and some three
-    more for its start and end; more than one run costs the kernel that adds them.  A run keeps at least 192 keys of the
+    more for its start and end; more than one run costs the kernel that adds them, as long as three tiles.  A run keeps at least 192 keys of the
     ``reach`` a row can see.  (Enough runs for two blocks per multiprocessor, whatever the last round: 8 rows of 8 key/value
     heads at context 2000 38 us, now 30; 16 rows at 4000 102, now 84; 48 rows at 4000 233, now 181.)"""
     tiles, resident = -(-reach // 64), 2 * SM_COUNT
     best, least = 1, None
     for splits in range(1, max(1, min(reach // 192, 64)) + 1):
         rounds = -(-rows * kv_heads * splits // resident)
-        cost = rounds * (-(-tiles // splits) + 3) + (1 if splits > 1 else 0)
+        cost = rounds * (-(-tiles // splits) + 3) + (3 if splits > 1 else 0)
         if least is None or cost < least:
             best, least = splits, cost
     return best
