@@ -342,30 +342,17 @@ chunk_scan_kernel(const int* __restrict__ seg_info, const float* qn, const float
         const float* T = s + L::kT;
         const float* Qm = s + L::kQm;
         const float* vcol = s + L::kV + warp * kWide + myc;
+        // token j's value as the lane's m-th token sees it: a later one not at all, be it infinite or no number (the delta
+        // rule's whole mixer at 2048 tokens: 510 us, 482 without; the other recurrences take no longer)
+        auto before = [&](float x, int j, int m) -> float { return j >= kGroup * m && j > kGroup * m + tr ? 0.0f : x; };
         float o[NL];
         if (kCorr) {
-            bool odd = false;
 #pragma unroll
-            for (int m = 0; m < NL; ++m) {
-                xk[m] = vcol[(kGroup * m + tr) * COLS] - xk[m];
-                xs[(kGroup * m + tr) * kWide + myc] = xk[m];
-                odd |= !(fabsf(xk[m]) < INFINITY);
-            }
-            odd = __any_sync(0xffffffffu, odd);
+            for (int m = 0; m < NL; ++m) xs[(kGroup * m + tr) * kWide + myc] = vcol[(kGroup * m + tr) * COLS] - xk[m];
             __syncwarp();
             float u[NL];
 #pragma unroll
             for (int m = 0; m < NL; ++m) o[m] = xq[m], u[m] = 0.0f;
-            if (odd) {
-                // zeros above the diagonals do not keep such a value away from the tokens before it
-#pragma unroll
-                for (int m = 0; m < NL; ++m)
-#pragma unroll 1
-                    for (int j = 0; j <= kGroup * m + tr; ++j) {
-                        u[m] = fmaf(T[(kGroup * m + tr) * kPad + j], xs[j * kWide + myc], u[m]);
-                        o[m] = fmaf(Qm[(kGroup * m + tr) * kPad + j], xs[j * kWide + myc], o[m]);
-                    }
-            } else
 #pragma unroll
             for (int j = 0; j < kC; j += 4) {
                 const float x0 = xs[j * kWide + myc], x1 = xs[(j + 1) * kWide + myc], x2 = xs[(j + 2) * kWide + myc], x3 = xs[(j + 3) * kWide + myc];
@@ -374,8 +361,9 @@ chunk_scan_kernel(const int* __restrict__ seg_info, const float* qn, const float
                     if (kGroup * (m + 1) <= j) continue;        // T and Q T are zero above their diagonals
                     const float4 t4 = *reinterpret_cast<const float4*>(T + (kGroup * m + tr) * kPad + j);
                     const float4 q4 = *reinterpret_cast<const float4*>(Qm + (kGroup * m + tr) * kPad + j);
-                    u[m] = fmaf(t4.x, x0, fmaf(t4.y, x1, fmaf(t4.z, x2, fmaf(t4.w, x3, u[m]))));
-                    o[m] = fmaf(q4.x, x0, fmaf(q4.y, x1, fmaf(q4.z, x2, fmaf(q4.w, x3, o[m]))));
+                    const float y0 = before(x0, j, m), y1 = before(x1, j + 1, m), y2 = before(x2, j + 2, m), y3 = before(x3, j + 3, m);
+                    u[m] = fmaf(t4.x, y0, fmaf(t4.y, y1, fmaf(t4.z, y2, fmaf(t4.w, y3, u[m]))));
+                    o[m] = fmaf(q4.x, y0, fmaf(q4.y, y1, fmaf(q4.z, y2, fmaf(q4.w, y3, o[m]))));
                 }
             }
 #pragma unroll
@@ -387,8 +375,6 @@ chunk_scan_kernel(const int* __restrict__ seg_info, const float* qn, const float
                 o[m] = xq[m] * T[kGroup * m + tr];
                 us[(kGroup * m + tr) * kWide + myc] = T[kPad + kGroup * m + tr] * vcol[(kGroup * m + tr) * COLS];
             }
-            // token j's value as the lane's m-th token sees it: a later one not at all, be it infinite or no number
-            auto before = [&](float x, int j, int m) -> float { return j >= kGroup * m && j > kGroup * m + tr ? 0.0f : x; };
 #pragma unroll
             for (int j = 0; j < kC; j += 4) {
                 float y[4];
