@@ -107,6 +107,46 @@ def test_chunks_are_the_recurrence(mode, heads, kv_heads, dk, dv, lengths, monke
     assert torch.equal(o2[kept], o[kept])
 
 
+@pytest.mark.parametrize("by_chunks", [True, False])
+@pytest.mark.parametrize("mode,operands", [("delta", "q k v decay beta"), ("channel", "q k v decay beta"), ("channel, no weights", "q k v decay"),
+                                           ("head", "q k v beta fgate"), ("fixed", "q k v")])
+@pytest.mark.parametrize("heads,kv_heads,dk,dv", [(4, 2, 128, 128), (40, 40, 64, 64)])      # two columns per lane and four
+@pytest.mark.parametrize("odd", [float("nan"), float("inf")])
+def test_an_odd_token_reaches_no_read_out_before_it(by_chunks, mode, operands, heads, kv_heads, dk, dv, odd, monkeypatch):
+    """One token of every portion has an infinity or a NaN in one operand; what is read out before it stays bit for bit."""
+    from tiny_llm_infer_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(11)
+    lengths, at = (50, 16, 37), (21, 15, 36)                       # inside a chunk, a chunk's last, a portion's last
+    starts = [0, 50, 66]
+    tokens = sum(lengths)
+    seg = torch.tensor([[s, starts[s], lengths[s], 0] for s in range(3)], dtype=torch.int32, device=DEV)
+    q, k = (torch.nn.functional.normalize(torch.randn(tokens, kv_heads, dk, generator=g, device=DEV), dim=-1) for _ in range(2))
+    v, S0 = torch.randn(tokens, heads, dv, generator=g, device=DEV), torch.randn(3, heads, dk, dv, generator=g, device=DEV)
+    rand = {n: torch.rand(*shape, generator=g, device=DEV) for n, shape in
+            (("decay", (tokens, heads, dk)), ("beta", (tokens, heads)), ("fgate", (tokens, heads)), ("fixed", (heads,)))}
+    clean = {"q": q, "k": k, "v": v, "decay": rand["decay"] if "decay" in operands else None,
+             "beta": rand["beta"] if "beta" in operands else None, "fgate": rand["fixed"] if mode == "fixed" else rand["fgate"] if mode == "head" else None}
+    code = {"delta": ops.SCAN_DELTA, "head": ops.SCAN_HEAD_DECAY, "fixed": ops.SCAN_FIXED_DECAY}.get(mode, ops.SCAN_PLAIN)
+    monkeypatch.setattr(ops, "CHUNK_TOKENS", 1 if by_chunks else 1 << 30)
+
+    def run(t):
+        state, o, before = pack(S0), torch.zeros(tokens, heads, dv, device=DEV), ops.launches
+        ops._scan(code, seg, tokens, None, t["q"], t["k"], t["v"], t["decay"], t["beta"], state, heads, kv_heads, dk, dv, o, fgate=t["fgate"])
+        assert ops.launches - before == (2 if by_chunks else 1)
+        return o
+    want = run(clean)
+    assert torch.isfinite(want).all()
+    kept = torch.ones(tokens, dtype=torch.bool, device=DEV)
+    for s in range(3):
+        kept[starts[s] + at[s]:starts[s] + lengths[s]] = False
+    for name in operands.split():
+        spoilt = clean[name].clone()
+        spoilt[[starts[s] + at[s] for s in range(3)]] = odd
+        got = run({**clean, name: spoilt})
+        assert torch.equal(got[kept], want[kept]), name
+        assert not torch.isfinite(got[[starts[s] + at[s] for s in range(3)]]).all(), name
+
+
 @pytest.mark.parametrize("mode", ["delta", "channel", "head", "fixed", "erase"])
 @pytest.mark.parametrize("rows", [1, 5, 70])
 @pytest.mark.parametrize("heads,kv_heads,dk,dv", [(4, 2, 128, 128), (3, 3, 64, 24), (2, 2, 128, 200), (6, 6, 64, 128)])

@@ -150,7 +150,8 @@ chunk_pairs_kernel(const int* __restrict__ seg_info, int segments, const float* 
                 } else if (lane == 0) {
                     T[i] = 1.0f;
                 }
-                if (lane < 16) Q[i * kC + col] = s * w_own;
+                // of a later token nothing, not zero times its weight: that may be infinite or no number
+                if (lane < 16) Q[i * kC + col] = col <= i ? s * w_own : 0.0f;
             }
         }
         // row 1: what token j's values are multiplied by in the state, its weight and the decays after it
