@@ -199,7 +199,8 @@ class LLMEngine:
         current = self._flying.pop(0)
         plan = current.plan
         tokens = self.sampler.fetch(current.ticket)
-        self.runner.check_kernels()
+        # a step that samples has been waited for; one that does not is, as all that was launched is
+        self.runner.check_kernels(current.step if current.rows else None)
         sampled = [-1] * len(plan.sequences)
         generated = 0
         for idx, tok in zip(current.row_of, tokens):

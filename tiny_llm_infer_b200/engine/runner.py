@@ -84,6 +84,7 @@ class PreparedStep:
     ctx: Optional[StepContext] = None             # the general path's context
     graph_key: Optional[Tuple[int, int]] = None   # (rows bucket, context bucket) of a one-token step
     wanted: Optional[List[int]] = None            # rows wanted of a one-token step
+    bounded: bool = False                         # once run: it launched kernels with bounded waits
 
 
 class ModelRunner:
@@ -102,6 +103,7 @@ class ModelRunner:
         self._graph_pool = None
         self._prompt_pool = None
         self._capture_stream = None
+        self._check_stream = None
         self._prompt_graphs: dict = {}
         self._prompt_seen: dict = {}
         self._graph_logits: Optional[torch.Tensor] = None
@@ -120,10 +122,19 @@ class ModelRunner:
         self._uploaded: Optional[torch.cuda.Event] = None
         self._prepared: Optional[PreparedStep] = None      # the host buffer holds this step
 
-    def check_kernels(self) -> None:
+    def check_kernels(self, step: Optional[PreparedStep] = None) -> None:
         """Raise if a kernel with bounded waits gave up since the last check (reads a device
-        word: call it where the host waits for the step anyway)."""
-        if self.is_cuda and ops.tcgen05_calls != self._checked_calls:
+        word: call it where the host waits for the step anyway).  ``step``: only if that step, which
+        has been waited for, launched any; steps launched after it are not waited for."""
+        if not self.is_cuda:
+            return
+        if step is not None:
+            if step.bounded:
+                if self._check_stream is None:
+                    self._check_stream = torch.cuda.Stream(device=self.device)
+                with torch.cuda.stream(self._check_stream):
+                    ops.check_error_word(self.device)
+        elif ops.tcgen05_calls != self._checked_calls:
             self._checked_calls = ops.tcgen05_calls
             ops.check_error_word(self.device)
 
@@ -279,6 +290,7 @@ class ModelRunner:
                     raise StepError(f"request {e.request!r}: token id outside [0, {self.vocab})")
                 host[place] = int(token)
                 e.tokens[e.late] = int(token)          # what commit() hashes
+        calls = ops.tcgen05_calls
         self._upload(words)
         if late_source is not None and n_late:
             d, at = self._dev, prepared.upload
@@ -291,6 +303,7 @@ class ModelRunner:
                 logits = self.model.forward(prepared.ctx, self.cache)
             else:
                 logits = self._step_prompt_graph(signature, prepared.ctx)
+        prepared.bounded = ops.tcgen05_calls != calls
         for request, length, tokens in prepared.commits:
             self.cache.commit(request, length, tokens)
         return logits
@@ -427,9 +440,10 @@ class ModelRunner:
         key, rows, wanted = prepared.graph_key, len(prepared.entries), prepared.wanted
         if key not in self._graphs:
             self._capture(key)
-        graph, kernels = self._graphs[key]
+        graph, kernels, tc_calls = self._graphs[key]
         graph.replay()
         ops.launches += kernels                      # the replay launches what the capture recorded
+        ops.tcgen05_calls += tc_calls                # and check_kernels has to look at the waits of every replay
         logits = self._graph_logits
         if wanted == list(range(rows)):
             return logits[:rows]
@@ -479,11 +493,10 @@ class ModelRunner:
             rows = min(self.GRAPH_MAX_ROWS, self.max_batch_tokens)
             self._graph_logits = torch.empty((rows, self.vocab), dtype=torch.float32, device=self.device)
         graph = torch.cuda.CUDAGraph()
-        before = ops.launches
+        launches, tc_calls = ops.launches, ops.tcgen05_calls
         with self._capturing(graph, self._graph_pool):
             # the result goes to a buffer of the runner's own, so that the graphs' private
             # memory can be shared between them
             self._graph_logits[:bucket].copy_(self.model.forward(ctx, self.cache))
-        kernels = ops.launches - before
-        ops.launches = before                        # capturing launches nothing
-        self._graphs[key] = (graph, kernels)
+        self._graphs[key] = (graph, ops.launches - launches, ops.tcgen05_calls - tc_calls)
+        ops.launches, ops.tcgen05_calls = launches, tc_calls  # capturing launches nothing
