@@ -71,3 +71,51 @@ def test_changes_of_the_score_and_the_output(form, heads, kv_heads, lengths, bef
     bound = 3 * 2.0 ** -8 * planes[1].abs().max().item()
     assert (out[0] - out[1]).abs().max().item() <= bound
     assert ((out[0] - out[1]).norm() / out[1].norm()).item() <= 2.0 ** -7       # roundings are not all of one sign
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+@pytest.mark.parametrize("heads,kv_heads,lengths,befores", [
+    (4, 2, (130, 2, 257), (0, 333, 61)), (3, 3, (300,), (17,)), (2, 1, (65,), (1500,)),
+])
+def test_odd_values_reach_only_the_rows_that_see_them(form, heads, kv_heads, lengths, befores):
+    """Infinities and NaN in values of a portion, in an old one, and in what another request left behind the last token: where
+    results are finite and what they are is as in the general kernel, which looks at a row's own keys only."""
+    from tiny_llm_infer_b200 import ops
+    f = dict(FORMS[form])
+    g = torch.Generator(device=DEV).manual_seed(6)
+
+    def randn(*shape):
+        return torch.randn(*shape, generator=g, device=DEV)
+    ctx = context(lengths, befores)
+    pages = -(-ctx.max_context // PAGE)
+    order = torch.randperm(len(lengths) * pages, generator=g, device=DEV).to(torch.int32).view(len(lengths), pages)
+    keys, values = (randn(len(lengths) * pages, kv_heads, PAGE, D).bfloat16() for _ in range(2))
+    largest = values.abs().max().item()
+    for s, (n, p0) in enumerate(zip(lengths, befores)):
+        def value(pos):
+            return values[order[s, pos // PAGE].long(), :, pos % PAGE]
+        value(p0 + n // 2)[0, 5] = float("inf")
+        value(p0 + n - 1)[:, 77] = float("nan")
+        value(p0 // 3)[:, 9] = -float("inf")
+        for pos in range(p0 + n, -(-(p0 + n) // PAGE) * PAGE):
+            value(pos)[:] = float("nan")
+            keys[order[s, pos // PAGE].long(), :, pos % PAGE] = float("nan")
+    q = randn(ctx.tokens, heads * D).bfloat16()
+    per_head = f.get("gate") == "heads"
+    gate = randn(ctx.tokens, heads if per_head else heads * D).bfloat16() if f.get("gate") else None
+    kw = dict(softcap=f.get("softcap", 0.0), chunk=f.get("chunk", 0), window=f.get("window", 0), sink=f.get("sink", False),
+              slopes=torch.rand(heads, generator=g, device=DEV) * 0.05 if f.get("slopes") else None, gate=gate,
+              gate_per_head=per_head, sink_logits=randn(heads) if f.get("learned") else None)
+    out = []
+    for c in (ctx, None):
+        o, before = torch.empty_like(q), ops.tcgen05_calls
+        ops.attention_biased(q, keys, values, ctx.positions, ctx.token_slot, order, PAGE, heads, kv_heads, D, D, D ** -0.5, o, ctx=c, **kw)
+        assert (ops.tcgen05_calls > before) == (c is not None)
+        out.append(o.double())
+    ops.check_error_word(q.device)
+    finite = torch.isfinite(out[1])
+    assert finite.float().mean() > 0.9 and not finite.all()
+    assert torch.equal(torch.isfinite(out[0]), finite)
+    got, want = out[0][finite], out[1][finite]
+    assert (got - want).abs().max().item() <= 3 * 2.0 ** -8 * largest          # as above
+    assert ((got - want).norm() / want.norm()).item() <= 2.0 ** -7

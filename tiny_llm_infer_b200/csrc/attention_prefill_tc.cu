@@ -187,15 +187,16 @@ struct QTile {
 // 2 scale / cap and cap_out = cap, both times log2(e); else s scale.  slopes [q_heads] (or null): s - slope * distance.
 // chunk > 0: keys of the query's own chunk of positions only.  sink: exp(sink_logit[head]), one without logits, joins the
 // denominator.  gate (or null): the output times sigmoid of it, [tokens] rows `gate_stride` apart with a number per element
-// or, `gate_per_head`, per query head; gate_vec: its rows allow 16-byte accesses.
+// or, `gate_per_head`, per query head; gate_vec: its rows allow 16-byte accesses.  q: the queries as they lie in memory.
 struct Changes {
     float cap_in, cap_out;
     int chunk, sink;
     const float* slopes;
     const bf16* gate;
     int gate_stride, gate_per_head, gate_vec;
+    const bf16* q;
 };
-constexpr Changes kNoChanges{0.0f, 0.0f, 0, 0, nullptr, nullptr, 0, 0, 0};
+constexpr Changes kNoChanges{0.0f, 0.0f, 0, 0, nullptr, nullptr, 0, 0, 0, nullptr};
 enum ScoreForm : int { kPlain = 0, kBiased = 1, kChanged = 2 };
 
 __device__ __forceinline__ float rcp(float x) {
@@ -204,6 +205,82 @@ __device__ __forceinline__ float rcp(float x) {
     return y;
 }
 __device__ __forceinline__ float sigmoid_of(bf16 g) { return 1.0f / (1.0f + expf(-__bfloat162float(g))); }
+
+__device__ __forceinline__ float4 four_of(const bf16* p) {      // on an 8-byte boundary
+    const uint2 raw = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ uint32_t odd_of(float4 v) {          // bit e: element e is infinite or no number
+    return (isfinite(v.x) ? 0u : 1u) | (isfinite(v.y) ? 0u : 2u) | (isfinite(v.z) ? 0u : 4u) | (isfinite(v.w) ? 0u : 8u);
+}
+
+// A row whose O came out infinite or no number though the sum of its weights is a number.  The matrix products weigh the keys
+// of a tile that the row does not see by zero, and zero times an infinite value is no number; such a value may be a later
+// token's, one behind the window, or what an earlier request left in the last page.  The warp looks at those keys, and where
+// their values are the cause and not the row's own keys', goes through the row's keys one by one: 32 lanes, four columns each.
+// A row with finite values never comes here; one with odd values of its own leaves after its masked keys (at most a tile of
+// rows and keys) have been looked at.
+struct OddRow {
+    const bf16 *q, *k, *v;                 // the row's query; keys and values of its head
+    const int* table;
+    int rows_per_page, page_size;
+    int pos, lo;                           // it sees the keys lo .. pos
+    int k0, k1, last;                      // the block's tiles hold the keys [k0, k1), as far as the 16-key group of `last`
+    float cap_in, cap_out, scale_log2e, slope2;
+};
+__device__ __noinline__ bool odd_row(const OddRow& a, float4& o, float& m, float& l) {
+    const int lane = threadIdx.x & 31;
+    auto row_of = [&](int key) -> long long {                   // of the planes; -1: nothing was loaded
+        const int page = a.table[key / a.page_size];
+        return page < 0 ? -1 : (long long)page * a.rows_per_page + key % a.page_size;
+    };
+    auto odd_at = [&](int key) -> uint32_t {
+        const long long row = row_of(key);
+        return row < 0 ? 0u : odd_of(four_of(a.v + row * kHD + lane * 4));
+    };
+    uint32_t hidden = 0;
+    for (int key = a.k0; key < min(a.lo, a.k1); ++key) hidden |= odd_at(key);
+    for (int key = max(a.k0, a.pos + 1); key < a.k1 && (key & ~15) <= a.last; ++key) hidden |= odd_at(key);
+    const int first = max(a.lo, a.k0), end = min(a.pos + 1, a.k1);
+    if (first < end) hidden &= ~(odd_at(end - 1));
+    if (!__any_sync(0xffffffffu, hidden != 0)) return false;
+    const float4 q = four_of(a.q + lane * 4);
+    o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    m = -INFINITY, l = 0.0f;
+    for (int key0 = first; key0 < end; key0 += 4) {
+        float dot[4];
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const long long row = key0 + i < end ? row_of(key0 + i) : -1;
+            v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            dot[i] = 0.0f;
+            if (row >= 0) {
+                const float4 k = four_of(a.k + row * kHD + lane * 4);
+                v[i] = four_of(a.v + row * kHD + lane * 4);
+                dot[i] = q.x * k.x + q.y * k.y + q.z * k.z + q.w * k.w;
+            }
+        }
+#pragma unroll
+        for (int x = 16; x > 0; x >>= 1)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dot[i] += __shfl_xor_sync(0xffffffffu, dot[i], x);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (key0 + i >= end) break;
+            float score = a.cap_in > 0.0f ? fmaf(-2.0f * a.cap_out, rcp(ex2(dot[i] * a.cap_in) + 1.0f), a.cap_out) : dot[i] * a.scale_log2e;
+            score = fmaf(-a.slope2, (float)(a.pos - key0 - i), score);
+            const float top = fmaxf(m, score), use = top == -INFINITY ? 0.0f : top, f = ex2(m - use), w = ex2(score - use);
+            m = top;
+            l = fmaf(l, f, w);
+            o.x = fmaf(w, v[i].x, o.x * f); o.y = fmaf(w, v[i].y, o.y * f);
+            o.z = fmaf(w, v[i].z, o.z * f); o.w = fmaf(w, v[i].w, o.w * f);
+        }
+    }
+    return true;
+}
 
 // Keys and values lie in planes of their own: row (page * rows_per_page + head * page_size + place in the
 // page) of 128 elements from `k_base` and from `v_base` (the two halves of a page of the plain cache, or two
@@ -625,6 +702,8 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
             else asm volatile("bar.sync 2, 128;\n" ::: "memory");
         }
         const bool finish = alive && !__any_sync(0xffffffffu, *aborted != 0);
+        const float l_keys = l_run;                             // without a sink
+        float odd = 0.0f;                                       // no number where O has an infinity or none
         if (finish && splits > 1) {
             // ---- one of several runs of keys: O as it stands, its reference maximum and its sum
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -634,6 +713,9 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                 uint32_t o[32];
                 tmem_ld32(tmem_ox + c, o);
                 tmem_ld_wait();
+                if (kChange)
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) odd = fmaf(__uint_as_float(o[e]), 0.0f, odd);
                 if (r < t.rows) {
                     uint4* dst = reinterpret_cast<uint4*>(part_o + index * kHD + c);
 #pragma unroll
@@ -661,6 +743,9 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                 uint32_t o[32];
                 tmem_ld32(tmem_ox + c, o);
                 tmem_ld_wait();
+                if (kChange)
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) odd = fmaf(__uint_as_float(o[e]), 0.0f, odd);
                 if (kChange && gate_row != nullptr) {
                     if (ch.gate_vec) {
 #pragma unroll
@@ -700,6 +785,37 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                                  : "r"(stage + rr * 256 + ((c ^ (rr & 15)) << 4)));
                     *reinterpret_cast<uint4*>(out + ((size_t)(start + t.q_off + rr) * q_heads + t.head) * kHD + c * 8) = val;
                 }
+            }
+        }
+        if (kChange && finish) {
+            __syncwarp();                                       // what follows is written over what the warp has stored above
+            uint32_t rows = __ballot_sync(0xffffffffu, r < t.rows && !(odd == 0.0f) && isfinite(l_keys));
+            for (; rows != 0; rows &= rows - 1) {
+                const int rr = quad * 32 + __ffs(rows) - 1;
+                const size_t token = start + t.q_off + rr;
+                const long long head_row = (long long)g * page_size;
+                const OddRow a{ch.q + (token * q_heads + t.head) * kHD, k_base + head_row * kHD, v_base + head_row * kHD,
+                               block_table + (size_t)slot * max_pages, rows_per_page, page_size, t.first_pos + rr,
+                               first_key(t.first_pos + rr), t.kt_first * kBN, (t.kt_first + t.n) * kBN, last_pos,
+                               ch.cap_in, ch.cap_out, scale_log2e, slope2};
+                float4 o;
+                float m, l;
+                if (!odd_row(a, o, m, l)) continue;
+                if (splits > 1) {
+                    const size_t index = part_index(t, rr);
+                    *reinterpret_cast<float4*>(part_o + index * kHD + lane * 4) = o;
+                    if (lane == 0) part_ml[index * 2] = m, part_ml[index * 2 + 1] = l;
+                    continue;
+                }
+                if (sink_logit != nullptr) l += ex2(sink_logit[t.head] * kLog2e - m);
+                else if (ch.sink) l += ex2(-m);
+                const float inv = 1.0f / l;
+                float gate[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+                if (ch.gate != nullptr)
+                    for (int e = 0; e < 4; ++e)
+                        gate[e] = sigmoid_of(ch.gate[token * ch.gate_stride + (ch.gate_per_head ? t.head : t.head * kHD + lane * 4 + e)]);
+                *reinterpret_cast<uint2*>(out + (token * q_heads + t.head) * kHD + lane * 4) =
+                    make_uint2(pack2(o.x * inv * gate[0], o.y * inv * gate[1]), pack2(o.z * inv * gate[2], o.w * inv * gate[3]));
             }
         }
     }
@@ -879,7 +995,7 @@ extern "C" int tllm_attention_planes_prefill_tc(
     TLLM_REQUIRE(!changed || dist_bias == nullptr, "attention_planes_prefill_tc: a table of biases comes alone");
     const pftc::Changes ch{softcap > 0.0f ? 2.0f * scale / softcap * pftc::kLog2e : 0.0f, softcap * pftc::kLog2e, chunk, sink, slopes,
                            (const bf16*)gate, gate_stride, gate_per_head,
-                           gate_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(gate) & 15u) == 0};
+                           gate_stride % 8 == 0 && (reinterpret_cast<uintptr_t>(gate) & 15u) == 0, (const bf16*)q};
     return launch_prefill_tc("attention_planes_prefill_tc", q, tokens, k_plane, v_plane, page_stride / 128,
                              (long long)num_pages * (page_stride / 128), seg_info, tiles, n_tiles, block_table,
                              max_pages, page_size, q_heads, kv_heads, window, scale, dist_bias, dist_len, sink_logit,
