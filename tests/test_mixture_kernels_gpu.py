@@ -87,3 +87,33 @@ def test_combine_adds_the_choices(width, top, y_dtype, identity):
     own = torch.where((ids >= real)[..., None], x.double()[:, None], own)
     want = shared.double() * torch.sigmoid(logit.double())[:, None] + (weights.double()[..., None] * own).sum(1)
     assert ((got - want).abs() <= (2.0 ** -8 + 1e-6) * want.abs() + 1e-5).all()
+
+
+@pytest.mark.parametrize("rows", [9, 40])
+def test_rows_off_the_16_byte_grid(rows):
+    """The part takes rows that start anywhere (9 rows and more: fewer are refused by the router's product), on the kernels that
+    look at the alignment; the lists' own product refuses them on the host."""
+    from tiny_llm_infer_b200 import ops
+    from tiny_llm_infer_b200.parts import lookup
+    width, experts, top, inter = 64, 6, 2, 48
+    g = torch.Generator(device=DEV).manual_seed(5)
+    part = lookup("feed_forward", "moe")(width, experts, top, inter, torch.bfloat16, DEV)
+    part.load({name: (torch.randn(*spec.shape, generator=g, device=DEV) * 0.2).bfloat16()
+               for name, spec in part.param_specs(width, experts, top, inter).items()})
+    x = torch.randn(rows, width, generator=g, device=DEV).bfloat16()
+    off = torch.zeros(rows * width + 3, dtype=torch.bfloat16, device=DEV)[3:].view(rows, width)
+    off.copy_(x)
+    assert off.data_ptr() % 16 and off.is_contiguous()
+    before = ops.tcgen05_calls
+    got = part.forward(off, None).double()
+    assert ops.tcgen05_calls == before
+    want = part.forward(x, None).double()
+    assert ops.tcgen05_calls == before + 2
+    ops.check_error_word(torch.device(DEV))
+    # both round the units' outputs and the result to bfloat16 (2^-9 of each, root mean square less)
+    assert ((got - want).norm() / want.norm()).item() <= 2.0 ** -8
+    plan = ops.MoePlan(torch.zeros(rows, 1, dtype=torch.int32, device=DEV), experts, 64, tensor_memory=True)
+    with pytest.raises(ops.KernelError, match="aligned"):
+        ops.moe_grouped(off, part.w_gate_up, plan, 1, gated=True, gather=True, interleaved=True)
+    with pytest.raises(ops.KernelError, match="aligned"):
+        ops.moe_grouped(off, part.w_gate_up, plan, 1, gated=True, gather=False, interleaved=True)

@@ -639,6 +639,7 @@ int tllm_moe_grouped(const void* A, int lda, const int* src_of, const float* wei
 int tllm_moe_gather(const void* x, const int* src_of, const float* weight_of, int top, void* xs, int rows, int width,
                     cudaStream_t stream) {
     TLLM_REQUIRE(rows >= 0 && width > 0 && width % 8 == 0 && top > 0, "moe_gather: bad sizes");
+    TLLM_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(xs)) & 15u) == 0, "moe_gather: rows must be 16-byte aligned");
     const size_t chunks = (size_t)rows * (width / 8);
     if (chunks == 0) return 0;
     size_t g = (chunks + 255) / 256;

@@ -152,7 +152,8 @@ class MixtureOfExperts:
             ids, weights = ops.moe_route(z, self.top, softmax_weights=self.router_scores == "softmax")
         rows = ids.numel()
         w_first = self.w_gate_up if self.gated else self.w_up
-        tensor_cores = (self.interleaved or not self.gated) and x.dtype == w_first.dtype \
+        # rows that do not start on a 16-byte boundary (a view into something else) stay with the kernels that look at that
+        tensor_cores = (self.interleaved or not self.gated) and x.dtype == w_first.dtype and x.data_ptr() % 16 == 0 \
             and ops.moe_tcgen05_pays(rows, self.experts, self.inter, self.hidden, x.dtype)
         plan = ops.MoePlan(ids, self.experts + self.identity, ops.moe_row_box(rows, self.experts) if tensor_cores else None,
                            real=self.experts, tensor_memory=tensor_cores)
