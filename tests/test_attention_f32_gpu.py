@@ -63,3 +63,30 @@ def test_tiles_are_the_general_kernel(hd, heads, kv_heads, page, window, lengths
     last = torch.zeros(row, dtype=torch.bool, device=DEV)
     last[[first + n - 1 for _, first, n, _ in seg if n > 1]] = True
     assert torch.equal(o.double()[~last], out[0][~last])
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+def test_portions_of_no_request_become_zero(hd):
+    from tiny_llm_infer_b200 import ops
+    from tiny_llm_infer_b200.engine.batch import StepContext
+    lengths, slots, heads, kv_heads, page = (70, 40, 1), (-1, 0, -1), 4, 2, 16
+
+    def ints(v):
+        return torch.tensor(v, dtype=torch.int32, device=DEV)
+    rows = sum(lengths)
+    ctx = StepContext(tokens=rows, token_ids=None, positions=ints([i for n in lengths for i in range(n)]),
+                      token_slot=ints([s for s, n in zip(slots, lengths) for _ in range(n)]), want_rows=None, segments=[],
+                      seg_info=ints([[-1, 0, 70, 0], [0, 70, 40, 0], [-1, 110, 1, 0]]), dec_rows=ints([110]), n_dec=1,
+                      pf_tiles=ints([(0, 0), (0, 64), (1, 0)]), n_tiles=3, max_context=70, max_segment=70)
+    g = torch.Generator(device=DEV).manual_seed(8)
+    table = ints([[2, 0, 1]])
+    cache = torch.randn(3, 2, kv_heads, page, hd, generator=g, device=DEV)
+    q = torch.randn(rows, heads * hd, generator=g, device=DEV)
+    out = []
+    for c in (ctx, None):
+        o = torch.full_like(q, float("nan"))
+        ops.paged_attention(q, cache, ctx.positions, ctx.token_slot, table, page, heads, kv_heads, hd, None, hd ** -0.5, o, ctx=c)
+        out.append(o)
+    for o in out:
+        assert (o[:70] == 0).all() and (o[110:] == 0).all()
+    assert torch.allclose(out[0][70:110], out[1][70:110], rtol=1e-5, atol=1e-5)

@@ -37,7 +37,12 @@ paged_attention_f32_kernel(const float* q, const float* cache, const int* __rest
     const int seg = tiles[2 * blockIdx.y], q_off = tiles[2 * blockIdx.y + 1], head = blockIdx.x;
     const int slot = seg_info[4 * seg], start = seg_info[4 * seg + 1], len = seg_info[4 * seg + 2], pos0 = seg_info[4 * seg + 3];
     const int rows_here = min(kTM, len - q_off), first_pos = pos0 + q_off, last_pos = first_pos + rows_here - 1;
-    if (slot < 0 || rows_here <= 0) return;
+    if (rows_here <= 0) return;
+    if (slot < 0) {                                             // rows of no request, as in the general kernel
+        for (int i = threadIdx.x; i < rows_here * HD; i += kF32Threads)
+            out[((size_t)(start + q_off + i / HD) * q_heads + head) * HD + i % HD] = 0.0f;
+        return;
+    }
     const int g = head / (q_heads / kv_heads);
     const int* table = block_table + (size_t)slot * max_pages;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;     // keys tx + 16 i, rows 8 ty + r
