@@ -1,5 +1,6 @@
 """The rules by which the kernel wrappers size their grids and choose a product: pure
 functions of the sizes, checked without a GPU."""
+import pytest
 import torch
 
 from tiny_llm_infer_b200 import ops
@@ -33,3 +34,18 @@ def test_the_tcgen05_product_is_chosen_where_its_tiles_fill_the_gpu():
     assert not ops.tcgen05_pays(2048, 6144, 4096, bf)            # 8 x 24 tiles: a ragged second round
     assert not ops.tcgen05_pays(64, 4096, 4096, bf) and not ops.tcgen05_pays(2048, 4096, 4096, torch.float32)
     assert not ops.tcgen05_pays(2048, 4096, 4100, bf)            # K no multiple of 8
+
+
+@pytest.mark.parametrize("mode,segments,each,heads,dk,cols,chunks", [
+    # (recurrence, portions, tokens of each, heads, key elements, value columns): measured to be faster by chunks, or not
+    ("delta", 1, 2048, 32, 128, 128, True), ("delta", 8, 256, 64, 128, 128, True), ("delta", 1, 2048, 32, 64, 128, True),
+    ("delta", 3, 701, 32, 64, 128, True), ("delta", 4, 256, 32, 64, 128, False), ("delta", 12, 701, 64, 64, 64, False),
+    ("delta", 6, 256, 64, 128, 16, False), ("delta", 4, 256, 16, 64, 256, False), ("plain", 8, 256, 64, 64, 16, False),
+    ("plain", 8, 256, 32, 64, 64, False), ("plain", 8, 256, 32, 128, 64, True), ("plain", 8, 256, 32, 64, 128, True),
+    ("head", 8, 256, 64, 64, 64, True), ("head", 12, 256, 64, 64, 16, False), ("head", 1, 1023, 64, 128, 64, True),
+    ("fixed", 3, 701, 32, 128, 128, True), ("fixed", 8, 160, 32, 64, 64, False), ("fixed", 4, 90, 16, 64, 128, False),
+    ("delta", 1, 64, 32, 128, 128, False), ("delta", 8, 64, 32, 128, 128, True), ("delta", 64, 2, 32, 128, 128, False),
+])
+def test_recurrences_go_by_chunks_where_that_is_faster(mode, segments, each, heads, dk, cols, chunks):
+    code = {"delta": ops.SCAN_DELTA, "plain": ops.SCAN_PLAIN, "head": ops.SCAN_HEAD_DECAY, "fixed": ops.SCAN_FIXED_DECAY}[mode]
+    assert ops.chunks_pay(code, segments, segments * each, heads, dk, cols) == chunks

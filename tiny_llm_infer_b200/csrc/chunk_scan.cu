@@ -470,9 +470,9 @@ static int launch_chunks(const int* seg_info, int segments, int rows, const floa
         seg_info, segments, qn, kn, decay, beta, fgate, heads, kv_heads, pairs);
     if (int rc = finish_launch("chunk_pairs")) return rc;
     // Blocks of 32 columns, four per lane, read the tokens' rows from shared memory least often, which is what bounds a full grid
-    // (2048 tokens of 32 heads of 128 x 128, delta rule, with the pairs: 353 us; two per lane 378, blocks of 16 columns 485 and
-    // 404).  Where they would leave a quarter of the multiprocessors without a block, 16 columns, two per lane (16 heads: 227 us
-    // against 327; four per lane 338).
+    // (2048 tokens, 128 x 128, delta rule, with the pairs, from a cold L2: 64 heads 601 us, two per lane 755, blocks of 16 columns
+    // 951 and 794; 32 heads 384, 388, 497 and 411).  Where they would leave a quarter of the multiprocessors without a block, 16
+    // columns, two per lane (16 heads: 235 us against 366; four per lane 359).
     const int sms = sm_count_cached() > 0 ? sm_count_cached() : 148;
 #define CHUNK_LAUNCH(COLS, NL) \
     return launch_chunk_scan<DK, KIND, COLS, NL>(seg_info, segments, qn, kn, vv, decay, pairs, state, state_stride, heads, kv_heads, dv, o_raw, stream)

@@ -1028,19 +1028,37 @@ CHUNK_MODES = (SCAN_DELTA, SCAN_PLAIN, SCAN_HEAD_DECAY, SCAN_FIXED_DECAY)      #
 # Tokens per portion, on average, from which on the recurrences run by chunks if the step is large (64 * 32768 tokens x heads x
 # key elements), and from two and a half times which on in any case.  Token by token a portion takes a quarter of a
 # microsecond per token whatever else there is, and a step of many portions or heads as long as its work; by chunks there
-# are two kernels and less work.  The delta rule with 32 heads of 128 x 128: one portion of 64 tokens 24 us against 26, of 256 77
-# against 56; eight of 32 tokens 54 against 53, of 64 99 against 80.  Between the lines both take some 40 us, and the second
-# launch costs more than it saves (four portions of 90 tokens, 16 heads of 64 x 128: the whole op 40 us against 48).
+# are two kernels and less work.  The delta rule with 32 heads of 128 x 128, token by token and by chunks: one portion of 64
+# tokens 27 and 32 us, of 256 80 and 65; eight of 48 tokens 82 and 77, of 64 104 and 91.  Between the lines both take some 40 us,
+# and the second launch costs more than it saves (four portions of 90 tokens, 16 heads of 64 x 128: 29 and 30 us, of the whole
+# op 40 and 48).
 CHUNK_TOKENS = 64
+
+
+def chunks_pay(mode: int, segments: int, tokens: int, heads: int, dk: int, cols: int) -> bool:
+    """Whether a recurrence over portions is faster by chunks than token by token, with ``cols`` value columns per head.
+
+    Beside the lines at ``CHUNK_TOKENS`` (which move with it): the chunks' matrices are made once per (portion, head), whatever
+    the columns, and token by token every column is a thread's own work.  So with many of either the chunks pay only where a head
+    has enough columns.  Token by token and by chunks, portions of 256 tokens: decays per channel, eight portions of 64 heads
+    of 64 x 16 82 and 112 us, of 64 x 48 (32 heads) 100 and 112, of 64 x 64 101 and 110; of 128 x 16 129 and 147; one decay
+    per head, twelve of 64 heads of 64 x 16 96 and 114.  The delta rule's chunks do twice the work of the others', so with keys of
+    64 elements they win only while the columns of a step are few: 16 heads of 64 x 128 529 and 169 us for 2048 tokens, three
+    portions of 32 heads up to a fifth faster, four 111 and 126, twelve of 64 heads of 64 x 64 310 and 341."""
+    if tokens < CHUNK_TOKENS * segments or not (2 * tokens >= 5 * CHUNK_TOKENS * segments or tokens * heads * dk >= CHUNK_TOKENS << 15):
+        return False
+    pairs = segments * heads * CHUNK_TOKENS / 64
+    if mode == SCAN_DELTA and dk == 64:
+        return pairs <= 160 and pairs * cols <= 96 * 128
+    return pairs <= 160 or cols >= (48 if dk == 128 else 64 if mode == SCAN_HEAD_DECAY else 128)
 
 
 def _scan(mode, seg_info, tokens, token_slot, qn, kn, vv, decay, beta, state, heads, kv_heads, dk, cols, o_raw, fgate=None,
           erase=None, aux_off=0, floor_eps=0.0, den=None) -> None:
     """The recurrence itself: by chunks of sixteen tokens for prompt portions, else token by token."""
     segments = tokens if seg_info is None else seg_info.shape[0]
-    if seg_info is not None and tokens >= CHUNK_TOKENS * segments and mode in CHUNK_MODES and 0 < segments <= 65535 \
-            and (2 * tokens >= 5 * CHUNK_TOKENS * segments or tokens * heads * dk >= CHUNK_TOKENS << 15) \
-            and dk in (64, 128) and cols % 16 == 0:
+    if seg_info is not None and mode in CHUNK_MODES and 0 < segments <= 65535 and dk in (64, 128) and cols % 16 == 0 \
+            and chunks_pay(mode, segments, tokens, heads, dk, cols):
         # T and Q T of every chunk and head: a chunk of sixteen tokens at most per sixteen rows and one more per portion
         pairs = torch.empty((tokens // 16 + segments) * heads * 512, dtype=torch.float32, device=qn.device)
         _check(lib().tllm_chunk_scan(_p(seg_info), segments, tokens, _p(qn), _p(kn), _p(vv), _p(decay), _p(beta), _p(fgate),
