@@ -49,3 +49,15 @@ def test_the_tcgen05_product_is_chosen_where_its_tiles_fill_the_gpu():
 def test_recurrences_go_by_chunks_where_that_is_faster(mode, segments, each, heads, dk, cols, chunks):
     code = {"delta": ops.SCAN_DELTA, "plain": ops.SCAN_PLAIN, "head": ops.SCAN_HEAD_DECAY, "fixed": ops.SCAN_FIXED_DECAY}[mode]
     assert ops.chunks_pay(code, segments, segments * each, heads, dk, cols) == chunks
+
+
+def test_runs_of_keys_of_one_token_attention():
+    runs = ops.biased_decode_splits
+    assert runs(8, 8, 2000) == 4 and runs(16, 8, 4000) == 2 and runs(40, 8, 4000) == 3 and runs(64, 8, 2000) == 1
+    assert runs(80, 2, 1000) == 3 and runs(40, 4, 1000) == 3 and runs(20, 8, 1000) == 3      # whole rounds alone would take one
+    assert runs(1, 1, 100) == 1 and runs(1, 1, 1 << 20) == 64
+    for rows in (1, 3, 8, 64, 300):
+        for reach in (1, 200, 611, 5000):
+            assert 1 <= runs(rows, 8, reach) <= max(1, min(reach // 192, 64))
+    before = runs.cache_info().hits                      # a step asks once per layer: the search is not made again
+    assert runs(8, 8, 2000) == 4 and runs.cache_info().hits == before + 1 and runs.cache_info().maxsize
