@@ -661,14 +661,16 @@ def design_bench(args) -> int:
     w_d = (torch.randn(E, W, I, device=device) * 0.02).to(bf)
     zr = torch.randn(T, E, device=device)
     ids, wts = ops.moe_route(zr, top)
-    on_tensor_memory = ops.moe_tcgen05_pays(T * top, E, I, W, bf)
-    plan = ops.MoePlan(ids, E, ops.MOE_TCGEN05_TILE if on_tensor_memory else None)
-    flops = 2.0 * T * top * 3 * W * I
 
-    def experts():
-        a = ops.moe_grouped(x, w_gu, plan, top, gated=True, gather=True, weights=wts, interleaved=True)
-        return ops.moe_grouped(a, w_d, plan, top, gated=False, gather=False)
-    ms = timed(experts)
+    def plan_of(ids):                              # as the part makes it
+        return ops.MoePlan(ids, E, ops.moe_row_box(ids.numel(), E), tensor_memory=True)
+
+    def products(rows_in, plan, weights):
+        a = ops.moe_grouped(rows_in, w_gu, plan, top, gated=True, gather=True, weights=weights, interleaved=True)
+        return ops.moe_grouped(a, w_d, plan, top, gated=False, gather=False, out_dtype=ops.moe_result_dtype(plan.n, E, bf))
+    plan = plan_of(ids)
+    flops = 2.0 * T * top * 3 * W * I
+    ms = timed(lambda: products(x, plan, wts))
     kern["moe_grouped_products_2048_tokens"] = {"us": round(ms * 1e3, 1), "tflops": round(flops / ms / 1e9, 1),
                                                 "frac_tensor": round(flops / ms / 1e9 / pk["bf16_tflops"], 3)}
     # four times the rows: an expert's 128-row tiles are then mostly full (at 2048 tokens an expert gets 128 rows
@@ -676,12 +678,8 @@ def design_bench(args) -> int:
     T4 = 4 * T
     x4 = torch.randn(T4, W, device=device).to(bf)
     ids4, wts4 = ops.moe_route(torch.randn(T4, E, device=device), top)
-    plan4 = ops.MoePlan(ids4, E, ops.MOE_TCGEN05_TILE if ops.moe_tcgen05_pays(T4 * top, E, I, W, bf) else None)
-
-    def experts4():
-        a = ops.moe_grouped(x4, w_gu, plan4, top, gated=True, gather=True, weights=wts4, interleaved=True)
-        return ops.moe_grouped(a, w_d, plan4, top, gated=False, gather=False)
-    ms = timed(experts4)
+    plan4 = plan_of(ids4)
+    ms = timed(lambda: products(x4, plan4, wts4))
     kern["moe_grouped_products_8192_tokens"] = {"us": round(ms * 1e3, 1), "tflops": round(4 * flops / ms / 1e9, 1),
                                                 "frac_tensor": round(4 * flops / ms / 1e9 / pk["bf16_tflops"], 3)}
     del x4, ids4, wts4, plan4
@@ -692,13 +690,9 @@ def design_bench(args) -> int:
                                                     "frac_tensor": round(flops / ms / 1e9 / pk["bf16_tflops"], 3)}
     x8 = x[:8].contiguous()
     ids8, wts8 = ops.moe_route(zr[:8].contiguous(), top)
-    plan8 = ops.MoePlan(ids8, E)
+    plan8 = plan_of(ids8)
     nbytes = 8 * top * 3 * W * I * 2           # 32 different experts at most
-
-    def experts8():
-        a = ops.moe_grouped(x8, w_gu, plan8, top, gated=True, gather=True, weights=wts8, interleaved=True)
-        return ops.moe_grouped(a, w_d, plan8, top, gated=False, gather=False)
-    ms = timed(experts8)
+    ms = timed(lambda: products(x8, plan8, wts8))
     kern["moe_grouped_products_8_rows"] = {"us": round(ms * 1e3, 1), "gbs_at_most": round(nbytes / ms / 1e6, 1)}
     ms = timed(lambda: ops.linear(ops.linear_swiglu(x8, wd_gu, bf, interleaved=True), wd_d, out_dtype=bf))
     kern["dense_products_8_rows_of_one_expert_set"] = {"us": round(ms * 1e3, 1), "gbs": round(top * 3 * W * I * 2 / ms / 1e6, 1)}
