@@ -14,9 +14,10 @@
 //            gather its rows from the tokens (scaled by the assignment's weight, for routers whose
 //            weight multiplies the expert's input) and apply act(gate) * up in its epilogue; bfloat16
 //            with interleaved gate and up rows runs on the tcgen05 product (gemm_tcgen05.cu), which reads its rows
-//            by TMA: `gather` lays the token rows out in the plan's order first.  Stacked [gate; up] weights run on
-//            mma.sync tiles (64 rows x 64 weight rows x 32 deep, operands prefetched through registers), float32 and
-//            odd sizes one thread per output with the sum over k in order;
+//            by TMA: `gather` lays the token rows out in the plan's order first.  Stacked [gate; up] weights (and
+//            interleaved ones over a plan that is not made for that product) run on mma.sync tiles (64 rows x 64
+//            weight rows x 32 deep, operands prefetched through registers), float32 and odd sizes one thread per
+//            output with the sum over k in order;
 //   combine  out[t] = shared[t] + sum over the token's assignments of (weight *) y[row], in float32; an
 //            assignment to an expert past the last real one (an identity expert) adds the token's input instead.
 //
@@ -635,7 +636,7 @@ int tllm_moe_grouped(const void* A, int lda, const int* src_of, const float* wei
     return finish_launch("moe_grouped");
 }
 
-// y_dtype: float32 rows, or rows in the storage type (the grouped tcgen05 product writes bfloat16).
+// x and xs on 16-byte boundaries.
 int tllm_moe_gather(const void* x, const int* src_of, const float* weight_of, int top, void* xs, int rows, int width,
                     cudaStream_t stream) {
     TLLM_REQUIRE(rows >= 0 && width > 0 && width % 8 == 0 && top > 0, "moe_gather: bad sizes");
@@ -648,6 +649,7 @@ int tllm_moe_gather(const void* x, const int* src_of, const float* weight_of, in
     return finish_launch("moe_gather");
 }
 
+// y_dtype: float32 rows, or rows in the storage type (the tcgen05 product writes either).
 // x, expert_of_row, real: all or none; assignments to experts from `real` on add the token's row of x.
 int tllm_moe_combine(const void* y, int y_dtype, const int* row_of, const float* weight_of, int top, const void* shared,
                      void* out, int dtype, int tokens, int width, const void* x, const int* expert_of_row, int real,

@@ -1412,7 +1412,8 @@ class MoePlan:
                                    _p(self.tile_row0), _stream()), "moe_plan")
 
 
-MOE_TCGEN05_ROWS = 1        # from this many (token, choice) rows on the experts' products run on tcgen05
+MOE_TCGEN05_ROWS = 1        # from this many (token, choice) rows on the experts' products run on tcgen05: all of them (a larger
+                            # number sends smaller steps to the mma.sync tiles, to compare the two)
 MOE_TCGEN05_TILE = 128
 MOE_NARROW_ROWS = 1024      # from this many rows on (and 32 per expert) their results are kept in the storage type
 
