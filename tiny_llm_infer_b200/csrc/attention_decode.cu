@@ -275,7 +275,7 @@ template <int HD>
 static int launch_decode(const void* q, const void* cache, const int* positions, const int* token_slot,
                          const int* rows, int n_rows, const int* block_table, int max_pages,
                          int page_size, int q_heads, int kv_heads, int window, float scale, int splits,
-                         float* part_o, float* part_ml, void* out, cudaStream_t stream) {
+                         float* part_o, float* part_ml, void* out, bool shared, cudaStream_t stream) {
     const size_t smem = (size_t)kDecWarps * kDecStages * 2 * kTileKeys * HD * 2;
     static OncePerDevice configured;
     if (configured.first()) {
@@ -290,7 +290,9 @@ static int launch_decode(const void* q, const void* cache, const int* positions,
     // Qwen3-8B sizes at batch 1: 3.33 instead of 3.38 ms); with more blocks than that the early ones
     // are in the way of the kernel before (batch 8: 4.12 instead of 4.08 ms).
     const long long blocks = (long long)splits * kv_heads * n_rows;
-    const int cls = blocks <= sm_count_cached() ? kPdlAlways : kPdlAttention;
+    // Rows of one request in one step (`shared`) read keys that the kernel before has yet to write, so what is
+    // fetched before the wait would be too early for them: an ordinary launch, whatever the classes say.
+    const int cls = shared ? 0 : blocks <= sm_count_cached() ? kPdlAlways : kPdlAttention;
     launch_pdl(cls, paged_attention_decode_kernel<HD>, grid, dim3(kDecWarps * 32), smem, stream,
         (const bf16*)q, (const bf16*)cache, positions, token_slot, rows, block_table, max_pages, page_size,
         q_heads, kv_heads, window, scale * 1.4426950408889634f, splits, part_o, part_ml, (bf16*)out);
@@ -307,10 +309,11 @@ using namespace tllm;
 
 // Scratch the caller provides when splits > 1:
 //   part_o  float[n_rows * q_heads * splits * head_dim],  part_ml  float[n_rows * q_heads * splits * 2].
-extern "C" int tllm_paged_attention_decode(
+// shared: whether rows may belong to one request (a short prompt portion taken row by row).
+extern "C" int tllm_paged_attention_decode_rows(
     const void* q, const void* cache, const int* positions, const int* token_slot, const int* rows,
     int n_rows, const int* block_table, int max_pages, int page_size, int q_heads, int kv_heads,
-    int head_dim, int window, float scale, int splits, float* part_o, float* part_ml, void* out,
+    int head_dim, int window, float scale, int splits, float* part_o, float* part_ml, void* out, int shared,
     cudaStream_t stream) {
     TLLM_REQUIRE(q_heads > 0 && kv_heads > 0 && q_heads % kv_heads == 0 && q_heads / kv_heads <= 16,
                  "paged_attention_decode: %d query heads over %d key/value heads (at most 16 per group)",
@@ -323,9 +326,19 @@ extern "C" int tllm_paged_attention_decode(
     if (n_rows == 0) return 0;
     if (head_dim == 64)
         return launch_decode<64>(q, cache, positions, token_slot, rows, n_rows, block_table, max_pages, page_size,
-                                 q_heads, kv_heads, window, scale, splits, part_o, part_ml, out, stream);
+                                 q_heads, kv_heads, window, scale, splits, part_o, part_ml, out, shared != 0, stream);
     return launch_decode<128>(q, cache, positions, token_slot, rows, n_rows, block_table, max_pages, page_size,
-                              q_heads, kv_heads, window, scale, splits, part_o, part_ml, out, stream);
+                              q_heads, kv_heads, window, scale, splits, part_o, part_ml, out, shared != 0, stream);
+}
+
+extern "C" int tllm_paged_attention_decode(
+    const void* q, const void* cache, const int* positions, const int* token_slot, const int* rows,
+    int n_rows, const int* block_table, int max_pages, int page_size, int q_heads, int kv_heads,
+    int head_dim, int window, float scale, int splits, float* part_o, float* part_ml, void* out,
+    cudaStream_t stream) {
+    return tllm_paged_attention_decode_rows(q, cache, positions, token_slot, rows, n_rows, block_table, max_pages,
+                                            page_size, q_heads, kv_heads, head_dim, window, scale, splits, part_o,
+                                            part_ml, out, 0, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

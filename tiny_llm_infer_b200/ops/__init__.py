@@ -123,8 +123,8 @@ def _declare(h) -> None:
         "tllm_gemm_tcgen05": [vp, vp, vp, i32, i32, i32, i32, f32, f32, vp, vp],
         "tllm_gemm_skinny_swiglu": [vp, vp, vp, i32, i32, i32, i32, f32, f32, vp],
         "tllm_gemm_skinny_act": [vp, vp, vp, i32, i32, i32, i32, vp],
-        "tllm_paged_attention_decode": [vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, f32,
-                                        i32, vp, vp, vp, vp],
+        "tllm_paged_attention_decode_rows": [vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, f32,
+                                             i32, vp, vp, vp, i32, vp],
         "tllm_paged_attention_prefill": [vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, f32, vp, vp],
         "tllm_paged_attention_prefill_tc": [vp, i32, vp, i32, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, f32,
                                             vp, i32, vp, vp, vp, vp],
@@ -391,8 +391,9 @@ def fast_attention_ok(dtype, page_size: int, q_heads: int, kv_heads: int, head_d
 
 
 def paged_attention_decode(q, cache, positions, token_slot, rows, n_rows, block_table, page_size,
-                           q_heads, kv_heads, head_dim, window, scale, out, max_context, splits=None):
-    """Attention of one-token rows (``rows``: their indices, None for all), keys split over
+                           q_heads, kv_heads, head_dim, window, scale, out, max_context, splits=None, shared=False):
+    """Attention of one-token rows (``rows``: their indices, None for all; ``shared``: several may belong to one
+    request), keys split over
     ``splits`` blocks per (row, key/value head); the splits' partial results go through scratch
     in global memory to a second small kernel that combines them in the order of the splits."""
     _cuda(q, cache, positions, token_slot, rows, block_table, out)
@@ -403,10 +404,10 @@ def paged_attention_decode(q, cache, positions, token_slot, rows, n_rows, block_
         n = n_rows * q_heads * splits
         ws = workspace(q.device, n * (head_dim + 2))
         part_o, part_ml = ws[:n * head_dim], ws[n * head_dim:n * (head_dim + 2)]
-    _check(lib().tllm_paged_attention_decode(
+    _check(lib().tllm_paged_attention_decode_rows(
         _p(q), _p(cache), _p(positions), _p(token_slot), _p(rows), n_rows, _p(block_table),
         block_table.shape[1], page_size, q_heads, kv_heads, head_dim, int(window or 0), float(scale),
-        splits, _p(part_o), _p(part_ml), _p(out), _stream()), "paged_attention_decode",
+        splits, _p(part_o), _p(part_ml), _p(out), int(shared), _stream()), "paged_attention_decode",
         kernels=2 if splits > 1 else 1)
     return out
 
@@ -485,7 +486,7 @@ def paged_attention(q: torch.Tensor, cache: torch.Tensor, positions, token_slot,
         if ctx.n_dec:
             paged_attention_decode(q, cache, positions, token_slot, ctx.dec_rows, ctx.n_dec, block_table,
                                    page_size, q_heads, kv_heads, head_dim, window, scale, out,
-                                   ctx.max_context)
+                                   ctx.max_context, shared=getattr(ctx, "shared_rows", False))
         if ctx.n_tiles:
             if PREFILL_TCGEN05 and head_dim == 128 and getattr(ctx, "n_tiles256", 0):
                 pairs = prefill_tcgen05_block_rows(q_heads, kv_heads) == 128

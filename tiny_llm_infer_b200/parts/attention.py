@@ -26,6 +26,7 @@ from .spec import CacheSpec, ParamSpec, PartSpec, StateSpec
 @register("mixer", "gq_attention")
 class GroupedQueryAttention:
     graph_safe = True      # every launch reads the step's data from device buffers: capturable
+    rowwise = True         # all keys of a step are written before any row attends: a portion may go row by row
 
     def __init__(self, hidden_size: int, q_heads: int, kv_heads: int, head_dim: int,
                  dtype: torch.dtype, device, qk_norm_eps: Optional[float] = None,

@@ -72,6 +72,7 @@ class Block:
 
 @register("block", "prenorm")
 class PreNormBlock(Block):
+    rowwise = True         # the arrangement itself looks at no other row
     roles = {"norm1": "norm", "mixer": "mixer", "norm2": "norm", "ffn": "feed_forward"}
 
     def forward(self, h: torch.Tensor, pending: Optional[torch.Tensor], ctx, cache) -> torch.Tensor:

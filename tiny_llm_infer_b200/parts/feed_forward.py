@@ -21,6 +21,7 @@ from .spec import ParamSpec
 
 @register("feed_forward", "swiglu")
 class SwiGLUFeedForward:
+    rowwise = True
     NAMES = ("gate_proj.weight", "up_proj.weight", "down_proj.weight")
 
     def __init__(self, hidden_size: int, intermediate_size: int, dtype: torch.dtype, device,
