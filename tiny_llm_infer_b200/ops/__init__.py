@@ -552,6 +552,21 @@ def uniform_of(seed: int, token: int) -> float:
 
 
 SKINNY_MAX_ROWS = 8       # up to this many rows the weight-streaming product beats the library
+SKINNY_WIDE_ROWS = 16     # and up to this many where few blocks share the weight: see skinny_pays
+
+
+def skinny_pays(x: torch.Tensor, weight: torch.Tensor, gated: bool = False) -> bool:
+    """Whether a bfloat16 product goes to the weight-streaming kernel, which gives 16 weight rows to a block.
+    Beyond eight rows of x a block holds two row tiles and its registers leave two blocks per SM: one round
+    of those is ahead of the library's kernel (16 rows, Qwen3-0.6B sizes: q/k/v 3.9 us against 4.3, output 5.0 against 6.9,
+    down 6.1 against 8.8), more are not (8B sizes: q/k/v 16.9 against 12.2, gate/up 48 against 36); a gated product also
+    saves the activation's kernel, which pays for half a round more (6.4 against 8.6; 8B sizes 49 against 41)."""
+    rows, k = x.shape
+    if k % 8 or not x.is_contiguous() or not weight.is_contiguous():
+        return False
+    blocks = -(-weight.shape[0] // 16)
+    return 0 < rows <= SKINNY_MAX_ROWS or (0 < rows <= SKINNY_WIDE_ROWS and blocks <= SM_COUNT * (3 if gated else 2)
+                                           and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
 
 
 def gemm_skinny(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
@@ -657,8 +672,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     if x.dtype != weight.dtype:
         x = cast(x, weight.dtype)
     rows, k = x.shape
-    if weight.dtype == torch.bfloat16 and 0 < rows <= SKINNY_MAX_ROWS and k % 8 == 0 \
-            and x.is_contiguous() and weight.is_contiguous() and want in _DT:
+    if weight.dtype == torch.bfloat16 and want in _DT and skinny_pays(x, weight):
         return gemm_skinny(x, weight, want)
     if want == torch.bfloat16 and tcgen05_pays(rows, weight.shape[0], k, weight.dtype) \
             and x.is_contiguous() and weight.is_contiguous():
@@ -692,7 +706,7 @@ def linear_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, out_dtype: torch.dty
         and w_gate_up.is_contiguous()
     if plain and tcgen05_pays(rows, inter, k, w_gate_up.dtype, col_tile=128):
         return gemm_tcgen05(x, w_gate_up, swiglu=True, interleaved=interleaved, act=act, consts=consts)
-    if plain and interleaved and 0 < rows <= SKINNY_MAX_ROWS and k % 8 == 0:
+    if plain and interleaved and skinny_pays(x, w_gate_up, gated=True):
         return gemm_skinny_swiglu(x, w_gate_up, act, consts)
     gate_up = linear(x, w_gate_up, out_dtype=out_dtype)
     out = torch.empty((rows, inter), dtype=out_dtype, device=x.device)
