@@ -12,23 +12,22 @@
 //
 // and the delta rule's u come from one triangular 16 x 16 matrix, u = T (v - x) with T = (1 + diag(beta) A)^-1 diag(beta),
 // which the columns of a head share; its read-outs from Q T, o_i = .. + sum_j (Q T)_ij (v - x)_j.  So the state is read twice
-// and written once per sixteen tokens, as small matrix products with sixteen independent sums each.  Every G is a product of
-// decays, made by multiplying them up from either side; nothing is divided and no exponential of a sum is taken, so the
-// results are as exact as the token's way.  All sums are float32.
+// and written once per sixteen tokens, as small matrix products.  Every G is a product of decays, made by multiplying them up from
+// either side; nothing is divided and no exponential of a sum is taken, so the results are as exact as the token's way.
 //
-//   chunk_pairs  one warp per (chunk, head): T and Q T, or Q, the decays from the chunk's start and the write weights.
-//   chunk_scan   one block per (portion, head, 32 or 16 columns); a warp owns 2 NL columns, a lane 8 rows (4 where keys have
-//                64 elements) of NL of them in registers.  The sums of a group of tokens meet over the sixteen lanes of a
-//                column by exchanging halves.
+//   chunk_pairs  one warp per (chunk, head): T and Q T, or Q, the decays from the chunk's start and the write weights
+//                (chunk_scalar_pairs where the decays are per head: one warp per chunk and key head).
+//   chunk_scan   one block per (portion, head, 32 or 16 columns): the state in the registers of four warps, its products on the
+//                tensor cores with every float32 operand in three bfloat16 parts.
 //
 // The layout of the request's state is the scan kernel's (row r * per + il of column j at [il][j][r]).
 #include "common.cuh"
+#include "mma_tiles.cuh"
 
 namespace tllm {
 
 constexpr int kC = 16;                         // tokens of a chunk
 constexpr int kPairFloats = 2 * kC * kC;       // T and Q T, or the scalars and Q, of one (chunk, head)
-constexpr int kPad = 20;                       // floats of a row of either in shared memory
 
 // What the sums need of a recurrence.  kDelta: decays per channel and the correction; kChannel: decays per channel, u = w v
 // (w = 1 where `beta` is null); kHead: one decay per (token, head) in `beta`, w in `fgate`; kFixed: one decay per head in
@@ -67,12 +66,49 @@ __device__ __forceinline__ float halves_sum(float (&v)[N], int lane) {
     return N == 16 ? v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16) : v[0];
 }
 
-// DK 128: a lane has four neighbouring channels; DK 64: the upper sixteen lanes carry zeros.
+__device__ __forceinline__ float low_float(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float high_float(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+
+// Two neighbours in three parts each, packed pairwise.
+__device__ __forceinline__ void split3(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
+    h = pack_bf16(x, y);
+    x -= low_float(h), y -= high_float(h);
+    m = pack_bf16(x, y);
+    x -= low_float(m), y -= high_float(m);
+    l = pack_bf16(x, y);
+}
+
+// The left operand of one step of sixteen terms from two tiles of accumulators.
+__device__ __forceinline__ void split_left(const float (&t0)[4], const float (&t1)[4], uint32_t (&a)[3][4]) {
+    split3(t0[0], t0[1], a[0][0], a[1][0], a[2][0]);
+    split3(t0[2], t0[3], a[0][1], a[1][1], a[2][1]);
+    split3(t1[0], t1[1], a[0][2], a[1][2], a[2][2]);
+    split3(t1[2], t1[3], a[0][3], a[1][3], a[2][3]);
+}
+
+// d[k] = a[k / PER] . (tile k of the tiles in b, two to a b) over sixteen terms each, N products side by side: each is a chain of six
+// dependent mma, and four or more chains keep the tensor pipe busy where one waits four times as long as it works.
+template <int N, int PER, int NA, int NB>
+__device__ __forceinline__ void products3(float (&d)[N][4], const uint32_t (&a)[NA][3][4], const uint32_t (&b)[NB][3][4]) {
+    constexpr int kLeft[6] = {2, 0, 1, 1, 0, 0}, kRight[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+    for (int k = 0; k < N; ++k) d[k][0] = d[k][1] = d[k][2] = d[k][3] = 0.0f;
+#pragma unroll
+    for (int s = 0; s < 6; ++s)
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const uint32_t bt[2] = {b[k / 2][kRight[s]][2 * (k % 2)], b[k / 2][kRight[s]][2 * (k % 2) + 1]};
+            mma_bf16_16816(d[k], a[k / PER][kLeft[s]], bt);
+        }
+}
+
+// Decays per channel.  DK 128: a lane has four neighbouring channels; DK 64: the upper sixteen lanes carry zeros.
 template <int DK, int KIND>
 __global__ void __launch_bounds__(128)
 chunk_pairs_kernel(const int* __restrict__ seg_info, int segments, const float* qn, const float* kn, const float* decay, const float* beta,
-                   const float* fgate, int heads, int kv_heads, float* pairs) {
-    constexpr bool kVec = KIND == kDelta || KIND == kChannel, kCorr = KIND == kDelta;
+                   int heads, int kv_heads, float* pairs) {
+    static_assert(KIND == kDelta || KIND == kChannel, "one decay per head: chunk_scalar_pairs_kernel");
+    constexpr bool kCorr = KIND == kDelta;
     const int seg = blockIdx.y, slot = seg_info[4 * seg], start = seg_info[4 * seg + 1], len = seg_info[4 * seg + 2];
     const int first = first_entry(seg_info, segments, seg);
     const int lane = threadIdx.x & 31, head = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -87,18 +123,10 @@ chunk_pairs_kernel(const int* __restrict__ seg_info, int segments, const float* 
         auto at = [&](const float* p, int i, int h, int hs) -> float4 {
             return live ? *reinterpret_cast<const float4*>(p + ((size_t)(start + c0 + i) * hs + h) * DK + lane * 4) : zero;
         };
-        // scalars of token `col`: its decay and the weight of its values
-        float a_own = 1.0f, w_own = 1.0f;
-        if (col < n) {
-            const size_t t = (size_t)(start + c0 + col) * heads + head;
-            if (KIND == kDelta || KIND == kChannel) w_own = beta != nullptr ? beta[t] : 1.0f;
-            if (KIND == kHead) { a_own = beta[t]; w_own = fgate[t]; }
-            if (KIND == kFixed) a_own = fgate[head];
-        }
+        const float w_own = col < n && beta != nullptr ? beta[(size_t)(start + c0 + col) * heads + head] : 1.0f;     // of token `col`
         float4 w[kC];                                               // k_j, decayed up to the token at hand
         float4 q4[4], g4[4];                                        // the next four tokens' q and decays
         float trow[kC];                                             // column `col` of T
-        float d = 1.0f, prefix = 1.0f;                              // scalar decays: of j up to i, and from the chunk's start
 #pragma unroll
         for (int i = 0; i < kC; ++i) w[i] = i < n ? at(kn, i, kvh, kv_heads) : zero;
 #pragma unroll
@@ -107,14 +135,12 @@ chunk_pairs_kernel(const int* __restrict__ seg_info, int segments, const float* 
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     q4[e] = i + e < n ? at(qn, i + e, kvh, kv_heads) : zero;
-                    if (kVec) g4[e] = i + e < n ? at(decay, i + e, head, heads) : one;
+                    g4[e] = i + e < n ? at(decay, i + e, head, heads) : one;
                 }
             const float4 k = w[i], q = q4[i % 4];                   // w[i] has no decay on it yet
             float s;                                                // lane j: Q_ij; with the correction lane 16 + j: A_ij
-            if (kVec) {
 #pragma unroll
-                for (int j = 0; j < i; ++j) w[j] = mul4(w[j], g4[i % 4]);
-            }
+            for (int j = 0; j < i; ++j) w[j] = mul4(w[j], g4[i % 4]);
             if (kCorr) {
                 float v[32];
 #pragma unroll
@@ -141,322 +167,461 @@ chunk_pairs_kernel(const int* __restrict__ seg_info, int segments, const float* 
 #pragma unroll
                 for (int j = 0; j < kC; ++j) v[j] = j <= i ? dot4(q, w[j]) : 0.0f;
                 s = halves_sum<16>(v, lane);
-                if (!kVec) {
-                    const float a = __shfl_sync(0xffffffffu, a_own, i);
-                    if (col < i) d *= a;                            // j < i: one more decay between j and i
-                    prefix *= a;
-                    s *= d;
-                    if (lane == 0) T[i] = prefix;
-                } else if (lane == 0) {
-                    T[i] = 1.0f;
-                }
+                if (lane == 0) T[i] = 1.0f;
                 // of a later token nothing, not zero times its weight: that may be infinite or no number
                 if (lane < 16) Q[i * kC + col] = col <= i ? s * w_own : 0.0f;
             }
         }
-        // row 1: what token j's values are multiplied by in the state, its weight and the decays after it
-        if (!kCorr && lane < 16) T[kC + col] = w_own * d;
+        if (!kCorr && lane < 16) T[kC + col] = w_own;               // row 1: what token j's values are multiplied by in the state
+    }
+}
+
+// One decay per head: Q_ij = w_j d_ij q_i^T k_j, where the products of a chunk's queries and keys are the same for all heads of a
+// key and d_ij is the product of the decays j + 1 .. i.  One warp per (chunk, key head): q and k straight from memory in the
+// operands' layout, and their product on the tensor cores as in the scan below.  Bound by reading q and k (2048 tokens, 32 heads
+// of 128: 67 MB).
+template <int DK, int KIND>
+__global__ void __launch_bounds__(128)
+chunk_scalar_pairs_kernel(const int* __restrict__ seg_info, int segments, const float* qn, const float* kn, const float* beta,
+                          const float* fgate, int heads, int kv_heads, float* pairs) {
+    const int seg = blockIdx.y, slot = seg_info[4 * seg], start = seg_info[4 * seg + 1], len = seg_info[4 * seg + 2];
+    const int first = first_entry(seg_info, segments, seg);
+    const int lane = threadIdx.x & 31, kvh = blockIdx.x * 4 + (threadIdx.x >> 5), rep = heads / kv_heads;
+    if (kvh >= kv_heads || slot < 0) return;
+    const int row = lane >> 2, two = (lane & 3) * 2, col = lane & 15;
+    for (int c0 = blockIdx.z * kC; c0 < len; c0 += gridDim.z * kC) {
+        const int n = min(kC, len - c0);
+        const size_t at = ((size_t)(start + c0) * kv_heads + kvh) * DK + two;
+        auto load = [&](const float* p, int i, int ch) -> float2 {
+            return i < n ? *reinterpret_cast<const float2*>(p + at + (size_t)i * kv_heads * DK + ch) : make_float2(0.0f, 0.0f);
+        };
+        float s[2][4];                                              // q_i^T k_j: rows i of the lane, row and row + 8; tiles of eight j
+        constexpr int kAhead = 4;                                   // steps of sixteen channels whose loads are on their way at once
+        float2 q[kAhead][4], k[kAhead][4];
+#pragma unroll
+        for (int ks = 0; ks < DK / 16; ++ks) {
+            if (ks % kAhead == 0)
+#pragma unroll
+                for (int m = 0; m < kAhead; ++m)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        q[m][e] = load(qn, row + (e & 1) * 8, (ks + m) * 16 + (e >> 1) * 8);
+                        k[m][e] = load(kn, row + (e >> 1) * 8, (ks + m) * 16 + (e & 1) * 8);
+                    }
+            uint32_t a[1][3][4], b[1][3][4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 x = q[ks % kAhead][e], y = k[ks % kAhead][e];
+                split3(x.x, x.y, a[0][0][e], a[0][1][e], a[0][2][e]);
+                split3(y.x, y.y, b[0][0][e], b[0][1][e], b[0][2][e]);
+            }
+            float d[2][4];
+            products3<2, 2>(d, a, b);
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) s[t][e] = ks == 0 ? d[t][e] : s[t][e] + d[t][e];
+        }
+        for (int h = 0; h < rep; ++h) {
+            const int head = kvh * rep + h;
+            float a_own = 1.0f, w_own = 1.0f;                       // token `col`'s decay and the weight of its values
+            if (col < n) {
+                const size_t t = (size_t)(start + c0 + col) * heads + head;
+                if (KIND == kHead) { a_own = beta[t]; w_own = fgate[t]; }
+                else a_own = fgate[head];
+            }
+            float d[2][4], since = 1.0f, after = 1.0f;              // of the lane's (i, j); from the chunk's start to `col`; after it
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) d[t][e] = 1.0f;
+#pragma unroll
+            for (int m = 0; m < kC; ++m) {
+                const float a = __shfl_sync(0xffffffffu, a_own, m);
+                if (m <= col) since *= a;
+                else after *= a;
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (m > t * 8 + two + (e & 1) && m <= row + (e >> 1) * 8) d[t][e] *= a;
+            }
+            float* T = pairs + ((size_t)(first + c0 / kC) * heads + head) * kPairFloats;
+            float* Q = T + kC * kC;
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                const int j = t * 8 + two;
+                const float w0 = __shfl_sync(0xffffffffu, w_own, j), w1 = __shfl_sync(0xffffffffu, w_own, j + 1);
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {
+                    const int i = row + (e >> 1) * 8;
+                    // of a later token nothing, not zero times its weight: that may be infinite or no number
+                    *reinterpret_cast<float2*>(Q + i * kC + j) = make_float2(j <= i ? s[t][e] * d[t][e] * w0 : 0.0f, j + 1 <= i ? s[t][e + 1] * d[t][e + 1] * w1 : 0.0f);
+                }
+            }
+            if (lane < 16) {                                        // row 0: the decays since the chunk's start; row 1: what token
+                T[col] = since;                                     // j's values are multiplied by in the state
+                T[kC + col] = w_own * after;
+            }
+        }
     }
 }
 
 __device__ __forceinline__ void cp16(float* dst, const float* src, bool valid) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0));
 }
-__device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
-__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
 
-// COLS columns per block (16 or 32), NL columns per lane (4 or 2).
-template <int DK, int KIND, int COLS, int NL>
+// ---------------------------------------------------------------- the scan over the chunks
+// All three products of a chunk (the read-outs S^T k and S^T q, the sums with T and Q T, the update u k^T) run on
+// mma.sync m16n8k16 with every float32 operand as the exact-to-2^-24 sum of three bfloat16 parts: a product is six mma, the
+// parts' products down to 2^-18 of the largest (what is left out is below 2^-26), smallest first, started from zero for every
+// sixteen terms and then added to the running float32 sum, which keeps the tensor core's cut-off sums out of long chains.  The
+// state lies transposed in the accumulators' layout ([columns][keys], 16 columns and DK / kParts keys per warp), which is at
+// once the layout of the left operand of the read-outs; u comes out of T's product as the left operand of the update; so
+// nothing but the warps' partial read-outs, which meet over the parts of the keys, passes through shared memory.
+//
+// Warps of their own split the tokens a chunk ahead, a thread per pair of channels of one operand; others fetch them.
+//
+// What bounds it: a chunk takes a block 2300 (one decay per head) to 3300 cycles (the delta rule), of which 880 to 1450 are mma (8.6
+// cycles each and scheduler); the rest is the chain from the read-outs over the meeting of the parts and T to the update, and the
+// splitting of the state.  Eight warps with half the keys each (273 to 296 us for the delta rule), the parts' meeting prefetched
+// around (280) and operands split once by the pairs' kernel into 44 KB records per chunk and head (267, for 180 MB of scratch) did
+// not shorten it.  Before, on the float32 pipe with a lane per 8 rows of 4 columns (two fused multiply-adds per instruction), and
+// now, with the pairs: 2048 tokens of 32 heads of 128 x 128, delta rule 386 and 273 us, one decay per head 245 and 183; 16 heads 237
+// and 204, 179 and 140; 64 heads of 128 x 64, 1023 tokens, one decay per head 140 and 108.  The error against 64 bits is no larger
+// (products to 2^-26, sums of sixteen terms added in float32).
+constexpr int kMatRow = 24;                    // bfloat16 elements of a row of T or Q in shared memory
+constexpr float kLargest = 3.38e38f;           // beyond it the first part would be an infinity
+
+// LIGHT: fewer helping warps and less fetched ahead, so that two blocks share a multiprocessor (recurrences of one decay per head).
+template <int DK, int KIND, int COLS, bool LIGHT>
 struct ChunkLayout {
-    static constexpr bool kVec = KIND == kDelta || KIND == kChannel;
-    static constexpr int kWarps = COLS / (2 * NL), kStages = kVec ? 3 : 2;
-    static constexpr int kIssuers = (kVec ? COLS / 8 : kWarps) * 32;      // decays per channel: warps of their own prepare the tokens
-    static constexpr int kThreads = kWarps * 32 + (kVec ? kIssuers : 0);
-    static constexpr int kK = 0, kQ = kC * DK, kG = 2 * kC * DK, kV = kG + (kVec ? kC * DK : 0), kT = kV + kC * COLS, kQm = kT + kC * kPad;
-    static constexpr int kGam = kQm + kC * kPad, kStage = kGam + (kVec ? DK : 0);
-    static constexpr int kX = kStages * kStage, kU = kX + kC * COLS, kFloats = kU + kC * COLS;
+    static constexpr bool kVec = KIND == kDelta || KIND == kChannel, kCorr = KIND == kDelta;
+    static constexpr int kTiles = COLS / 16, kParts = 4 / kTiles, kKeys = DK / kParts;    // warps: column tiles x parts of the keys
+    static constexpr int kArrays = kCorr ? 3 : 2, kMats = kCorr ? 2 : 1;
+    static constexpr int kSplitters = (LIGHT ? 1 : kArrays) * DK / 2, kLoaders = LIGHT ? 32 : 64, kThreads = 128 + kSplitters + kLoaders;
+    static constexpr int kSplit = kC * DK * 2, kMat = kC * kMatRow * 2;                  // bytes of one part of an operand
+    static constexpr int kMatAt = kArrays * 3 * kSplit, kGamAt = kMatAt + kMats * 3 * kMat, kStage = kGamAt + (kVec ? DK * 4 : 0);
+    static constexpr int kRaw = (kVec ? 3 : 2) * kC * DK * 4;
+    static constexpr int kVRow = COLS + 4, kRing = kC * kVRow * 4 + kPairFloats * 4;
+    static constexpr int kRaws = LIGHT ? 2 : 3;                                           // chunks fetched and not yet split
+    static constexpr int kRawAt = 2 * kStage, kRingAt = kRawAt + kRaws * kRaw, kSumsAt = kRingAt + 4 * kRing;
+    static constexpr int kBytes = kSumsAt + 4 * 16 * 32 * 4;
+    static constexpr int kBlocks = kBytes <= 113 * 1024 ? 2 : 1;                         // per SM
 };
 
-template <int DK, int KIND, int COLS, int NL>
-__global__ void __launch_bounds__(ChunkLayout<DK, KIND, COLS, NL>::kThreads, 512 / ChunkLayout<DK, KIND, COLS, NL>::kThreads)
+template <int DK, int KIND, int COLS, bool LIGHT>
+__global__ void __launch_bounds__(ChunkLayout<DK, KIND, COLS, LIGHT>::kThreads, ChunkLayout<DK, KIND, COLS, LIGHT>::kBlocks)
 chunk_scan_kernel(const int* __restrict__ seg_info, const float* qn, const float* kn, const float* vv, const float* decay,
                   const float* pairs, float* state, long long state_stride, int segments, int heads, int kv_heads, int dv, float* o_raw) {
-    using L = ChunkLayout<DK, KIND, COLS, NL>;
-    constexpr bool kVec = L::kVec, kCorr = KIND == kDelta;
-    constexpr int kH = DK / 64, kPairs = 2 * kH, kIssuers = L::kIssuers;           // a lane's runs of four rows
-    constexpr int kWide = 2 * NL, kGroup = kC / NL;                                // columns of a warp; tokens whose sums meet at once
-    extern __shared__ __align__(16) float sm[];
+    using L = ChunkLayout<DK, KIND, COLS, LIGHT>;
+    constexpr bool kVec = L::kVec, kCorr = L::kCorr;
+    extern __shared__ __align__(16) unsigned char sm[];
     const int seg = blockIdx.y, groups = dv / COLS, head = blockIdx.x / groups, col0 = blockIdx.x % groups * COLS;
     const int slot = seg_info[4 * seg], start = seg_info[4 * seg + 1], len = seg_info[4 * seg + 2];
     const int first = first_entry(seg_info, segments, seg);
     if (slot < 0 || len <= 0) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane & 15, cg = (lane >> 4) * NL;
-    const int kvh = head / (heads / kv_heads), mine = warp * kWide + cg;                      // first of the lane's columns
-    float* xs = sm + L::kX + warp * kC * kWide;
-    float* us = sm + L::kU + warp * kC * kWide;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kvh = head / (heads / kv_heads);
+    const int chunks = (len + kC - 1) / kC;
+    // byte of channel ch of token i in one part of an operand: 16-byte pieces, exchanged so that eight rows lie in eight banks
+    auto at = [](int i, int piece) { return i * (DK * 2) + ((piece ^ (i & 7)) << 4); };
 
-    const int me = kVec ? (int)threadIdx.x - L::kWarps * 32 : threadIdx.x;         // among the threads that copy
-    auto issue = [&](int c0, int st) {
-        const int n = min(kC, len - c0);
-        float* s = sm + st * L::kStage;
-        for (int i = me; i < kC * DK / 4; i += kIssuers) {
-            const int t = i / (DK / 4), e = (i % (DK / 4)) * 4;
-            const bool in = t < n;
-            const size_t row = (size_t)(start + c0 + (in ? t : 0));
-            cp16(s + L::kK + t * DK + e, kn + (row * kv_heads + kvh) * DK + e, in);
-            cp16(s + L::kQ + t * DK + e, qn + (row * kv_heads + kvh) * DK + e, in);
-            if (kVec) cp16(s + L::kG + t * DK + e, decay + (row * heads + head) * DK + e, in);
-        }
-        for (int i = me; i < kC * COLS / 4; i += kIssuers) {
-            const int t = i / (COLS / 4), e = (i % (COLS / 4)) * 4;
-            const bool in = t < n;
-            cp16(s + L::kV + t * COLS + e, vv + ((size_t)(start + c0 + (in ? t : 0)) * heads + head) * dv + col0 + e, in);
-        }
-        const float* p = pairs + ((size_t)(first + c0 / kC) * heads + head) * kPairFloats;
-        for (int i = me; i < kPairFloats / 4; i += kIssuers) {
-            const int t = (i & 63) / 4, e = (i & 3) * 4;
-            cp16(s + (i < 64 ? L::kT : L::kQm) + t * kPad + e, p + i * 4, true);
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-    };
-
-    // Decays per channel: q and (for the correction) k take on the decays since the chunk's start, and g's place the k's with
-    // the decays up to its end; a thread has a channel of all sixteen tokens.  Warps of their own do it, a chunk ahead.
-    auto prepare = [&](int c0, int st) {
-        const int n = min(kC, len - c0);
-        float* s = sm + st * L::kStage;
-        for (int ch = me; ch < DK; ch += kIssuers) {
-            float k[kC], g[kC], q[kC], p = 1.0f;
+    if (warp >= 4 + L::kSplitters / 32) {                       // fetch the tokens two or three chunks ahead, split T and Q T
+        const int me = threadIdx.x - 128 - L::kSplitters;
+        auto issue = [&](int c) {                               // one group of copies a call, an empty one past the end
+            if (c >= chunks) {
+                asm volatile("cp.async.commit_group;\n" ::);
+                return;
+            }
+            const int c0 = c * kC, n = min(kC, len - c0);
+            float* raw = reinterpret_cast<float*>(sm + L::kRawAt + c % L::kRaws * L::kRaw);
+            float* v = reinterpret_cast<float*>(sm + L::kRingAt + (c & 3) * L::kRing);
+            constexpr int kPieces = DK / 4, kVPieces = COLS / 4;
+            const int e = me % kPieces * 4, ve = me % kVPieces * 4;
+            const float* q = qn + ((size_t)(start + c0) * kv_heads + kvh) * DK + e;
+            const float* k = kn + ((size_t)(start + c0) * kv_heads + kvh) * DK + e;
+            const float* g = kVec ? decay + ((size_t)(start + c0) * heads + head) * DK + e : nullptr;
+            const float* x = vv + ((size_t)(start + c0) * heads + head) * dv + col0 + ve;
 #pragma unroll
-            for (int i = 0; i < kC; ++i) {
-                k[i] = s[L::kK + i * DK + ch];
-                g[i] = s[L::kG + i * DK + ch];
-                q[i] = s[L::kQ + i * DK + ch];
+            for (int s = 0; s < kC * kPieces / L::kLoaders; ++s) {
+                const int t = me / kPieces + s * (L::kLoaders / kPieces), from = t < n ? t : 0;
+                cp16(raw + t * DK + e, q + (size_t)from * kv_heads * DK, t < n);
+                cp16(raw + (kC + t) * DK + e, k + (size_t)from * kv_heads * DK, t < n);
+                if (kVec) cp16(raw + (2 * kC + t) * DK + e, g + (size_t)from * heads * DK, t < n);
             }
 #pragma unroll
-            for (int i = 0; i < kC; ++i) {
-                if (i >= n) g[i] = 1.0f;
-                p *= g[i];
-                s[L::kQ + i * DK + ch] = q[i] * p;
-                if (kCorr) s[L::kK + i * DK + ch] = k[i] * p;
+            for (int s = 0; s < kC * kVPieces / L::kLoaders; ++s) {
+                const int t = me / kVPieces + s * (L::kLoaders / kVPieces), from = t < n ? t : 0;
+                cp16(v + t * L::kVRow + ve, x + (size_t)from * heads * dv, t < n);
             }
-            s[L::kGam + ch] = p;
-            p = 1.0f;
+            const float* p = pairs + ((size_t)(first + c) * heads + head) * kPairFloats;
 #pragma unroll
-            for (int i = kC - 1; i >= 0; --i) {
-                s[L::kG + i * DK + ch] = k[i] * p;
-                p *= g[i];
+            for (int i = 0; i < kPairFloats / 4; i += L::kLoaders) cp16(v + kC * L::kVRow + (i + me) * 4, p + (i + me) * 4, true);
+            asm volatile("cp.async.commit_group;\n" ::);
+        };
+        auto split_mats = [&](int c) {
+            constexpr int kEach = L::kMats * kC * kC / 2 / L::kLoaders;
+            const float* mats = reinterpret_cast<const float*>(sm + L::kRingAt + (c & 3) * L::kRing) + kC * L::kVRow + (kCorr ? 0 : kC * kC);
+            unsigned char* to = sm + (c & 1) * L::kStage + L::kMatAt;
+            float2 x[kEach];
+#pragma unroll
+            for (int s = 0; s < kEach; ++s) x[s] = *reinterpret_cast<const float2*>(mats + (me + s * L::kLoaders) * 2);
+#pragma unroll
+            for (int s = 0; s < kEach; ++s) {
+                const int i = me + s * L::kLoaders, mat = i / (kC * kC / 2), row = i % (kC * kC / 2) / (kC / 2), e = i % (kC / 2) * 2;
+                uint32_t h, m, l;
+                split3(x[s].x, x[s].y, h, m, l);
+                unsigned char* at_row = to + mat * 3 * L::kMat + (row * kMatRow + e) * 2;
+                *reinterpret_cast<uint32_t*>(at_row) = h;
+                *reinterpret_cast<uint32_t*>(at_row + L::kMat) = m;
+                *reinterpret_cast<uint32_t*>(at_row + 2 * L::kMat) = l;
             }
-        }
-    };
-    if (kVec && warp >= L::kWarps) {
-        issue(0, 0);
-        if (kC < len) issue(kC, 1);
-        for (int c0 = 0, st = 0; c0 < len + kC; c0 += kC, st = st == 2 ? 0 : st + 1) {     // prepares c0 while c0 - kC is consumed
-            if (c0 < len) {
-                if (c0 + kC < len) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-                else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-                asm volatile("bar.sync 1, %0;\n" ::"n"(kIssuers) : "memory");             // the copies of all of these warps
-                prepare(c0, st);
-            }
-            __syncthreads();                                    // c0 - kC is done with: its stage, the one after next, is free
-            if (c0 + 2 * kC < len) issue(c0 + 2 * kC, st == 0 ? 2 : st - 1);
+        };
+#pragma unroll
+        for (int c = 0; c < L::kRaws - 1; ++c) issue(c);
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(L::kRaws - 2) : "memory");
+        __syncthreads();                                        // chunk 0 is here
+        issue(L::kRaws - 1);
+        for (int c = 0; c <= chunks; ++c) {
+            if (c < chunks) split_mats(c);
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(L::kRaws - 2) : "memory");
+            __syncthreads();                                    // chunk c is ready, chunk c + 1 here, chunk c - 1 done with
+            issue(c + L::kRaws);
         }
         return;
     }
-    if (!kVec) issue(0, 0);
-    // the lane's rows: 64 h + 4 r + e; row i of the state lies at [i % per][column][i / per]
-    constexpr int kR = DK <= 64 ? 4 : 8, kPer = DK / kR;
-    float* st_ptr = state + (long long)slot * state_stride + (size_t)head * DK * dv;
-    auto state_at = [&](int h, int e, int c) -> float& {
-        const int i = 64 * h + 4 * r + e;
-        return st_ptr[((size_t)(i % kPer) * dv + col0 + mine + c) * kR + i / kPer];
-    };
-    float2 S[NL][kPairs];
+    if (warp >= 4) {                                            // split the tokens of chunk c while chunk c - 1 is consumed
+        const int me = threadIdx.x - 128, ch = me % (DK / 2) * 2;
+        // operand 0: q with the decays since the chunk's start on it, 1: k with those up to its end, 2: k as q
+        __syncthreads();
+        for (int c = 0; c <= chunks; ++c) {
+            for (int array = me / (DK / 2); c < chunks && array < L::kArrays; array += L::kSplitters / (DK / 2)) {
+                const int n = min(kC, len - c * kC);
+                const float* raw = reinterpret_cast<const float*>(sm + L::kRawAt + c % L::kRaws * L::kRaw);
+                const float* src = raw + (array == 0 ? 0 : kC * DK) + ch;
+                unsigned char* stage = sm + (c & 1) * L::kStage;
+                unsigned char* dst = stage + array * 3 * L::kSplit + (ch & 7) * 2;
+                float2 p = make_float2(1.0f, 1.0f);
+                // several tokens' loads before the first store: the chains of a token's three parts overlap
+                constexpr int kBatch = 8;
+                auto batch = [&](int first_token, int step) {
+                    float2 x[kBatch], g[kBatch];
 #pragma unroll
-    for (int c = 0; c < NL; ++c)
+                    for (int s = 0; s < kBatch; ++s) {
+                        x[s] = *reinterpret_cast<const float2*>(src + (first_token + s * step) * DK);
+                        if (kVec) g[s] = *reinterpret_cast<const float2*>(raw + (2 * kC + first_token + s * step) * DK + ch);
+                    }
+                    uint32_t h[kBatch], m[kBatch], l[kBatch];
 #pragma unroll
-        for (int h = 0; h < kH; ++h) {
-            S[c][2 * h] = make_float2(state_at(h, 0, c), state_at(h, 1, c));
-            S[c][2 * h + 1] = make_float2(state_at(h, 2, c), state_at(h, 3, c));
-        }
-
-    if (kVec) __syncthreads();                                  // the first chunk is ready
-    for (int c0 = 0, st = 0; c0 < len; c0 += kC, st = st == L::kStages - 1 ? 0 : st + 1) {
-        const int n = min(kC, len - c0);
-        if (!kVec) {
-            if (c0 + kC < len) {
-                issue(c0 + kC, st ^ 1);
-                asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-            } else {
-                asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+                    for (int s = 0; s < kBatch; ++s) {
+                        if (kVec) {
+                            if (first_token + s * step >= n) g[s] = make_float2(1.0f, 1.0f);
+                            const float2 after = make_float2(p.x * g[s].x, p.y * g[s].y);
+                            if (step > 0) p = after;
+                            x[s].x *= p.x, x[s].y *= p.y;
+                            p = after;
+                        }
+                        split3(x[s].x, x[s].y, h[s], m[s], l[s]);
+                    }
+#pragma unroll
+                    for (int s = 0; s < kBatch; ++s) {
+                        unsigned char* to = dst + at(first_token + s * step, ch >> 3);
+                        *reinterpret_cast<uint32_t*>(to) = h[s];
+                        *reinterpret_cast<uint32_t*>(to + L::kSplit) = m[s];
+                        *reinterpret_cast<uint32_t*>(to + 2 * L::kSplit) = l[s];
+                    }
+                };
+                if (kVec && array == 1) {
+                    batch(kC - 1, -1);
+                    batch(kC - 1 - kBatch, -1);
+                } else {
+                    batch(0, 1);
+                    batch(kBatch, 1);
+                    if (kVec && array == 0) *reinterpret_cast<float2*>(stage + L::kGamAt + ch * 4) = p;
+                }
             }
             __syncthreads();
         }
-        float* s = sm + st * L::kStage;
-        // sums against the state before the chunk, kGroup tokens at a time; token kGroup g + r / NL of column r % NL ends here
-        float xk[NL], xq[NL];
+        return;
+    }
+    const int tile = warp % L::kTiles, part = warp / L::kTiles, key0 = part * L::kKeys;
+    const int row = lane >> 2, two = (lane & 3) * 2, mid = lane >> 3, mrow = lane & 7;
+    const int mine = tile * 16 + row;                           // the lane's first column of the block's, the other is 8 further
+    // row i of the state lies at [i % per][column][i / per]
+    constexpr int kR = DK <= 64 ? 4 : 8, kPer = DK / kR;
+    float* st_ptr = state + (long long)slot * state_stride + (size_t)head * DK * dv;
+    auto state_at = [&](int t, int e) -> float& {
+        const int i = key0 + t * 8 + two + (e & 1);
+        return st_ptr[((size_t)(i % kPer) * dv + col0 + mine + (e >> 1) * 8) * kR + i / kPer];
+    };
+    float S[L::kKeys / 8][4];
 #pragma unroll
-        for (int g = 0; g < NL; ++g) {
-            constexpr int kSums = kCorr ? 2 : 1;
-            float v[kSums][16];
+    for (int t = 0; t < L::kKeys / 8; ++t)
 #pragma unroll
-            for (int t = 0; t < kGroup; ++t) {
-                float2 acc[kSums][NL];
+        for (int e = 0; e < 4; ++e) S[t][e] = state_at(t, e);
+    float* sums = reinterpret_cast<float*>(sm + L::kSumsAt) + lane;                         // [warp][value][lane]
+
+    __syncthreads();
+    __syncthreads();                                            // the first chunk is ready
+    for (int c = 0; c < chunks; ++c) {
+        const int n = min(kC, len - c * kC);
+        const uint32_t stage = smem_u32(sm + (c & 1) * L::kStage);
+        const float* V = reinterpret_cast<const float*>(sm + L::kRingAt + (c & 3) * L::kRing);
+        const float* T = V + kC * L::kVRow;                     // float32: T and Q T, or the scalars and Q
+        // read-outs of the state before the chunk over this warp's keys: tiles of eight tokens of q, and of k
+        constexpr int kRead = kCorr ? 2 : 1;                    // operands read out: q, and k
+        constexpr int kAtOnce = L::kKeys / 16 >= 2 ? 2 : 1;     // steps of sixteen keys
+        float x[2 * kRead][4];
 #pragma unroll
-                for (int h = 0; h < kH; ++h) {
-                    const int off = (kGroup * g + t) * DK + 64 * h + 4 * r;
-                    const float4 q4 = *reinterpret_cast<const float4*>(s + L::kQ + off);
-                    float4 k4;
-                    if (kCorr) k4 = *reinterpret_cast<const float4*>(s + L::kK + off);
+        for (int ks = 0; ks < L::kKeys / 16; ks += kAtOnce) {
+            uint32_t a[kAtOnce][3][4], b[kAtOnce * kRead][3][4];
+            float d[2 * kAtOnce * kRead][4];
 #pragma unroll
-                    for (int c = 0; c < NL; ++c) {
-                        acc[0][c] = h == 0 ? __fmul2_rn(S[c][0], lo2(q4)) : __ffma2_rn(S[c][2 * h], lo2(q4), acc[0][c]);
-                        acc[0][c] = __ffma2_rn(S[c][2 * h + 1], hi2(q4), acc[0][c]);
-                        if (kCorr) {
-                            acc[kSums - 1][c] = h == 0 ? __fmul2_rn(S[c][0], lo2(k4)) : __ffma2_rn(S[c][2 * h], lo2(k4), acc[kSums - 1][c]);
-                            acc[kSums - 1][c] = __ffma2_rn(S[c][2 * h + 1], hi2(k4), acc[kSums - 1][c]);
-                        }
+            for (int k = 0; k < kAtOnce; ++k) {
+#pragma unroll
+                for (int w = 0; w < kRead; ++w)
+#pragma unroll
+                    for (int s = 0; s < 3; ++s)
+                        ldmatrix_x4(b[k * kRead + w][s], stage + ((w == 0 ? 0 : 2) * 3 + s) * L::kSplit + at((mid >> 1) * 8 + mrow, key0 / 8 + 2 * (ks + k) + (mid & 1)));
+                split_left(S[2 * (ks + k)], S[2 * (ks + k) + 1], a[k]);
+            }
+            products3<2 * kAtOnce * kRead, 2 * kRead>(d, a, b);
+#pragma unroll
+            for (int k = 0; k < kAtOnce; ++k)
+#pragma unroll
+                for (int t = 0; t < 2 * kRead; ++t)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) x[t][e] = ks + k == 0 ? d[t][e] : x[t][e] + d[k * 2 * kRead + t][e];
+        }
+        // the parts' sums meet, added in the parts' order by all of them; a warp needs those of k and its own tile of q
+#pragma unroll
+        for (int t = 0; t < 2 * kRead; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sums[(warp * 16 + t * 4 + e) * 32] = x[t][e];
+        asm volatile("bar.sync %0, %1;\n" ::"r"(2 + tile), "n"(L::kParts * 32) : "memory");
+        float o[4], y[2][4], u[2][4];
+        auto met = [&](int t, int e) {
+            float v = sums[(tile * 16 + t * 4 + e) * 32];
+#pragma unroll
+            for (int p = 1; p < L::kParts; ++p) v += sums[((p * L::kTiles + tile) * 16 + t * 4 + e) * 32];
+            return v;
+        };
+        const int mt = part & 1;                                // its tile of tokens to read out (parts 0 and 1)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] = met(mt, e);
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                y[t][e] = V[(t * 8 + two + (e & 1)) * L::kVRow + mine + (e >> 1) * 8];
+                if (kCorr) y[t][e] -= met(2 + t, e);
+            }
+        // A later token's value must not reach an earlier read-out through its weight of zero: infinities and values that
+        // are no numbers are left out of the products and brought in one by one.
+        bool odd = false;
+        float clean[2][4];
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const bool fine = fabsf(y[t][e]) <= kLargest;
+                odd |= !fine;
+                clean[t][e] = fine ? y[t][e] : 0.0f;
+            }
+        odd = __any_sync(0xffffffffu, odd);
+        {
+            uint32_t a[1][3][4], b[L::kMats][3][4];             // T's two tiles of tokens and this warp's of Q T, or that of Q
+            const uint32_t mats = stage + L::kMatAt + (((mid >> 1) * 8 + mrow) * kMatRow + (mid & 1) * 8) * 2;
+#pragma unroll
+            for (int m = 0; m < L::kMats; ++m)
+#pragma unroll
+                for (int s = 0; s < 3; ++s) ldmatrix_x4(b[m][s], mats + (m * 3 + s) * L::kMat);
+            if (mt) {
+#pragma unroll
+                for (int s = 0; s < 3; ++s) b[L::kMats - 1][s][0] = b[L::kMats - 1][s][2], b[L::kMats - 1][s][1] = b[L::kMats - 1][s][3];
+            }
+            split_left(clean[0], clean[1], a[0]);
+            float d[kCorr ? 3 : 1][4];
+            products3<kCorr ? 3 : 1, 3>(d, a, b);
+            if (kCorr) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) u[0][e] = d[0][e], u[1][e] = d[kCorr ? 1 : 0][e];
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = kCorr ? o[e] + d[kCorr ? 2 : 0][e] : fmaf(o[e], T[mt * 8 + two + (e & 1)], d[0][e]);
+        }
+        if (!kCorr) {
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) u[t][e] = T[kC + t * 8 + two + (e & 1)] * y[t][e];
+        }
+        if (odd) {
+#pragma unroll
+            for (int j = 0; j < kC; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {                   // the lane's two columns
+                    const float yj = __shfl_sync(0xffffffffu, y[j / 8][2 * h + (j & 1)], (lane & ~3) | (j & 7) >> 1);
+                    if (fabsf(yj) <= kLargest) continue;
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+#pragma unroll
+                        for (int t = 0; t < 2; ++t)
+                            if (kCorr && t * 8 + two + e >= j) u[t][2 * h + e] = fmaf(T[(t * 8 + two + e) * kC + j], yj, u[t][2 * h + e]);
+                        if (mt * 8 + two + e >= j) o[2 * h + e] = fmaf(T[kC * kC + (mt * 8 + two + e) * kC + j], yj, o[2 * h + e]);
                     }
                 }
-#pragma unroll
-                for (int w = 0; w < kSums; ++w)
-#pragma unroll
-                    for (int c = 0; c < NL; ++c) v[w][t * NL + c] = acc[w][c].x + acc[w][c].y;
-            }
-#pragma unroll
-            for (int half = 8; half > 0; half >>= 1) {
-                const bool up = r & half;
-#pragma unroll
-                for (int w = 0; w < kSums; ++w)
-#pragma unroll
-                    for (int i = 0; i < half; ++i) {
-                        const float keep = up ? v[w][i + half] : v[w][i], send = up ? v[w][i] : v[w][i + half];
-                        v[w][i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
-                    }
-            }
-            xq[g] = v[0][0];
-            if (kCorr) xk[g] = v[kSums - 1][0];
         }
-        const int tr = r / NL, myc = cg + r % NL;               // this lane's tokens are kGroup m + tr, its column of the warp's
-        const float* T = s + L::kT;
-        const float* Qm = s + L::kQm;
-        const float* vcol = s + L::kV + warp * kWide + myc;
-        // token j's value as the lane's m-th token sees it: a later one not at all, be it infinite or no number (the delta
-        // rule's whole mixer at 2048 tokens: 510 us, 482 without; the other recurrences take no longer)
-        auto before = [&](float x, int j, int m) -> float { return j >= kGroup * m && j > kGroup * m + tr ? 0.0f : x; };
-        float o[NL];
-        if (kCorr) {
+        if (part < 2) {
 #pragma unroll
-            for (int m = 0; m < NL; ++m) xs[(kGroup * m + tr) * kWide + myc] = vcol[(kGroup * m + tr) * COLS] - xk[m];
-            __syncwarp();
-            float u[NL];
-#pragma unroll
-            for (int m = 0; m < NL; ++m) o[m] = xq[m], u[m] = 0.0f;
-#pragma unroll
-            for (int j = 0; j < kC; j += 4) {
-                const float x0 = xs[j * kWide + myc], x1 = xs[(j + 1) * kWide + myc], x2 = xs[(j + 2) * kWide + myc], x3 = xs[(j + 3) * kWide + myc];
-#pragma unroll
-                for (int m = 0; m < NL; ++m) {
-                    if (kGroup * (m + 1) <= j) continue;        // T and Q T are zero above their diagonals
-                    const float4 t4 = *reinterpret_cast<const float4*>(T + (kGroup * m + tr) * kPad + j);
-                    const float4 q4 = *reinterpret_cast<const float4*>(Qm + (kGroup * m + tr) * kPad + j);
-                    const float y0 = before(x0, j, m), y1 = before(x1, j + 1, m), y2 = before(x2, j + 2, m), y3 = before(x3, j + 3, m);
-                    u[m] = fmaf(t4.x, y0, fmaf(t4.y, y1, fmaf(t4.z, y2, fmaf(t4.w, y3, u[m]))));
-                    o[m] = fmaf(q4.x, y0, fmaf(q4.y, y1, fmaf(q4.z, y2, fmaf(q4.w, y3, o[m]))));
-                }
+            for (int e = 0; e < 4; ++e) {
+                const int i = mt * 8 + two + (e & 1);
+                if (i < n) o_raw[((size_t)(start + c * kC + i) * heads + head) * dv + col0 + mine + (e >> 1) * 8] = o[e];
             }
-#pragma unroll
-            for (int m = 0; m < NL; ++m) us[(kGroup * m + tr) * kWide + myc] = u[m];
-            __syncwarp();
-        } else {
-#pragma unroll
-            for (int m = 0; m < NL; ++m) {
-                o[m] = xq[m] * T[kGroup * m + tr];
-                us[(kGroup * m + tr) * kWide + myc] = T[kPad + kGroup * m + tr] * vcol[(kGroup * m + tr) * COLS];
-            }
-#pragma unroll
-            for (int j = 0; j < kC; j += 4) {
-                float y[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) y[e] = vcol[(j + e) * COLS];
-#pragma unroll
-                for (int m = 0; m < NL; ++m) {
-                    if (kGroup * (m + 1) <= j) continue;
-                    const float4 q4 = *reinterpret_cast<const float4*>(Qm + (kGroup * m + tr) * kPad + j);
-                    o[m] = fmaf(q4.x, before(y[0], j, m), fmaf(q4.y, before(y[1], j + 1, m),
-                           fmaf(q4.z, before(y[2], j + 2, m), fmaf(q4.w, before(y[3], j + 3, m), o[m]))));
-                }
-            }
-            __syncwarp();
         }
-#pragma unroll
-        for (int m = 0; m < NL; ++m)
-            if (kGroup * m + tr < n) o_raw[((size_t)(start + c0 + kGroup * m + tr) * heads + head) * dv + col0 + warp * kWide + myc] = o[m];
         // the state moves on
-        if (kVec) {
+        uint32_t ua[1][3][4];
+        split_left(u[0], u[1], ua[0]);
 #pragma unroll
-            for (int h = 0; h < kH; ++h) {
-                const float4 g4 = *reinterpret_cast<const float4*>(s + L::kGam + 64 * h + 4 * r);
+        for (int ks = 0; ks < L::kKeys / 16; ks += kAtOnce) {
+            uint32_t b[kAtOnce][3][4];
+            float d[2 * kAtOnce][4];
 #pragma unroll
-                for (int c = 0; c < NL; ++c) {
-                    S[c][2 * h] = __fmul2_rn(S[c][2 * h], lo2(g4));
-                    S[c][2 * h + 1] = __fmul2_rn(S[c][2 * h + 1], hi2(g4));
-                }
-            }
-        } else {
-            const float2 g2 = dup(T[kC - 1]);
+            for (int k = 0; k < kAtOnce; ++k)
 #pragma unroll
-            for (int c = 0; c < NL; ++c)
+                for (int s = 0; s < 3; ++s)
+                    ldmatrix_x4_trans(b[k][s], stage + (3 + s) * L::kSplit + at((mid & 1) * 8 + mrow, key0 / 8 + 2 * (ks + k) + (mid >> 1)));
+            products3<2 * kAtOnce, 2 * kAtOnce>(d, ua, b);
 #pragma unroll
-                for (int p = 0; p < kPairs; ++p) S[c][p] = __fmul2_rn(S[c][p], g2);
-        }
-#pragma unroll
-        for (int j = 0; j < kC; ++j) {
-            float2 u2[NL];
-            if (NL == 4) {
-                const float4 u4 = *reinterpret_cast<const float4*>(us + j * kWide + cg);
-                u2[0] = dup(u4.x), u2[1] = dup(u4.y), u2[NL - 2] = dup(u4.z), u2[NL - 1] = dup(u4.w);
-            } else {
-                const float2 u4 = *reinterpret_cast<const float2*>(us + j * kWide + cg);
-                u2[0] = dup(u4.x), u2[1] = dup(u4.y);
-            }
-#pragma unroll
-            for (int h = 0; h < kH; ++h) {
-                const float4 k4 = *reinterpret_cast<const float4*>(s + (kVec ? L::kG : L::kK) + j * DK + 64 * h + 4 * r);
-#pragma unroll
-                for (int c = 0; c < NL; ++c) {
-                    S[c][2 * h] = __ffma2_rn(lo2(k4), u2[c], S[c][2 * h]);
-                    S[c][2 * h + 1] = __ffma2_rn(hi2(k4), u2[c], S[c][2 * h + 1]);
-                }
+            for (int t = 0; t < 2 * kAtOnce; ++t) {
+                float2 g;
+                if (kVec) g = *reinterpret_cast<const float2*>(sm + (c & 1) * L::kStage + L::kGamAt + (key0 + (2 * ks + t) * 8 + two) * 4);
+                else g.x = g.y = T[kC - 1];
+                float (&St)[4] = S[2 * ks + t];
+                St[0] = fmaf(St[0], g.x, d[t][0]), St[1] = fmaf(St[1], g.y, d[t][1]);
+                St[2] = fmaf(St[2], g.x, d[t][2]), St[3] = fmaf(St[3], g.y, d[t][3]);
             }
         }
-        __syncthreads();                                        // the stage may be filled again
+        __syncthreads();                                        // chunk c is done with, chunk c + 1 ready
     }
 #pragma unroll
-    for (int c = 0; c < NL; ++c)
+    for (int t = 0; t < L::kKeys / 8; ++t)
 #pragma unroll
-        for (int h = 0; h < kH; ++h) {
-            state_at(h, 0, c) = S[c][2 * h].x;
-            state_at(h, 1, c) = S[c][2 * h].y;
-            state_at(h, 2, c) = S[c][2 * h + 1].x;
-            state_at(h, 3, c) = S[c][2 * h + 1].y;
-        }
+        for (int e = 0; e < 4; ++e) state_at(t, e) = S[t][e];
 }
 
-template <int DK, int KIND, int COLS, int NL>
+template <int DK, int KIND, int COLS, bool LIGHT>
 static int launch_chunk_scan(const int* seg_info, int segments, const float* qn, const float* kn, const float* vv, const float* decay,
                              const float* pairs, float* state, long long state_stride, int heads, int kv_heads, int dv, float* o_raw,
                              cudaStream_t stream) {
-    constexpr size_t smem = ChunkLayout<DK, KIND, COLS, NL>::kFloats * sizeof(float);
+    using L = ChunkLayout<DK, KIND, COLS, LIGHT>;
     static OncePerDevice configured;
     if (configured.first()) {
-        cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<DK, KIND, COLS, NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<DK, KIND, COLS, LIGHT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
         if (e != cudaSuccess) { set_error("chunk_scan: %s", cudaGetErrorString(e)); return (int)e; }
         configured.done();
     }
-    chunk_scan_kernel<DK, KIND, COLS, NL><<<dim3(heads * (dv / COLS), segments), ChunkLayout<DK, KIND, COLS, NL>::kThreads, smem, stream>>>(
+    chunk_scan_kernel<DK, KIND, COLS, LIGHT><<<dim3(heads * (dv / COLS), segments), L::kThreads, L::kBytes, stream>>>(
         seg_info, qn, kn, vv, decay, pairs, state, state_stride, segments, heads, kv_heads, dv, o_raw);
     return finish_launch("chunk_scan");
 }
@@ -466,18 +631,26 @@ static int launch_chunks(const int* seg_info, int segments, int rows, const floa
                          const float* decay, const float* beta, const float* fgate, float* pairs, float* state,
                          long long state_stride, int heads, int kv_heads, int dv, float* o_raw, cudaStream_t stream) {
     const int each = (rows / kC + segments) / segments;        // chunks of a portion on average: a block each
-    chunk_pairs_kernel<DK, KIND><<<dim3((heads + 3) / 4, segments, each < 65535 ? each : 65535), 128, 0, stream>>>(
-        seg_info, segments, qn, kn, decay, beta, fgate, heads, kv_heads, pairs);
+    if constexpr (KIND == kDelta || KIND == kChannel)
+        chunk_pairs_kernel<DK, KIND><<<dim3((heads + 3) / 4, segments, each < 65535 ? each : 65535), 128, 0, stream>>>(
+            seg_info, segments, qn, kn, decay, beta, heads, kv_heads, pairs);
+    else
+        chunk_scalar_pairs_kernel<DK, KIND><<<dim3((kv_heads + 3) / 4, segments, each < 65535 ? each : 65535), 128, 0, stream>>>(
+            seg_info, segments, qn, kn, beta, fgate, heads, kv_heads, pairs);
     if (int rc = finish_launch("chunk_pairs")) return rc;
-    // Blocks of 32 columns, four per lane, read the tokens' rows from shared memory least often, which is what bounds a full grid
-    // (2048 tokens, 128 x 128, delta rule, with the pairs, from a cold L2: 64 heads 601 us, two per lane 755, blocks of 16 columns
-    // 951 and 794; 32 heads 384, 388, 497 and 411).  Where they would leave a quarter of the multiprocessors without a block, 16
-    // columns, two per lane (16 heads: 235 us against 366; four per lane 359).
+    // Blocks of 32 columns split a head's tokens half as often as blocks of 16, which are for grids that would leave a quarter of
+    // the multiprocessors without a block.  Where there are more blocks than multiprocessors, the light form of the recurrences
+    // with one decay per head holds two on each (three portions of 701 tokens, 32 heads of 128 x 128, constant decays: 189 us
+    // with the pairs against 196; 64 heads, 2048 tokens 324 against 349; a single round of blocks, 32 heads, 202 against 183).
     const int sms = sm_count_cached() > 0 ? sm_count_cached() : 148;
-#define CHUNK_LAUNCH(COLS, NL) \
-    return launch_chunk_scan<DK, KIND, COLS, NL>(seg_info, segments, qn, kn, vv, decay, pairs, state, state_stride, heads, kv_heads, dv, o_raw, stream)
-    if (dv % 32 == 0 && (long long)segments * heads * (dv / 32) * 4 >= 3LL * sms) CHUNK_LAUNCH(32, 4);
-    CHUNK_LAUNCH(16, 2);
+    const long long blocks = (long long)segments * heads * (dv / 32);
+#define CHUNK_LAUNCH(COLS, LIGHT) \
+    return launch_chunk_scan<DK, KIND, COLS, LIGHT>(seg_info, segments, qn, kn, vv, decay, pairs, state, state_stride, heads, kv_heads, dv, o_raw, stream)
+    if (dv % 32 != 0 || blocks * 4 < 3LL * sms) CHUNK_LAUNCH(16, false);
+    if constexpr (KIND == kHead || KIND == kFixed) {
+        if (blocks > sms) CHUNK_LAUNCH(32, true);
+    }
+    CHUNK_LAUNCH(32, false);
 #undef CHUNK_LAUNCH
 }
 
