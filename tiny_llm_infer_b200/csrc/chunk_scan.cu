@@ -66,18 +66,6 @@ __device__ __forceinline__ float halves_sum(float (&v)[N], int lane) {
     return N == 16 ? v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16) : v[0];
 }
 
-__device__ __forceinline__ float low_float(uint32_t p) { return __uint_as_float(p << 16); }
-__device__ __forceinline__ float high_float(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
-
-// Two neighbours in three parts each, packed pairwise.
-__device__ __forceinline__ void split3(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
-    h = pack_bf16(x, y);
-    x -= low_float(h), y -= high_float(h);
-    m = pack_bf16(x, y);
-    x -= low_float(m), y -= high_float(m);
-    l = pack_bf16(x, y);
-}
-
 // The left operand of one step of sixteen terms from two tiles of accumulators.
 __device__ __forceinline__ void split_left(const float (&t0)[4], const float (&t1)[4], uint32_t (&a)[3][4]) {
     split3(t0[0], t0[1], a[0][0], a[1][0], a[2][0]);

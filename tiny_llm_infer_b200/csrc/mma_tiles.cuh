@@ -50,6 +50,19 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// The two bfloat16 numbers of a packed pair.
+__device__ __forceinline__ float low_float(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float high_float(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+
+// Two neighbours as sums of three bfloat16 parts each (all 24 bits of them), packed pairwise.
+__device__ __forceinline__ void split3(float x, float y, uint32_t& h, uint32_t& m, uint32_t& l) {
+    h = pack_bf16(x, y);
+    x -= low_float(h), y -= high_float(h);
+    m = pack_bf16(x, y);
+    x -= low_float(m), y -= high_float(m);
+    l = pack_bf16(x, y);
+}
+
 // A tile of rows of HD bf16 (HD * 2 bytes per row, HD a multiple of 64) in shared memory.
 // The 16-byte chunk c of row r lives at chunk c ^ (r & 7): eight rows read at the same
 // logical chunk (one ldmatrix phase) fall into eight different bank groups.

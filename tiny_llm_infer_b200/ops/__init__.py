@@ -9,7 +9,8 @@ bfloat16, chosen by the number of rows: up to 8 the weight-streaming mma.sync pr
 (``gemm_tcgen05``).  Everything else is the library's (cuBLAS through ``torch.mm``), as in the reference, which calls
 ``cublasHgemm`` for every projection with more than one row
 (kernels/src/matmul_kernel_cuda.cu:83-91); in float32 mode it runs with the
-reduced-precision matrix modes switched off.
+reduced-precision matrix modes switched off, and large products run on the tensor cores with every operand in three
+bfloat16 parts (``gemm_f32_tcgen05``), closer to 64 bits than the library's.
 """
 from __future__ import annotations
 
@@ -121,6 +122,7 @@ def _declare(h) -> None:
         "tllm_gemm_skinny": [vp, vp, vp, i32, i32, i32, i32, vp],
         "tllm_gemm_plain": [vp, i32, vp, i32, vp, i32, i32, i32, i32, vp],
         "tllm_gemm_tcgen05": [vp, vp, vp, i32, i32, i32, i32, f32, f32, vp, vp],
+        "tllm_gemm_f32_tcgen05": [vp, vp, vp, i32, i32, i32, i32, vp, vp, vp],
         "tllm_gemm_skinny_swiglu": [vp, vp, vp, i32, i32, i32, i32, f32, f32, vp],
         "tllm_gemm_skinny_act": [vp, vp, vp, i32, i32, i32, i32, vp],
         "tllm_paged_attention_decode_rows": [vp, vp, vp, vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, f32,
@@ -651,6 +653,50 @@ def gemm_tcgen05(x: torch.Tensor, weight: torch.Tensor, swiglu: bool = False, sh
     return y
 
 
+def f32_splits(rows: int, out_cols: int, k: int) -> int:
+    """Shares of K in ``gemm_f32_tcgen05``: tiles of 128 x 128 go to one block per SM, so K is cut where few tiles would leave
+    SMs idle, as far as the saved rounds outweigh the second kernel that adds the shares (a slab of 64 takes 1.65 us, the
+    shares 3 us and their bytes at 5 TB/s)."""
+    tiles, slabs = -(-rows // 128) * -(-out_cols // 128), -(-k // 64)
+
+    def us(s):
+        each = -(-slabs // s)
+        used = -(-slabs // each)
+        return -(-tiles * used // SM_COUNT) * each * 1.65 + (0.0 if used == 1 else 3.0 + (2 * used + 1) * rows * out_cols * 4 / 5e6)
+    return min(range(1, min(slabs, 16) + 1), key=us)
+
+
+def f32_tcgen05_pays(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether a float32 product runs on the tensor cores rather than in the library: enough work for their start, and operands in
+    16-byte pieces.  The library's kernel and this one, rows x columns x K: 64 x 1024 x 2048 37 and 28 us, 64 x 4096 x 4096 78 and
+    38, 128 x 4096 x 1024 32 and 30 (64 rows 23 and 28), 595 x 4096 x 1024 123 and 62, 595 x 1024 x 2048 87 and 33,
+    2048 x 24576 x 4096 6955 and 2223; 595 x 96 x 64 11 and 12.  (With fewer rows it is ahead only from K = 3072 on.)"""
+    rows, k = x.shape
+    n = weight.shape[0]
+    return (rows >= 64 and rows * n * k >= (1 << 29 if k <= 1024 else 1 << 27) and k % 4 == 0 and n % 4 == 0
+            and x.is_contiguous() and weight.is_contiguous() and (x.data_ptr() | weight.data_ptr()) % 16 == 0
+            and not (x.requires_grad or weight.requires_grad))
+
+
+def gemm_f32_tcgen05(x: torch.Tensor, weight: torch.Tensor, splits: Optional[int] = None) -> torch.Tensor:
+    """y = x . weight^T in float32 on tcgen05 tensor cores, both operands as sums of three bfloat16 parts
+    (csrc/gemm_f32.cu)."""
+    _cuda(x, weight)
+    rows, k = x.shape
+    n = weight.shape[0]
+    assert weight.shape[1] == k and x.dtype == weight.dtype == torch.float32
+    y = torch.empty((rows, n), dtype=torch.float32, device=x.device)
+    if rows == 0:
+        return y
+    splits = f32_splits(rows, n, k) if splits is None else splits
+    shares = torch.empty(splits * rows * n, dtype=torch.float32, device=x.device) if splits > 1 else None
+    global tcgen05_calls
+    tcgen05_calls += 1
+    _check(lib().tllm_gemm_f32_tcgen05(_p(x), _p(weight), _p(y), rows, n, k, splits, _p(shares), _p(error_word(x.device)), _stream()),
+           "gemm_f32_tcgen05", kernels=2 if splits > 1 else 1)
+    return y
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None,
            bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y[T, N] = x[T, K] . weight[N, K]^T with float32 accumulation.  A weight kept in
@@ -667,7 +713,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     if weight.dtype == torch.float32:
         if torch.backends.cuda.matmul.allow_tf32 or torch.get_float32_matmul_precision() != "highest":
             raise KernelError("float32 products need the reduced-precision matrix modes off")
-        y = torch.mm(cast(x, torch.float32), weight.t())
+        x = cast(x, torch.float32)
+        y = gemm_f32_tcgen05(x, weight) if f32_tcgen05_pays(x, weight) else torch.mm(x, weight.t())
         return y if want == torch.float32 else cast(y, want)
     if x.dtype != weight.dtype:
         x = cast(x, weight.dtype)
