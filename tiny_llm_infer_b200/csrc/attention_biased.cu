@@ -1143,6 +1143,205 @@ attention_biased_decode_kernel(const bf16* q, const bf16* k_plane, const bf16* v
     }
 }
 
+// ---------------------------------------------------------------- one-token rows of few heads per key/value head
+// The same attention where at most eight query heads share a key/value head, one map, keys and values of HD = 64 or 128 and
+// pages of whole sixteens of keys.  The kernel above puts the heads into the 16 rows of the MMA's left operand, half or
+// more of which are then empty, and makes each warp execute some 1300 instructions for its 16 keys: with 194 registers and two
+// blocks per multiprocessor it issued 40% of the time and moved 3.0 TB/s (64 rows of contexts 1000 to 2000, 32 heads on 8 of 128, cap,
+// window, sink and gate: 134 us).  Here the keys are the left operand (16 keys x 8 heads: S^T = K Q^T, O^T = V^T P^T, the
+// weights turned round by movmatrix), so that nothing is computed twice or for no head; a warp walks 16-key tiles of its own
+// through a ring of its own, one page look-up each, with no barrier between the warps; the sums are scaled only when a
+// maximum rises.  The same step takes 79 us, 5.0 TB/s; what is left is its last blocks (512 on 444 places) and a tile ahead per warp.
+__device__ __forceinline__ uint32_t transposed_8x8(uint32_t x) {
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
+    return y;
+}
+
+constexpr int kFewWarps = 4, kFewKeys = 16, kFewStages = 2;
+
+template <int HD>
+__global__ void __launch_bounds__(kFewWarps * 32, 3)
+attention_biased_decode_few_kernel(const bf16* q, const bf16* k_plane, const bf16* v_plane, long long page_stride,
+                                   const int* __restrict__ positions, const int* __restrict__ token_slot,
+                                   const int* __restrict__ rows, const int* __restrict__ block_table, int max_pages,
+                                   int page_size, int page_shift, int q_heads, int kv_heads, ScoreMod mod,
+                                   const float* __restrict__ slopes, const float* __restrict__ sink_logit, int v_row,
+                                   const bf16* gate, int gate_stride, int splits, int sub_groups, float* part, bf16* __restrict__ out) {
+    extern __shared__ __align__(128) unsigned char pf_smem[];
+    TLLM_PDL_ENTER();
+    constexpr int kTileBytes = kFewKeys * HD * 2, kPieces = HD / 8, kRec = HD + 2;
+    const int t = rows != nullptr ? rows[blockIdx.x] : blockIdx.x;
+    const int g = blockIdx.y / sub_groups, split = blockIdx.z, group = q_heads / kv_heads / sub_groups;
+    const int head0 = g * (q_heads / kv_heads) + (blockIdx.y % sub_groups) * group;
+    const int slot = token_slot[t];
+    if (slot < 0) {
+        if (splits == 1)
+            for (int i = threadIdx.x; i < group * HD; i += blockDim.x) out[((size_t)t * q_heads + head0) * HD + i] = __float2bfloat16_rn(0.0f);
+        return;                       // the combining kernel writes the zeros of a row without a request
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, mid = lane >> 3, mrow = lane & 7;
+    const int pos = positions[t], lo = first_key(pos, mod);
+    const int* table = block_table + (size_t)slot * max_pages;
+    int kt_first = lo / kPfN, kt_last = pos / kPfN;                    // runs are cut at multiples of 64 keys, as above
+    if (splits > 1) {
+        const int per = (kt_last - kt_first + splits) / splits;
+        kt_first += split * per;
+        kt_last = min(kt_last, kt_first + per - 1);
+    }
+    const int k_first = max(lo, kt_first * kPfN), k_last = min(pos, kt_last * kPfN + kPfN - 1);      // the run's keys
+    const int last_tile = k_last >= k_first ? k_last / kFewKeys : -1;
+
+    // this lane's heads are 2 (lane % 4) and the next, its keys of a tile lane / 4 and eight further
+    const int h0 = (lane & 3) * 2;
+    const bool live[2] = {h0 < group, h0 + 1 < group};
+    float slope[2], m[2], l[2] = {0.0f, 0.0f};
+    const bool first = mod.sink && warp == 0 && split == 0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        slope[e] = slopes != nullptr && live[e] ? slopes[head0 + h0 + e] * kLog2e : 0.0f;
+        m[e] = first ? (sink_logit != nullptr && live[e] ? sink_logit[head0 + h0 + e] * kLog2e : 0.0f) : -INFINITY;
+        if (first && lane < 4) l[e] = 1.0f;
+    }
+    const float inv_cap = mod.softcap > 0.0f ? 1.0f / mod.softcap : 0.0f;
+    uint32_t qb[HD / 16][2];                                            // right operand: column lane / 4 is a head
+    const bf16* q_row = q + ((size_t)t * q_heads + head0 + (lane >> 2)) * HD;
+#pragma unroll
+    for (int ks = 0; ks < HD / 16; ++ks) {
+        qb[ks][0] = (lane >> 2) < group ? *reinterpret_cast<const uint32_t*>(q_row + ks * 16 + h0) : 0u;
+        qb[ks][1] = (lane >> 2) < group ? *reinterpret_cast<const uint32_t*>(q_row + ks * 16 + h0 + 8) : 0u;
+    }
+    float o[HD / 16][4];
+#pragma unroll
+    for (int i = 0; i < HD / 16; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
+
+    unsigned char* ring = pf_smem + warp * (kFewStages * 2 * kTileBytes);
+    auto issue = [&](int tile, int stage) {
+        if (tile <= last_tile) {
+            const int key0 = tile * kFewKeys;
+            int page_index, place;
+            page_of(key0, page_size, page_shift, page_index, place);    // a tile lies within a page
+            const int page = table[page_index];
+            const bool whole = page >= 0 && key0 >= k_first && key0 + kFewKeys - 1 <= k_last;
+            const long long in_page = (long long)g * page_size + place;
+            const int row = lane / kPieces, piece = lane % kPieces;
+            const bf16* kp = k_plane + (page >= 0 ? page * page_stride + (in_page + row) * HD + piece * 8 : 0);
+            const bf16* vp = v_plane + (page >= 0 ? page * page_stride + (in_page + row) * v_row + piece * 8 : 0);
+            const uint32_t ks = smem_u32(ring + stage * 2 * kTileBytes), vs = ks + kTileBytes;
+            constexpr int kStep = 32 / kPieces;                         // rows per round
+#pragma unroll
+            for (int i = 0; i < kFewKeys / kStep; ++i) {
+                const int key = key0 + row + i * kStep;
+                const bool ok = whole || (page >= 0 && key >= k_first && key <= k_last);
+                cp_async_16(ks + swizzled<HD>(row + i * kStep, piece), ok ? kp + i * kStep * HD : k_plane, ok);
+                cp_async_16(vs + swizzled<HD>(row + i * kStep, piece), ok ? vp + (long long)i * kStep * v_row : v_plane, ok);
+            }
+        }
+        cp_async_commit();
+    };
+
+    int tile = k_first / kFewKeys + warp;
+#pragma unroll
+    for (int st = 0; st < kFewStages - 1; ++st) issue(tile + st * kFewWarps, st);
+    for (int stage = 0; tile <= last_tile; tile += kFewWarps, stage = stage + 1 == kFewStages ? 0 : stage + 1) {
+        issue(tile + (kFewStages - 1) * kFewWarps, stage == 0 ? kFewStages - 1 : stage - 1);
+        cp_async_wait<kFewStages - 1>();
+        __syncwarp();
+        const uint32_t ks_base = smem_u32(ring + stage * 2 * kTileBytes), vs_base = ks_base + kTileBytes;
+        float sc[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}};      // two chains of half the width
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks) {
+            uint32_t ka[4];
+            ldmatrix_x4(ka, ks_base + swizzled<HD>((mid & 1) * 8 + mrow, 2 * ks + (mid >> 1)));
+            mma_bf16_16816(sc[ks & 1], ka, qb[ks]);
+        }
+        const int key0 = tile * kFewKeys + (lane >> 2);
+        const bool inner = tile * kFewKeys >= k_first && tile * kFewKeys + kFewKeys - 1 <= k_last;
+        float s[4], top[2];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {                                   // key0 + 8 (i / 2), head h0 + i % 2
+            const int j = key0 + (i >> 1) * 8, e = i & 1;
+            float v = mod_score_fast(sc[0][i] + sc[1][i], slope[e], (float)(pos - j), mod, inv_cap);
+            if (mod.dist_bias != nullptr) v += dist_bias_of(mod, head0 + (live[e] ? h0 + e : 0), pos - j) * kLog2e;
+            s[i] = live[e] && (inner || (j >= k_first && j <= k_last)) ? v : -INFINITY;
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            top[e] = fmaxf(s[e], s[2 + e]);
+#pragma unroll
+            for (int x = 4; x < 32; x <<= 1) top[e] = fmaxf(top[e], __shfl_xor_sync(0xffffffffu, top[e], x));
+            top[e] = fmaxf(top[e], m[e]);
+        }
+        if (__any_sync(0xffffffffu, top[0] > m[0] || top[1] > m[1])) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float c = top[e] == -INFINITY ? 1.0f : fast_exp2(m[e] - top[e]);      // 2^-inf = 0 before the first key
+                m[e] = top[e];
+                l[e] *= c;
+#pragma unroll
+                for (int i = 0; i < HD / 16; ++i) { o[i][e] *= c; o[i][2 + e] *= c; }
+            }
+        }
+        float p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            p[i] = fast_exp2(s[i] - (m[i & 1] == -INFINITY ? 0.0f : m[i & 1]));
+            l[i & 1] += p[i];
+        }
+        const uint32_t pb[2] = {transposed_8x8(pack_bf16(p[0], p[1])), transposed_8x8(pack_bf16(p[2], p[3]))};
+#pragma unroll
+        for (int c = 0; c < HD / 16; ++c) {
+            uint32_t va[4];
+            ldmatrix_x4_trans(va, vs_base + swizzled<HD>((mid >> 1) * 8 + mrow, 2 * c + (mid & 1)));
+            mma_bf16_16816(o[c], va, pb);
+        }
+        __syncwarp();                                                   // the tile's place may be filled again
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int x = 4; x < 32; x <<= 1) l[e] += __shfl_xor_sync(0xffffffffu, l[e], x);
+    __syncthreads();
+    // the warps meet: [warp][head][HD + 2] floats over the rings
+    float* meet = reinterpret_cast<float*>(pf_smem);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        if (!live[e]) continue;
+        float* d = meet + ((size_t)warp * group + h0 + e) * kRec;
+#pragma unroll
+        for (int i = 0; i < HD / 16; ++i) {
+            d[i * 16 + (lane >> 2)] = o[i][e];
+            d[i * 16 + (lane >> 2) + 8] = o[i][2 + e];
+        }
+        if (lane < 4) { d[HD] = m[e]; d[HD + 1] = l[e]; }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < group * HD; i += blockDim.x) {
+        const int h = i / HD, e = i % HD;
+        float mm = -INFINITY, total = 0.0f, v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kFewWarps; ++w) mm = fmaxf(mm, meet[((size_t)w * group + h) * kRec + HD]);
+#pragma unroll
+        for (int w = 0; w < kFewWarps; ++w) {
+            const float* src = meet + ((size_t)w * group + h) * kRec;
+            const float wt = src[HD] == -INFINITY ? 0.0f : fast_exp2(src[HD] - mm);
+            total += src[HD + 1] * wt;
+            v += src[e] * wt;
+        }
+        if (splits > 1) {                                               // as the kernel above leaves them
+            float* dst = part + (((size_t)blockIdx.x * q_heads + head0 + h) * splits + split) * kRec;
+            dst[e] = v;
+            if (e == 0) { dst[HD] = mm; dst[HD + 1] = total; }
+            continue;
+        }
+        v = total > 0.0f ? v / total : 0.0f;
+        if (gate != nullptr)
+            v *= 1.0f / (1.0f + expf(-__bfloat162float(gate[(size_t)t * gate_stride + gate_at(mod.gate_per_head, head0 + h, HD, e)])));
+        out[((size_t)t * q_heads + head0 + h) * HD + e] = __float2bfloat16_rn(v);
+    }
+}
+
 // The runs of a (row, head) added in their order (with two maps: of both, then the normed difference), the gate
 // applied, the result written.
 template <int MAPS>
@@ -1199,6 +1398,29 @@ static int biased_sub_groups(int group, int maps) {
     for (int s = 1; s <= group; ++s)
         if (group % s == 0 && group / s * maps <= 16) return s;
     return 0;
+}
+
+template <int HD>
+static int launch_biased_decode_few(const void* q, const void* kp, const void* vp, long long page_stride, const int* positions,
+                                    const int* token_slot, const int* rows, int n_rows, const int* block_table, int max_pages,
+                                    int page_size, int q_heads, int kv_heads, ScoreMod mod, const float* slopes, const float* sink_logit,
+                                    int v_row, const void* gate, int gate_stride, int splits, float* part, void* out, cudaStream_t stream) {
+    constexpr size_t kRings = (size_t)kFewWarps * kFewStages * 2 * kFewKeys * HD * 2, kMeet = (size_t)kFewWarps * 8 * (HD + 2) * 4;
+    constexpr size_t smem = kRings > kMeet ? kRings : kMeet;
+    static OncePerDevice configured;
+    if (configured.first()) {
+        cudaError_t e = cudaFuncSetAttribute(attention_biased_decode_few_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) { set_error("attention_biased_decode: %s", cudaGetErrorString(e)); return (int)e; }
+        configured.done();
+    }
+    int sub_groups = biased_sub_groups(q_heads / kv_heads, 1);
+    launch_pdl(kPdlAttention, attention_biased_decode_few_kernel<HD>, dim3(n_rows, kv_heads * sub_groups, splits), dim3(kFewWarps * 32), smem, stream,
+               (const bf16*)q, (const bf16*)kp, (const bf16*)vp, page_stride, positions, token_slot, rows, block_table, max_pages, page_size,
+               page_shift_of(page_size), q_heads, kv_heads, mod, slopes, sink_logit, v_row, (const bf16*)gate, gate_stride, splits, sub_groups, part, (bf16*)out);
+    if (splits > 1)
+        launch_pdl(kPdlCombine, attention_biased_combine_kernel<1>, dim3(n_rows, q_heads), dim3(HD), 0, stream, (const float*)part, token_slot, rows,
+                   q_heads, HD, splits, (const bf16*)gate, gate_stride, mod.gate_per_head, DiffMod{0.0f, 0.0f, 0.0f}, (bf16*)out);
+    return finish_launch("attention_biased_decode");
 }
 
 template <int DKP, int DVP, int MAPS>
@@ -1377,6 +1599,12 @@ int tllm_attention_biased_decode(
     TLLM_REQUIRE(splits >= 1 && splits <= 64 && (splits == 1 || part != nullptr), "attention_biased_decode: %d runs of keys", splits);
     if (n_rows == 0) return 0;
     const ScoreMod mod{scale, softcap, chunk, window, sink ? 1 : 0, dist_bias, dist_len, gate_per_head ? 1 : 0};
+    const int sub = biased_sub_groups(q_heads / kv_heads, 1);
+    if (maps == 1 && dk == dv && (dk == 64 || dk == 128) && sub > 0 && q_heads / kv_heads / sub <= 8 && page_size % kFewKeys == 0)
+        return dk == 128 ? launch_biased_decode_few<128>(q, k_plane, v_plane, page_stride, positions, token_slot, rows, n_rows, block_table, max_pages,
+                                                         page_size, q_heads, kv_heads, mod, slopes, sink_logit, v_row, gate, gate_stride, splits, part, out, stream)
+                         : launch_biased_decode_few<64>(q, k_plane, v_plane, page_stride, positions, token_slot, rows, n_rows, block_table, max_pages,
+                                                        page_size, q_heads, kv_heads, mod, slopes, sink_logit, v_row, gate, gate_stride, splits, part, out, stream);
 #define DEC_M(A, B, M) launch_biased_decode<A, B, M>(q, k_plane, v_plane, page_stride, positions, token_slot, rows, n_rows, block_table, \
                                              max_pages, page_size, q_heads, kv_heads, dk, dv, mod, diff, slopes, sink_logit, v_row, gate, gate_stride, \
                                              splits, part, out, stream)
