@@ -857,35 +857,57 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
 
 // out[row, head, :] = sum_z O_z 2^(m_z - M) / sum_z l_z 2^(m_z - M) over the runs of keys, in
 // index order; a run that held no key for the row has m = -inf and is passed over.  A block
-// takes kCombineRows rows of one entry of the tile list and one head.
-constexpr int kCombineRows = 8;
-__global__ void paged_attention_prefill_combine_kernel(const float* part_o, const float* part_ml,
-                                                       const int* __restrict__ seg_info,
-                                                       const int* __restrict__ tiles, int rows_per_tile,
-                                                       int q_heads, int splits, const float* __restrict__ sink_logit,
-                                                       const Changes ch, bf16* __restrict__ out) {
-    const int seg = tiles[2 * blockIdx.x], q_off = tiles[2 * blockIdx.x + 1], head = blockIdx.y, d = threadIdx.x;
+// takes kCombineRows rows of one entry of the tile list and one head, a warp a row; what eight runs left of it is on its way
+// at once.  (One row of a block after the other, a thread per column and run after run, took 14.4 us for 509 rows of 32 heads
+// in two runs, 21 MB.)
+constexpr int kCombineRows = 8, kMaxRuns = 8;
+__global__ void __launch_bounds__(kCombineRows * 32)
+paged_attention_prefill_combine_kernel(const float* part_o, const float* part_ml, const int* __restrict__ seg_info,
+                                       const int* __restrict__ tiles, int rows_per_tile, int q_heads, int splits,
+                                       const float* __restrict__ sink_logit, const Changes ch, bf16* __restrict__ out) {
+    const int seg = tiles[2 * blockIdx.x], q_off = tiles[2 * blockIdx.x + 1], head = blockIdx.y;
     const int start = seg_info[4 * seg + 1], len = seg_info[4 * seg + 2];
-    for (int i = 0; i < kCombineRows; ++i) {
-        const int r = q_off + blockIdx.z * kCombineRows + i;
-        if (r >= len || r >= q_off + rows_per_tile) return;
-        const size_t base = ((size_t)(start + r) * q_heads + head) * splits;
-        float mm = -INFINITY;
-        for (int z = 0; z < splits; ++z) mm = fmaxf(mm, part_ml[(base + z) * 2]);
-        float total = 0.0f, acc = 0.0f;
-        for (int z = 0; z < splits; ++z) {
-            const float mz = part_ml[(base + z) * 2];
-            if (mz == -INFINITY) continue;
-            const float f = exp2f(mz - mm);
-            total += part_ml[(base + z) * 2 + 1] * f;
-            acc += part_o[(base + z) * kHD + d] * f;
+    const int r = q_off + blockIdx.z * kCombineRows + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= len || r >= q_off + rows_per_tile) return;
+    const size_t base = ((size_t)(start + r) * q_heads + head) * splits;
+    float2 ml[kMaxRuns];
+    float4 o[kMaxRuns];
+    auto fetch = [&](int z0) {
+#pragma unroll
+        for (int z = 0; z < kMaxRuns; ++z) {
+            const bool in = z0 + z < splits;
+            ml[z] = in ? *reinterpret_cast<const float2*>(part_ml + (base + z0 + z) * 2) : make_float2(-INFINITY, 0.0f);
+            o[z] = in ? *reinterpret_cast<const float4*>(part_o + (base + z0 + z) * kHD + lane * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
-        if (sink_logit != nullptr) total += exp2f(sink_logit[head] * kLog2e - mm);
-        else if (ch.sink) total += exp2f(-mm);
-        float v = acc / total;
-        if (ch.gate != nullptr) v *= sigmoid_of(ch.gate[(size_t)(start + r) * ch.gate_stride + (ch.gate_per_head ? head : head * kHD + d)]);
-        out[((size_t)(start + r) * q_heads + head) * kHD + d] = __float2bfloat16_rn(v);
+    };
+    fetch(0);
+    float mm = -INFINITY, total = 0.0f;
+#pragma unroll
+    for (int z = 0; z < kMaxRuns; ++z) mm = fmaxf(mm, ml[z].x);
+    for (int z = kMaxRuns; z < splits; ++z) mm = fmaxf(mm, part_ml[(base + z) * 2]);
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int z0 = 0; z0 < splits; z0 += kMaxRuns) {
+        if (z0 > 0) fetch(z0);
+#pragma unroll
+        for (int z = 0; z < kMaxRuns; ++z) {
+            if (ml[z].x == -INFINITY) continue;
+            const float f = exp2f(ml[z].x - mm);
+            total += ml[z].y * f;
+            acc.x += o[z].x * f; acc.y += o[z].y * f; acc.z += o[z].z * f; acc.w += o[z].w * f;
+        }
     }
+    if (sink_logit != nullptr) total += exp2f(sink_logit[head] * kLog2e - mm);
+    else if (ch.sink) total += exp2f(-mm);
+    float v[4] = {acc.x / total, acc.y / total, acc.z / total, acc.w / total};
+    if (ch.gate != nullptr) {
+        const bf16* g = ch.gate + (size_t)(start + r) * ch.gate_stride + (ch.gate_per_head ? head : head * kHD + lane * 4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] *= sigmoid_of(g[ch.gate_per_head ? 0 : e]);
+    }
+    uint2 raw;
+    *reinterpret_cast<__nv_bfloat162*>(&raw.x) = __floats2bfloat162_rn(v[0], v[1]);
+    *reinterpret_cast<__nv_bfloat162*>(&raw.y) = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(out + ((size_t)(start + r) * q_heads + head) * kHD + lane * 4) = raw;
 }
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -980,7 +1002,7 @@ static int launch_prefill_tc(const char* name, const void* q, int tokens, const 
 #undef PFTC
     int rc = finish_launch(name);
     if (rc != 0 || splits == 1) return rc;
-    pftc::paged_attention_prefill_combine_kernel<<<dim3(n_tiles, q_heads, rows_per_tile / pftc::kCombineRows), 128, 0, stream>>>(
+    pftc::paged_attention_prefill_combine_kernel<<<dim3(n_tiles, q_heads, rows_per_tile / pftc::kCombineRows), pftc::kCombineRows * 32, 0, stream>>>(
         part_o, part_ml, seg_info, tiles, rows_per_tile, q_heads, splits, sink_logit, ch, (bf16*)out);
     return finish_launch("paged_attention_prefill_combine");
 }
