@@ -564,10 +564,10 @@ def skinny_pays(x: torch.Tensor, weight: torch.Tensor, gated: bool = False) -> b
     down 6.1 against 8.8), more are not (8B sizes: q/k/v 16.9 against 12.2, gate/up 48 against 36); a gated product also
     saves the activation's kernel, which pays for half a round more (6.4 against 8.6; 8B sizes 49 against 41)."""
     rows, k = x.shape
-    if k % 8 or not x.is_contiguous() or not weight.is_contiguous():
+    if not 0 < rows <= SKINNY_WIDE_ROWS or k % 8 or not x.is_contiguous() or not weight.is_contiguous():
         return False
     blocks = -(-weight.shape[0] // 16)
-    return 0 < rows <= SKINNY_MAX_ROWS or (0 < rows <= SKINNY_WIDE_ROWS and blocks <= SM_COUNT * (3 if gated else 2)
+    return rows <= SKINNY_MAX_ROWS or (blocks <= SM_COUNT * (3 if gated else 2)
                                            and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
 
 
