@@ -1100,7 +1100,8 @@ CHUNK_MODES = (SCAN_DELTA, SCAN_PLAIN, SCAN_HEAD_DECAY, SCAN_FIXED_DECAY)      #
 # are two kernels and less work.  The delta rule with 32 heads of 128 x 128, token by token and by chunks: one portion of 64
 # tokens 27 and 32 us, of 256 80 and 65; eight of 48 tokens 82 and 77, of 64 104 and 91.  Between the lines both take some 40 us,
 # and the second launch costs more than it saves (four portions of 90 tokens, 16 heads of 64 x 128: 29 and 30 us, of the whole
-# op 40 and 48).
+# op 40 and 48).  The chunks' figures are those of their float32-pipe kernels; on the tensor cores portions of 2048 tokens take three
+# quarters of the time, one portion of 100 tokens as long (37.7 us against 36.9), so the lines stay.
 CHUNK_TOKENS = 64
 
 
