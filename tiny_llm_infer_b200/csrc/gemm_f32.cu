@@ -27,19 +27,6 @@ constexpr int kFTile = 128, kFK = 64, kFStages = 2, kFPart = kFTile * kFK * 2, k
 constexpr int kFSplitters = 256, kFAdders = 256, kFThreads = kFSplitters + kFAdders + 32;
 constexpr int kFTogether = 2;                // slabs whose products meet in one pair of accumulators (128 terms)
 
-struct F32Wait {
-    volatile int* aborted;
-    int* error_word;
-    // Waits (bounded) for a phase; false, with the error word set, when the limit ran out or another warp gave up.
-    __device__ __forceinline__ bool operator()(uint64_t* bar, uint32_t parity, int code) const {
-        if (!mbar_wait(bar, parity)) {
-            atomicExch(error_word, code);
-            *aborted = 1;
-        }
-        return !*aborted;
-    }
-};
-
 __global__ void __launch_bounds__(kFThreads, 1)
 gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K, int tiles_m,
                         int tiles, int splits, int slabs_each, int* __restrict__ error_word) {
@@ -71,7 +58,7 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = tmem_base_slot;
-    const F32Wait wait{&abort_flag, error_word};
+    volatile int* aborted = &abort_flag;
     // unit u: tile u % tiles (rows of x fastest), share u / tiles of its slabs
     auto slabs_of = [&](int u) { return min(slabs_each, all_slabs - u / tiles * slabs_each); };
 
@@ -94,12 +81,13 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
             }
         };
         int it = 0;
+        bool alive = true;
         if ((int)blockIdx.x < units) fetch(blockIdx.x, 0);
-        for (int u = blockIdx.x; u < units && !abort_flag; u += gridDim.x) {
+        for (int u = blockIdx.x; u < units && alive; u += gridDim.x) {
             const int slabs = slabs_of(u);
             for (int slab = 0; slab < slabs; ++slab, ++it) {
                 const int s = it % kFStages;
-                if (it >= kFStages && !wait(&empty_bar[s], ((it / kFStages) - 1) & 1, 11)) break;
+                if (it >= kFStages && !warp_wait(&empty_bar[s], ((it / kFStages) - 1) & 1, aborted, error_word, 11)) { alive = false; break; }
                 unsigned char* stage = ring + s * kFStage;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -126,9 +114,16 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
             constexpr uint32_t idesc = instr_desc_bf16(kFTile, kFTile);
             constexpr int kLeft[6] = {2, 0, 1, 1, 0, 0}, kRight[6] = {0, 2, 1, 0, 1, 0};
             int it = 0, group = 0;
-            for (int u = blockIdx.x; u < units && !abort_flag; u += gridDim.x) {
+            const auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+                if (!mbar_wait(bar, parity)) {
+                    atomicExch(error_word, code);
+                    *aborted = 1;
+                }
+                return !*aborted;
+            };
+            for (int u = blockIdx.x; u < units && !*aborted; u += gridDim.x) {
                 const int slabs = slabs_of(u);
-                for (int slab = 0; slab < slabs && !abort_flag; slab += kFTogether, ++group) {
+                for (int slab = 0; slab < slabs && !*aborted; slab += kFTogether, ++group) {
                     const int buf = group & 1;
                     if (group >= 2 && !wait(&acc_empty[buf], ((group >> 1) - 1) & 1, 14)) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -148,7 +143,7 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
                     umma_commit(&acc_full[buf]);
                 }
             }
-            if (abort_flag) {                        // do not leave while products are in flight
+            if (*aborted) {                          // do not leave while products are in flight
                 umma_commit(&drained);
                 mbar_wait(&drained, 0);
             }
@@ -157,14 +152,15 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
         // ------------------------------------------------------------ add the accumulators up (a row and 64 columns per thread)
         const int quad = warp & 3, half = (warp >> 2) & 1;
         int group = 0;
-        for (int u = blockIdx.x; u < units && !abort_flag; u += gridDim.x) {
+        bool alive = true;
+        for (int u = blockIdx.x; u < units; u += gridDim.x) {
             const int slabs = slabs_of(u);
             float sum[64];
 #pragma unroll
             for (int i = 0; i < 64; ++i) sum[i] = 0.0f;
             for (int slab = 0; slab < slabs; slab += kFTogether, ++group) {
                 const int buf = group & 1;
-                if (!wait(&acc_full[buf], (group >> 1) & 1, 13)) break;
+                if (!warp_wait(&acc_full[buf], (group >> 1) & 1, aborted, error_word, 13)) { alive = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t from = tmem + buf * 256 + half * 64 + ((uint32_t)(quad * 32) << 16);
 #pragma unroll
@@ -181,7 +177,7 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&acc_empty[buf]);
             }
-            if (abort_flag) break;
+            if (!alive) break;
             const int tile = u % tiles, row = tile % tiles_m * kFTile + quad * 32 + lane, col0 = tile / tiles_m * kFTile + half * 64;
             if (row < M) {
                 float* dst = y + ((size_t)(u / tiles) * M + row) * N + col0;

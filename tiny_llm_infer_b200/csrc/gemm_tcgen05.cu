@@ -229,12 +229,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
             const int buf = local % kNumBuf;
             const int tile_m = t % tiles_m, tile_n = t / tiles_m;
             const int row_base = tile_m * kRows;
-            const bool ready = mbar_wait(&acc_full[buf], (local / kNumBuf) & 1);
-            if (!ready) {
-                if (lane == 0) atomicExch(error_word, 3);
-                *aborted = 1;
-            }
-            if (*aborted) break;
+            if (!warp_wait(&acc_full[buf], (local / kNumBuf) & 1, aborted, error_word, 3)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll 1
             for (int mt = 0; mt < MT; ++mt) {
@@ -481,11 +476,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             const int tile = t / tiles_n, row0 = lists.tile_row0[tile];
             const int rows = min(tile_rows, lists.offsets[lists.tile_expert[tile] + 1] - row0);
             const int buf = local & 1;
-            if (!mbar_wait(&acc_full[buf], (local >> 1) & 1)) {
-                if (lane == 0) atomicExch(error_word, 3);
-                *aborted = 1;
-            }
-            if (*aborted) break;
+            if (!warp_wait(&acc_full[buf], (local >> 1) & 1, aborted, error_word, 3)) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 #pragma unroll 1
             for (int m = 0; m < SLABS; ++m) {

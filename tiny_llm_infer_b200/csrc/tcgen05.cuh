@@ -37,6 +37,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
     }
     return false;
 }
+// The same by all lanes of a warp that goes on to instructions of the whole warp (tcgen05.ld, __syncwarp): its lanes go on or give
+// up together, also where one alone ran out or saw another warp's flag.  On giving up, the error word has the code and the
+// block's flag is set.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* aborted, int* error_word, int code) {
+    const bool ok = mbar_wait(bar, parity);
+    if (!ok) {
+        atomicExch(error_word, code);
+        *aborted = 1;
+    }
+    return __all_sync(0xffffffffu, ok && !*aborted);
+}
 
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
     asm volatile(
