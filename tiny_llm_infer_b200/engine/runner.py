@@ -82,9 +82,10 @@ class PreparedStep:
     upload: int                                   # int32 words of the host buffer to send
     late: List[Tuple[int, int]]
     ctx: Optional[StepContext] = None             # the general path's context
-    graph_key: Optional[tuple] = None             # (rows bucket, context bucket) of a step taken row by row;
-                                                  # a third, True, where rows may belong to one request
-    wanted: Optional[List[int]] = None            # rows wanted of such a step
+    graph_key: Optional[tuple] = None             # (rows bucket, context bucket) of a one-token step to replay, with
+                                                  # (wanted bucket) as a third of a short portion taken row by row
+    wanted: Optional[List[int]] = None            # rows wanted of a step taken row by row
+    first_of: Optional[tuple] = None              # the graph key of a short portion whose graph is yet to be captured
     bounded: bool = False                         # once run: it launched kernels with bounded waits
 
 
@@ -306,6 +307,9 @@ class ModelRunner:
             ops.feed_tokens(d, d[at:at + n_late], d[at + n_late:at + 2 * n_late], late_source[0])
         if prepared.graph_key is not None:
             logits = self._run_graph(prepared)
+        elif prepared.first_of is not None:
+            logits = self.model.forward(prepared.ctx, self.cache)[:len(prepared.wanted)]
+            self._rows_seen.add(prepared.first_of)
         else:
             signature = self._prompt_signature(prepared.ctx)
             if signature is None:
@@ -447,26 +451,34 @@ class ModelRunner:
 
     # ---- short portions row by row
     # A step of a few prompt tokens (a short question, the next turn of a chat, alone or beside decode rows)
-    # is launch-bound too: 16 tokens of a 28-layer Qwen3-0.6B-sized model take the host 3.8 ms to issue and the
+    # is launch-bound too: 16 tokens of a 28-layer Qwen3-0.6B-sized model take the host 3 ms to issue and the
     # GPU 0.8 to run.  Its rows are taken one by one, as decode rows are: all keys of the step are in the
-    # cache before a row attends, and a row sees those up to its own position.  The graph is captured when a
-    # (rows, context) bucket comes a second time; the first goes the general way, at its old price.
+    # cache before a row attends, and a row sees those up to its own position.  Whether a step is taken so follows
+    # from the step alone, never from what the runner has done before: the first of a (rows, context, wanted) bucket
+    # launches the bucket's kernels one by one, which is the warm-up of the graph that the second captures, and
+    # the bits are those of the replays.  (That one capture costs, once per bucket: 4.5 to 7 ms where the general way
+    # takes 3 to 4, at Qwen3-0.6B sizes; 1.7 to 2.3 where it takes 0.8 with four layers of Qwen3-8B sizes.)
+    # Decode graphs captured after six of these replay no slower (Qwen3-8B sizes, batch 8: 3.24 to 3.28 ms, without 3.25 to 3.29).
     # A row reads its keys by itself, so the line is drawn at rows * context.  Steps at Qwen3-0.6B sizes, row by row
-    # against the general way: 16 rows of a new request 1.22 against 4.5 ms, 128 rows 1.49 against 3.75; behind 800 keys
-    # 128 rows 2.69 against 3.77, 256 rows 4.63 against 4.17; behind 3500 keys 32 rows 2.70 against 4.14, 128 rows 6.5
-    # against 4.16.  Four layers of Qwen3-8B sizes: 128 rows 0.68 against 0.80, behind 800 keys the same, 32 rows behind
-    # 3500 keys 0.88 against 0.91, 64 rows 1.07 against 0.93.
+    # (replayed) against the general way, ms: 16 rows of a new request 1.04 against 3.0, 128 rows 1.57 against 3.8; behind
+    # 800 keys 128 rows 2.77 against 3.8, 256 rows 4.63 against 4.17; behind 3500 keys 32 rows 2.9 against 4.1, 128 rows 6.5
+    # against 4.16.  Four layers of Qwen3-8B sizes: 128 rows 0.68 against 0.81, behind 800 keys the same, 32 rows behind
+    # 3500 keys 0.85 against 0.88, 64 rows 1.07 against 0.93.
     ROWS_GRAPH_MAX = 128
     ROWS_GRAPH_KEYS = 128 * 1024
 
-    def _rows_key(self, rows: int, context: int) -> Tuple[int, int]:
+    def _rows_key(self, rows: int, context: int, wanted: int) -> Tuple[int, int, int]:
         bucket = 1
         while bucket < rows:
             bucket *= 2
         ctx_bucket = 256
         while ctx_bucket < context:
             ctx_bucket *= 2
-        return min(bucket, self.max_batch_tokens), ctx_bucket
+        want_bucket = min(wanted, 1)
+        while want_bucket < wanted:
+            want_bucket *= 2
+        bucket = min(bucket, self.max_batch_tokens)
+        return bucket, ctx_bucket, min(want_bucket, bucket)
 
     def _rows_graphable(self, entries: Sequence[StepEntry]) -> bool:
         rows = sum(len(e.tokens) for e in entries)
@@ -477,34 +489,33 @@ class ModelRunner:
                 and sum(len(e.want) for e in entries) <= rows):
             return False                              # refusals are worded by the general way
         context = max((self.cache.computed(e.request) if self.cache.has(e.request) else 0) + len(e.tokens) for e in entries)
-        key = self._rows_key(rows, context)
-        if key[0] * key[1] > self.ROWS_GRAPH_KEYS:
-            return False
-        if key not in self._rows_seen:
-            self._rows_seen.add(key)
-            return False
-        return True
+        bucket, ctx_bucket, _ = self._rows_key(rows, context, 0)
+        return bucket * ctx_bucket <= self.ROWS_GRAPH_KEYS
 
     def _prepare_rows_graph(self, entries: Sequence[StepEntry]) -> PreparedStep:
         prepared = self._prepare_general(entries)     # the general layout: ids | positions | slots | wanted rows | ...
         rows, wanted, host = prepared.ctx.tokens, int(prepared.ctx.want_rows.shape[0]), self._host.numpy()
-        key = self._rows_key(rows, prepared.ctx.max_context)
-        bucket = key[0]
+        key = self._rows_key(rows, prepared.ctx.max_context, wanted)
+        bucket, _, want_bucket = key
         flat = host[:3 * rows + wanted].copy()
         host[0:bucket] = -1
         host[bucket:2 * bucket] = 0
-        host[2 * bucket:4 * bucket] = -1
+        host[2 * bucket:3 * bucket + want_bucket] = -1
         for i in range(3):
             host[i * bucket:i * bucket + rows] = flat[i * rows:(i + 1) * rows]
         host[3 * bucket:3 * bucket + wanted] = flat[3 * rows:]
-        return PreparedStep(entries, prepared.commits, 4 * bucket, prepared.late, graph_key=key + (True,),
-                            wanted=list(range(wanted)))
+        step = PreparedStep(entries, prepared.commits, 3 * bucket + want_bucket, prepared.late, wanted=list(range(wanted)))
+        if key in self._rows_seen:
+            step.graph_key = key
+        else:
+            step.first_of, step.ctx = key, self._bucket_context(key)
+        return step
 
     def _run_graph(self, prepared: PreparedStep) -> torch.Tensor:
         key, wanted = prepared.graph_key, prepared.wanted
         rows = len(prepared.entries) if len(key) == 2 else len(wanted)
         if key not in self._graphs:
-            self._capture(key)
+            self._capture(key, warm=len(key) > 2)
         graph, kernels, tc_calls = self._graphs[key]
         graph.replay()
         ops.launches += kernels                      # the replay launches what the capture recorded
@@ -534,23 +545,30 @@ class ModelRunner:
                 graph.capture_end()
         torch.cuda.current_stream().wait_stream(side)
 
-    def _capture(self, key) -> None:
-        bucket, ctx_bucket = key[:2]                   # (and, of portions taken row by row, True)
+    def _bucket_context(self, key) -> StepContext:
+        """The context of a bucket's steps: their rows in the runner's fixed buffers, padded to the bucket."""
+        bucket, ctx_bucket = key[:2]
+        want_bucket = key[2] if len(key) > 2 else bucket
         d = self._dev
-        ctx = StepContext(
+        return StepContext(
             tokens=bucket, token_ids=d[0:bucket], positions=d[bucket:2 * bucket],
-            token_slot=d[2 * bucket:3 * bucket], want_rows=d[3 * bucket:4 * bucket], segments=[],
+            token_slot=d[2 * bucket:3 * bucket], want_rows=d[3 * bucket:3 * bucket + want_bucket], segments=[],
             seg_info=None, dec_rows=None, n_dec=bucket, pf_tiles=d[0:0].view(-1, 2), n_tiles=0,
             decode_only=True, max_context=ctx_bucket, max_segment=1, shared_rows=len(key) > 2)
-        # warm-up: sizes workspaces, loads kernels.  A mixer with a per-request state would apply this step to
-        # it twice (here and in the replay), so then the warm-up runs with every row marked as padding
-        slots = d[2 * bucket:3 * bucket]
-        saved = slots.clone() if self.cache.state else None
-        if saved is not None:
-            slots.fill_(-1)
-        self.model.forward(ctx, self.cache)
-        if saved is not None:
-            slots.copy_(saved)
+
+    def _capture(self, key, warm: bool = False) -> None:
+        """Capture a bucket's step; ``warm``: its kernels have run before (a short portion's first step)."""
+        ctx = self._bucket_context(key)
+        if not warm:
+            # sizes workspaces, loads kernels.  A mixer with a per-request state would apply this step to
+            # it twice (here and in the replay), so then the warm-up runs with every row marked as padding
+            slots = ctx.token_slot
+            saved = slots.clone() if self.cache.state else None
+            if saved is not None:
+                slots.fill_(-1)
+            self.model.forward(ctx, self.cache)
+            if saved is not None:
+                slots.copy_(saved)
         torch.cuda.current_stream().synchronize()
         if self._graph_pool is None:
             self._graph_pool = torch.cuda.graph_pool_handle()
@@ -562,6 +580,6 @@ class ModelRunner:
         with self._capturing(graph, self._graph_pool):
             # the result goes to a buffer of the runner's own, so that the graphs' private
             # memory can be shared between them
-            self._graph_logits[:bucket].copy_(self.model.forward(ctx, self.cache))
+            self._graph_logits[:ctx.want_rows.shape[0]].copy_(self.model.forward(ctx, self.cache))
         self._graphs[key] = (graph, ops.launches - launches, ops.tcgen05_calls - tc_calls)
         ops.launches, ops.tcgen05_calls = launches, tc_calls  # capturing launches nothing
