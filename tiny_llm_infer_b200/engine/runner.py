@@ -464,8 +464,13 @@ class ModelRunner:
     # 800 keys 128 rows 2.77 against 3.8, 256 rows 4.63 against 4.17; behind 3500 keys 32 rows 2.9 against 4.1, 128 rows 6.5
     # against 4.16.  Four layers of Qwen3-8B sizes: 128 rows 0.68 against 0.81, behind 800 keys the same, 32 rows behind
     # 3500 keys 0.85 against 0.88, 64 rows 1.07 against 0.93.
+    # In float32 a portion's tiles share the keys that rows taken one by one read each for itself with the general
+    # kernel, so the line is nearer (ROWS_GRAPH_F32_CONTEXT).  Qwen3-0.6B sizes: 128 rows of a new request 3.45 against 4.68 ms,
+    # 8 rows 3.24 against 4.22, 128 rows behind 300 keys 6.97 against 6.08, behind 800 12.9 against 8.97, 3 rows behind 900
+    # 9.38 against 8.39, 8 rows behind 3500 26.4 against 23.7; 64 rows and fewer behind 300 to 450 gain or lose 4 to 8%.
     ROWS_GRAPH_MAX = 128
     ROWS_GRAPH_KEYS = 128 * 1024
+    ROWS_GRAPH_F32_CONTEXT = 256
 
     def _rows_key(self, rows: int, context: int, wanted: int) -> Tuple[int, int, int]:
         bucket = 1
@@ -490,6 +495,8 @@ class ModelRunner:
             return False                              # refusals are worded by the general way
         context = max((self.cache.computed(e.request) if self.cache.has(e.request) else 0) + len(e.tokens) for e in entries)
         bucket, ctx_bucket, _ = self._rows_key(rows, context, 0)
+        if self.model.dtype == torch.float32 and ctx_bucket > self.ROWS_GRAPH_F32_CONTEXT:
+            return False
         return bucket * ctx_bucket <= self.ROWS_GRAPH_KEYS
 
     def _prepare_rows_graph(self, entries: Sequence[StepEntry]) -> PreparedStep:
