@@ -554,21 +554,29 @@ def uniform_of(seed: int, token: int) -> float:
 
 
 SKINNY_MAX_ROWS = 8       # up to this many rows the weight-streaming product beats the library
-SKINNY_WIDE_ROWS = 16     # and up to this many where few blocks share the weight: see skinny_pays
+SKINNY_WIDE_ROWS = 16     # and up to this many with few blocks or short sums: see skinny_pays
 
 
 def skinny_pays(x: torch.Tensor, weight: torch.Tensor, gated: bool = False) -> bool:
     """Whether a bfloat16 product goes to the weight-streaming kernel, which gives 16 weight rows to a block.
-    Beyond eight rows of x a block holds two row tiles and its registers leave two blocks per SM: one round
-    of those is ahead of the library's kernel (16 rows, Qwen3-0.6B sizes: q/k/v 3.9 us against 4.3, output 5.0 against 6.9,
-    down 6.1 against 8.8), more are not (8B sizes: q/k/v 16.9 against 12.2, gate/up 48 against 36); a gated product also
-    saves the activation's kernel, which pays for half a round more (6.4 against 8.6; 8B sizes 49 against 41)."""
+    Beyond eight rows of x a block holds two row tiles and its registers leave two blocks per SM, so it is ahead of the library
+    only where a block's sums are short or half the SMs are enough for all blocks.  16 rows, weights from HBM, this kernel and the
+    library's, us: columns x K 4096 x 1024 3.8 and 4.3, 4736 x 1536 4.9 and 5.2, 1024 x 2048 4.9 and 6.4, 1024 x 3072 6.1 and 8.3,
+    1184 x 4096 6.8 and 7.5; but 2560 x 2048 5.4 and 5.2, 4096 x 12288 21.6 and 20.9, 2560 x 9728 17.2 and 14.7, 1184 x 8192 12.7
+    and 12.2.  A gated product also saves the activation's kernel: two blocks per SM and K up to 8192 pay (inter x K 2368 x 4096 10.0
+    and 12.3, 2048 x 8192 16.9 and 17.3), three only with short sums (3072 x 1024 6.3 and 7.7, 3552 x 1536 8.3 and 9.0, 2560 x 1664
+    9.1 and 8.6, 3552 x 2560 12.5 and 11.4)."""
     rows, k = x.shape
     if not 0 < rows <= SKINNY_WIDE_ROWS or k % 8 or not x.is_contiguous() or not weight.is_contiguous():
         return False
+    if rows <= SKINNY_MAX_ROWS:
+        return True
     blocks = -(-weight.shape[0] // 16)
-    return rows <= SKINNY_MAX_ROWS or (blocks <= SM_COUNT * (3 if gated else 2)
-                                           and (x.data_ptr() | weight.data_ptr()) % 16 == 0)
+    if gated:
+        fast = blocks <= 3 * SM_COUNT and k <= 1536 or blocks <= 2 * SM_COUNT and k <= 8192
+    else:
+        fast = blocks <= 2 * SM_COUNT and k <= 1536 or blocks <= SM_COUNT // 2 and k <= 4096
+    return fast and (x.data_ptr() | weight.data_ptr()) % 16 == 0
 
 
 def gemm_skinny(x: torch.Tensor, weight: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
