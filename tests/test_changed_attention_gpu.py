@@ -119,3 +119,36 @@ def test_odd_values_reach_only_the_rows_that_see_them(form, heads, kv_heads, len
     got, want = out[0][finite], out[1][finite]
     assert (got - want).abs().max().item() <= 3 * 2.0 ** -8 * largest          # as above
     assert ((got - want).norm() / want.norm()).item() <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+@pytest.mark.parametrize("heads,kv_heads,lengths,befores", [(4, 2, (130, 2, 257), (0, 333, 61)), (3, 3, (301,), (17,)), (2, 1, (65,), (1500,))])
+def test_what_lies_behind_the_last_token_changes_no_bit(form, heads, kv_heads, lengths, befores):
+    """Keys and values that another request left in the last page, small beside the cap or far beyond it."""
+    from tiny_llm_infer_b200 import ops
+    f = dict(FORMS[form])
+    g = torch.Generator(device=DEV).manual_seed(8)
+
+    def randn(*shape):
+        return torch.randn(*shape, generator=g, device=DEV)
+    ctx = context(lengths, befores)
+    pages = -(-ctx.max_context // PAGE)
+    order = torch.randperm(len(lengths) * pages, generator=g, device=DEV).to(torch.int32).view(len(lengths), pages)
+    keys, values = (randn(len(lengths) * pages, kv_heads, PAGE, D).bfloat16() for _ in range(2))
+    q = (randn(ctx.tokens, heads * D) * 0.3).bfloat16()            # scores on either side of 0.4 of the cap of 2, within it of 9
+    per_head = f.get("gate") == "heads"
+    gate = randn(ctx.tokens, heads if per_head else heads * D).bfloat16() if f.get("gate") else None
+    kw = dict(softcap=f.get("softcap", 0.0), chunk=f.get("chunk", 0), window=f.get("window", 0), sink=f.get("sink", False),
+              slopes=torch.rand(heads, generator=g, device=DEV) * 0.05 if f.get("slopes") else None, gate=gate,
+              gate_per_head=per_head, sink_logits=randn(heads) if f.get("learned") else None)
+    out = []
+    for left in (0.0, 1.0, 100.0):
+        for s, (n, p0) in enumerate(zip(lengths, befores)):
+            for pos in range(p0 + n, -(-(p0 + n) // PAGE) * PAGE):
+                for plane in (keys, values):
+                    plane[order[s, pos // PAGE].long(), :, pos % PAGE] = (randn(kv_heads, D) * left).bfloat16()
+        o = torch.empty_like(q)
+        ops.attention_biased(q, keys, values, ctx.positions, ctx.token_slot, order, PAGE, heads, kv_heads, D, D, D ** -0.5, o, ctx=ctx, **kw)
+        out.append(o)
+    ops.check_error_word(q.device)
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])

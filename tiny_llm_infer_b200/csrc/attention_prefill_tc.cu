@@ -204,26 +204,6 @@ __device__ __forceinline__ float rcp(float x) {
     asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
     return y;
 }
-// cap tanh(s / cap) times log2(e) for scores with |y| = |s| / cap <= kTanhSeries by the Taylor series of tanh to y^11 on the
-// fused multiply-add pipe, two scores per instruction: within 6e-8 of the value there (the next term, 0.0036 y^12 of it), where
-// 1 - 2 / (e^2y + 1) is some 1e-7 of the cap off.  per_score: y of a score of one; cap_out: the cap times log2(e).
-constexpr float kHalfLn2 = 0.34657359027997264f, kTanhSeries = 0.4f;
-__device__ __forceinline__ void cap_by_series(uint32_t (&sv)[kBN], float per_score, float cap_out) {
-    const float2 to_y = make_float2(per_score, per_score), to_out = make_float2(per_score * cap_out, per_score * cap_out);
-    const float c[5] = {-1.0f / 3.0f, 2.0f / 15.0f, -17.0f / 315.0f, 62.0f / 2835.0f, -1382.0f / 155925.0f};
-#pragma unroll
-    for (int i = 0; i < kBN; i += 2) {
-        const float2 v = make_float2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
-        const float2 y = __fmul2_rn(v, to_y), z = __fmul2_rn(y, y);
-        float2 p = make_float2(c[4], c[4]);
-#pragma unroll
-        for (int k = 3; k >= 0; --k) p = __ffma2_rn(p, z, make_float2(c[k], c[k]));
-        p = __ffma2_rn(p, z, make_float2(1.0f, 1.0f));
-        const float2 out = __fmul2_rn(__fmul2_rn(v, to_out), p);
-        sv[i] = __float_as_uint(out.x);
-        sv[i + 1] = __float_as_uint(out.y);
-    }
-}
 __device__ __forceinline__ float sigmoid_of(bf16 g) { return 1.0f / (1.0f + expf(-__bfloat162float(g))); }
 
 __device__ __forceinline__ float4 four_of(const bf16* p) {      // on an 8-byte boundary
@@ -310,9 +290,7 @@ __device__ __noinline__ bool odd_row(const OddRow& a, float4& o, float& m, float
 // kChanged: the changes above, but no table.  A capped score costs two exponential-unit instructions more (e^2x and the
 // reciprocal of tanh x = 1 - 2 / (e^2x + 1)); with them that unit sets the pace: 3 x 128 x 128 instructions on 16 a cycle are
 // 3070 cycles per pair of query tiles and 64 keys, where the plain form takes 1950.  One prompt of 2048 tokens, 32 heads
-// on 8, cap, window, learned sink and a gate per head: 85.5 us (363 on the mma.sync tiles of attention_biased.cu).  Tiles whose
-// scores all stay within 0.4 of the cap take tanh's series on the multiply-add pipe instead (a warp of rows decides): the same
-// prompt 82 us against 88 on one day; the chain of a tile's softmax, not that unit alone, bounds it now.
+// on 8, cap, window, learned sink and a gate per head: 85.5 us (363 on the mma.sync tiles of attention_biased.cu).
 template <int kForm>
 __global__ void __launch_bounds__(kThreads, 1)
 paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const bf16* __restrict__ k_base,
@@ -638,14 +616,7 @@ paged_attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, con
                 }
             }
             if constexpr (kChange) {
-                float largest = 0.0f;
                 if (ch.cap_in > 0.0f) {
-#pragma unroll
-                    for (int i = 0; i < kBN; ++i) largest = fmaxf(largest, fabsf(__uint_as_float(sv[i])));
-                }
-                if (ch.cap_in > 0.0f && __all_sync(0xffffffffu, largest * (ch.cap_in * kHalfLn2) <= kTanhSeries)) {
-                    cap_by_series(sv, ch.cap_in * kHalfLn2, ch.cap_out);
-                } else if (ch.cap_in > 0.0f) {
                     // e overflows to infinity (tanh 1) and underflows to zero (tanh -1) where it should
 #pragma unroll
                     for (int i = 0; i < kBN; ++i)
