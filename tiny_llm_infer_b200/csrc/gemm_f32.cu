@@ -10,6 +10,8 @@
 // Warps 0 to 7 fetch both operands as float32 (each thread eight pieces of eight numbers, the next slab's loads on their way
 // while the present one is split), split them and write the six bfloat16 slabs of 128 x 64 in the 128-byte swizzle; one thread of
 // warp 16 issues 24 MMAs (128 x 128 x 16) per slab of 64; warps 8 to 15 add the accumulators up, two sets of which take turns.
+// Sums that are no finite numbers are made again at the end from the operands as they are, so that infinities, overflows and numbers
+// that bfloat16 cannot hold come out as a float32 product has them.  Below some 2^-110 an operand's last part loses bits.
 // No scratch and no second copy of a weight exists.  Work for few tiles is cut over K, the shares' sums added in their order by a
 // second kernel.
 //
@@ -25,6 +27,7 @@ namespace tllm {
 
 constexpr int kFTile = 128, kFK = 64, kFStages = 2, kFPart = kFTile * kFK * 2, kFStage = 6 * kFPart;
 constexpr int kFSplitters = 256, kFAdders = 256, kFThreads = kFSplitters + kFAdders + 32;
+constexpr float kFLargest = 3.402823466e38f; // the largest finite number
 constexpr int kFTogether = 2;                // slabs whose products meet in one pair of accumulators (128 terms)
 
 __global__ void __launch_bounds__(kFThreads, 1)
@@ -33,7 +36,7 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[kFStages], empty_bar[kFStages], acc_full[2], acc_empty[2], drained;
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, odd_flag;
     unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int all_slabs = (K + kFK - 1) / kFK, units = tiles * splits;
@@ -47,7 +50,7 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
             mbar_init(&acc_empty[b], kFAdders / 32);
         }
         mbar_init(&drained, 1);
-        abort_flag = 0;
+        abort_flag = odd_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 16) {
@@ -152,7 +155,7 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
         // ------------------------------------------------------------ add the accumulators up (a row and 64 columns per thread)
         const int quad = warp & 3, half = (warp >> 2) & 1;
         int group = 0;
-        bool alive = true;
+        bool alive = true, odd = false;
         for (int u = blockIdx.x; u < units; u += gridDim.x) {
             const int slabs = slabs_of(u);
             float sum[64];
@@ -181,14 +184,41 @@ gemm_f32_tcgen05_kernel(const float* __restrict__ x, const float* __restrict__ w
             const int tile = u % tiles, row = tile % tiles_m * kFTile + quad * 32 + lane, col0 = tile / tiles_m * kFTile + half * 64;
             if (row < M) {
                 float* dst = y + ((size_t)(u / tiles) * M + row) * N + col0;
+                float largest = 0.0f;                // NaN where any sum is an infinity or no number
+#pragma unroll
+                for (int i = 0; i < 64; ++i) largest = fmaf(sum[i], 0.0f, largest);
+                odd |= largest != largest;
 #pragma unroll
                 for (int i = 0; i < 64; i += 4)
                     if (col0 + i < N) *reinterpret_cast<float4*>(dst + i) = make_float4(sum[i], sum[i + 1], sum[i + 2], sum[i + 3]);
             }
         }
+        if (odd) odd_flag = 1;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
+    if (odd_flag && !abort_flag) {
+        // A sum that is no finite number is made again from the float32 operands, a thread each, over its share of K in order: an
+        // infinity's second part is no number and its product with a part of zero neither, and a number beyond the largest
+        // bfloat16 goes in as an infinity.  Given up once it is no number, which it then stays.
+        for (int u = blockIdx.x; u < units; u += gridDim.x) {
+            const int tile = u % tiles, m0 = tile % tiles_m * kFTile, n0 = tile / tiles_m * kFTile;
+            const int k0 = u / tiles * slabs_each * kFK, k1 = min(K, k0 + slabs_of(u) * kFK);
+            for (int i = threadIdx.x; i < kFTile * kFTile; i += kFThreads) {
+                const int row = m0 + i / kFTile, col = n0 + i % kFTile;
+                if (row >= M || col >= N) continue;
+                float* at = y + ((size_t)(u / tiles) * M + row) * N + col;
+                if (fabsf(*at) <= kFLargest) continue;
+                float sum = 0.0f;
+                for (int k = k0; k < k1 && sum == sum; k += 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(x + (size_t)row * K + k);
+                    const float4 b = *reinterpret_cast<const float4*>(w + (size_t)col * K + k);
+                    sum = fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, sum))));
+                }
+                *at = sum;
+            }
+        }
+    }
     if (warp == 16) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
 }
 
