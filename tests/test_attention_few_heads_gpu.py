@@ -1,13 +1,14 @@
-"""One-token rows with at most eight query heads per key/value head (the keys as the MMA's left operand) against 64 bits: first
-and last keys of tiles and of runs of keys, pages that are no power of two, every change of the score, places of the pages that
-nobody has written."""
+"""One-token rows with at most eight query heads per block (the keys as the MMA's left operand; 24 heads on one go twelve to a block,
+as the left operand themselves) against 64 bits: first and last keys of tiles and of runs of keys, pages that are no power of two,
+every change of the score, places of the pages that nobody has written."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("heads,kv_heads,dim,page", [(8, 8, 128, 16), (32, 8, 128, 16), (16, 2, 64, 48), (12, 4, 64, 32), (24, 1, 128, 16)])
+@pytest.mark.parametrize("heads,kv_heads,dim,page", [(8, 8, 128, 16), (32, 8, 128, 16), (16, 2, 64, 48), (12, 4, 64, 32), (24, 1, 128, 16),
+                                                        (21, 1, 128, 16), (50, 2, 64, 48)])       # three blocks of seven heads, five of five, per key/value head
 @pytest.mark.parametrize("change", ["none", "cap window sink gate", "slopes chunk", "bias learned"])
 @pytest.mark.parametrize("crowd", [0, 40])
 def test_one_token_rows(heads, kv_heads, dim, page, change, crowd):

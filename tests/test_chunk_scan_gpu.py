@@ -23,7 +23,9 @@ def unpack(flat, heads, dk, dv):
 
 
 @pytest.mark.parametrize("mode", ["delta", "channel", "channel, no weights", "head", "fixed"])
-@pytest.mark.parametrize("heads,kv_heads,dk,dv", [(4, 2, 128, 128), (3, 3, 64, 48), (8, 8, 128, 16), (40, 40, 64, 64)])
+# blocks of 16 columns, and of 32 (from 111 blocks of these on): of one decay per head in the form of one block per SM up to 148 of
+# them (one portion of 32 x 128 or 64 x 64 columns), of two beyond
+@pytest.mark.parametrize("heads,kv_heads,dk,dv", [(4, 2, 128, 128), (3, 3, 64, 48), (8, 8, 128, 16), (40, 40, 64, 64), (32, 8, 128, 128), (64, 16, 64, 64)])
 @pytest.mark.parametrize("lengths", [(1, 15, 16, 17, 33), (200,), (64, 0, 31, 47)])
 def test_chunks_are_the_recurrence(mode, heads, kv_heads, dk, dv, lengths, monkeypatch):
     from tiny_llm_infer_b200 import ops
@@ -110,7 +112,8 @@ def test_chunks_are_the_recurrence(mode, heads, kv_heads, dk, dv, lengths, monke
 @pytest.mark.parametrize("by_chunks", [True, False])
 @pytest.mark.parametrize("mode,operands", [("delta", "q k v decay beta"), ("channel", "q k v decay beta"), ("channel, no weights", "q k v decay"),
                                            ("head", "q k v beta fgate"), ("fixed", "q k v")])
-@pytest.mark.parametrize("heads,kv_heads,dk,dv", [(4, 2, 128, 128), (40, 40, 64, 64)])      # two columns per lane and four
+# blocks of 16 columns; of 32, more than 148 of them, at both widths of keys; of 32, at most 148
+@pytest.mark.parametrize("heads,kv_heads,dk,dv", [(4, 2, 128, 128), (40, 40, 64, 64), (32, 8, 128, 128), (12, 4, 128, 128), (24, 8, 64, 64)])
 @pytest.mark.parametrize("odd", [float("nan"), float("inf")])
 def test_an_odd_token_reaches_no_read_out_before_it(by_chunks, mode, operands, heads, kv_heads, dk, dv, odd, monkeypatch):
     """One token of every portion has an infinity or a NaN in one operand; what is read out before it stays bit for bit."""

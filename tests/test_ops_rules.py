@@ -83,3 +83,32 @@ def test_products_of_few_rows_want_whole_rows_on_16_bytes():
         assert ops.skinny_pays(base[off:off + rows * 64].view(rows, 64), w) == pays
     assert not ops.skinny_pays(torch.empty(64, 16, dtype=torch.bfloat16).t(), w)
     assert not ops.skinny_pays(torch.empty(16, 64, dtype=torch.bfloat16), torch.empty(64, 64, dtype=torch.bfloat16).t())
+
+
+@pytest.mark.parametrize("rows,columns,k,pays", [
+    (64, 8192, 1024, True), (64, 8188, 1024, False), (512, 1024, 1024, True), (595, 4096, 1024, True), (63, 16384, 1024, False),
+    (64, 2048, 1028, True), (64, 2036, 1028, False), (128, 832, 1280, True), (64, 1408, 1536, True), (64, 1024, 2048, True),
+    (64, 1020, 2048, False), (595, 1024, 2048, True), (595, 96, 64, False), (64, 4096, 4098, False), (64, 4098, 4096, False), (9, 8192, 8192, False),
+])
+def test_large_float32_products_run_on_the_tensor_cores(rows, columns, k, pays):
+    assert ops.f32_tcgen05_pays(torch.empty(rows, k), torch.empty(columns, k)) == pays
+
+
+def test_float32_operands_off_the_grid_stay_with_the_library():
+    w = torch.empty(2048, 2048)
+    base = torch.empty(64 * 2048 + 4)
+    for off, pays in ((0, True), (4, True), (1, False), (2, False)):
+        assert ops.f32_tcgen05_pays(base[off:off + 64 * 2048].view(64, 2048), w) == pays
+    x = torch.empty(64, 2048)
+    assert not ops.f32_tcgen05_pays(torch.empty(2048, 64).t(), w) and not ops.f32_tcgen05_pays(x, torch.empty(2048, 4096)[:, ::2])
+    assert not ops.f32_tcgen05_pays(x, torch.empty(2048, 2048, requires_grad=True))
+
+
+def test_shares_of_float32_sums_fill_the_gpu():
+    assert ops.f32_splits(595, 4096, 1024) == 2 and ops.f32_splits(2048, 24576, 4096) == 1        # 160 tiles; far more than SMs
+    assert ops.f32_splits(595, 1024, 2048) == 3 and ops.f32_splits(64, 1024, 2048) > 3 and ops.f32_splits(64, 4, 64) == 1
+    for rows in (64, 300, 595, 2048):
+        for columns in (96, 1024, 4096):
+            for k in (64, 1028, 4096, 12288):
+                s, slabs, tiles = ops.f32_splits(rows, columns, k), -(-k // 64), -(-rows // 128) * -(-columns // 128)
+                assert 1 <= s <= min(slabs, 16) and (s == 1 or -(-tiles * s // ops.SM_COUNT) * -(-slabs // s) < -(-tiles // ops.SM_COUNT) * slabs)
