@@ -152,3 +152,26 @@ def test_what_lies_behind_the_last_token_changes_no_bit(form, heads, kv_heads, l
         out.append(o)
     ops.check_error_word(q.device)
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+
+
+def test_maxima_and_sums_of_runs_may_lie_on_any_float():
+    """The library's entry wants 16-byte boundaries of the partial results, not of their maxima and sums."""
+    from tiny_llm_infer_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(9)
+    heads, kv_heads, ctx = 2, 1, context((65,), (1500,))
+    pages, splits = -(-ctx.max_context // PAGE), 4
+    table = torch.randperm(pages, generator=g, device=DEV).to(torch.int32).view(1, pages)
+    cache = torch.randn(pages, 2, kv_heads, PAGE, D, generator=g, device=DEV).bfloat16()
+    q = torch.randn(ctx.tokens, heads * D, generator=g, device=DEV).bfloat16()
+    part_o = torch.empty(ctx.tokens * heads * splits * D, device=DEV)
+    room, out = torch.empty(ctx.tokens * heads * splits * 2 + 1, device=DEV), []
+    for off in (0, 1):
+        part_ml, o = room[off:], torch.empty_like(q)
+        rc = ops.lib().tllm_paged_attention_prefill_tc(
+            q.data_ptr(), ctx.tokens, cache.data_ptr(), pages, ctx.seg_info.data_ptr(), ctx.pf_tiles.data_ptr(), ctx.n_tiles128,
+            table.data_ptr(), pages, PAGE, heads, kv_heads, D, 0, D ** -0.5, o.data_ptr(), splits, part_o.data_ptr(), part_ml.data_ptr(),
+            ops.error_word(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        out.append(o)
+    ops.check_error_word(q.device)
+    assert torch.equal(out[0], out[1]) and torch.isfinite(out[0]).all()

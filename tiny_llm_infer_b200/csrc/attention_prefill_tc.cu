@@ -847,7 +847,8 @@ paged_attention_prefill_combine_kernel(const float* part_o, const float* part_ml
 #pragma unroll
         for (int z = 0; z < kMaxRuns; ++z) {
             const bool in = z0 + z < splits;
-            ml[z] = in ? *reinterpret_cast<const float2*>(part_ml + (base + z0 + z) * 2) : make_float2(-INFINITY, 0.0f);
+            const float* pair = part_ml + (base + z0 + z) * 2;           // on any float: only part_o has to lie on 16 bytes
+            ml[z] = in ? make_float2(pair[0], pair[1]) : make_float2(-INFINITY, 0.0f);
             o[z] = in ? *reinterpret_cast<const float4*>(part_o + (base + z0 + z) * kHD + lane * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     };
