@@ -66,3 +66,13 @@ def test_generation_stops_at_the_step_that_failed(tmp_path, monkeypatch, overlap
     with pytest.raises(ops.KernelError, match="code 5"):
         generate(failing)
     ops.check_error_word(torch.device(DEV))                        # read and cleared
+
+
+def test_a_device_without_an_index_has_the_word_its_tensors_report_to():
+    from tiny_llm_infer_b200 import ops
+    x = torch.zeros(1, device="cuda")
+    ops.error_word(x.device).fill_(9)
+    with pytest.raises(ops.KernelError, match="code 9"):
+        ops.check_error_word("cuda")
+    ops.check_error_word(torch.device("cuda"))
+    ops.check_error_word(x.device)

@@ -612,6 +612,8 @@ def error_word(device) -> torch.Tensor:
     """Device int32 that kernels with bounded waits (the tcgen05 product) set to a non-zero
     code when a wait ran out.  ``check_error_word`` reads it (a synchronisation)."""
     key = str(device)
+    if key == "cuda":                        # without an index: the word of the current device, as its tensors name it
+        key = f"cuda:{torch.cuda.current_device()}"
     if key not in _error_words:
         _error_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return _error_words[key]
