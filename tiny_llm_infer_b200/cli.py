@@ -53,7 +53,7 @@ def build_parser() -> argparse.ArgumentParser:
     ap.add_argument("--no-prefix-caching", action="store_true",
                     help="compute every prompt in full (the reference always shares hashed pages)")
     ap.add_argument("--prompt-graphs", action="store_true",
-                    help="replay prompt steps whose layout repeats as CUDA graphs too")
+                    help="replay prompt steps of any size whose layout repeats as CUDA graphs too (short ones always are)")
     ap.add_argument("--no-overlap-scheduling", action="store_true",
                     help="schedule a step only after the one before it has finished on the GPU")
     ap.add_argument("--num-seqs", type=int, default=8)

@@ -290,8 +290,10 @@ class LLM:
     full pages; it stays off by itself for models with windows or per-request state.
     ``overlap_scheduling`` (on): the host schedules and lays out a step while the GPU runs
     the one before it; the tokens are the same either way.  ``use_cuda_graphs`` (on): steps of
-    one-token rows are replayed as CUDA graphs; ``prompt_graphs`` (off): steps with prompt
-    portions whose layout repeats too (faster prompts, slightly slower decoding afterwards).
+    one-token rows are replayed as CUDA graphs, and so are short steps with prompt portions of models
+    whose rows only the cache joins (``ModelRunner.ROWS_GRAPH_MAX``), whose rows then go through the
+    kernels of one-token rows: their logits differ from those without graphs in rounding.  ``prompt_graphs``
+    (off): larger steps with prompt portions whose layout repeats too (faster prompts, slightly slower decoding afterwards).
     """
 
     def __init__(self, model: str, dtype: str = "bfloat16", max_model_len: int = 2048,

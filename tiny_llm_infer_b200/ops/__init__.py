@@ -4,13 +4,14 @@ other implementation: if the kernel library cannot be built or loaded, the first
 raises ``KernelLibraryError``.
 
 The matrix product (``linear``, ``linear_swiglu``) has two kernels of this package for
-bfloat16, chosen by the number of rows: up to 8 the weight-streaming mma.sync product
-(``gemm_skinny``), from 256 on, where the tiles fill the GPU, the TMA + tcgen05 product
+bfloat16, chosen by the number of rows: up to 8, and up to 16 with short sums or few columns
+(``skinny_pays``), the weight-streaming mma.sync product (``gemm_skinny``), from 256 on, where the tiles fill the GPU, the TMA + tcgen05 product
 (``gemm_tcgen05``).  Everything else is the library's (cuBLAS through ``torch.mm``), as in the reference, which calls
 ``cublasHgemm`` for every projection with more than one row
 (kernels/src/matmul_kernel_cuda.cu:83-91); in float32 mode it runs with the
-reduced-precision matrix modes switched off, and large products run on the tensor cores with every operand in three
-bfloat16 parts (``gemm_f32_tcgen05``), closer to 64 bits than the library's.
+reduced-precision matrix modes switched off, and large products (64 rows or more, ``f32_tcgen05_pays``) run on the tensor cores with
+every operand in three bfloat16 parts (``gemm_f32_tcgen05``), closer to 64 bits than the library's.  So the last bits of a row depend
+on how many rows share its product, in float32 too (there from 64 rows on, where the shares of K follow the rows).
 """
 from __future__ import annotations
 
@@ -680,7 +681,10 @@ def f32_tcgen05_pays(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether a float32 product runs on the tensor cores rather than in the library: enough work for their start, and operands in
     16-byte pieces.  The library's kernel and this one, rows x columns x K: 64 x 1024 x 2048 37 and 28 us, 64 x 4096 x 4096 78 and
     38, 128 x 4096 x 1024 32 and 30 (64 rows 23 and 28), 595 x 4096 x 1024 123 and 62, 595 x 1024 x 2048 87 and 33,
-    2048 x 24576 x 4096 6955 and 2223; 595 x 96 x 64 11 and 12.  (With fewer rows it is ahead only from K = 3072 on.)"""
+    2048 x 24576 x 4096 6955 and 2223; 595 x 96 x 64 11 and 12.  (With fewer rows it is ahead only from K = 3072 on.)  At the lines,
+    weights from HBM and the kernels back to back: 64 x 8192 x 1024 33 and 23, 512 x 1024 x 1024 30 and 17, 64 x 2048 x 1028 26 and 12,
+    128 x 832 x 1280 30 and 14, 64 x 1408 x 1536 37 and 14.  (Back to back, weights in L2, it is ahead below the
+    lines too: 64 x 1024 x 1024 19 and 10.)"""
     rows, k = x.shape
     n = weight.shape[0]
     return (rows >= 64 and rows * n * k >= (1 << 29 if k <= 1024 else 1 << 27) and k % 4 == 0 and n % 4 == 0
@@ -792,7 +796,10 @@ def biased_decode_splits(rows: int, kv_heads: int, reach: int) -> int:
     rows, 1 to 8 key/value heads, 260 to 8000 keys: a tenth less time on average where all rows are as long, 7% where the
     shortest has half the keys; of these 8 rows of 8 heads at 2000 keys 40 us, now 34, 16 at 4000 105 and 87, 40 at 4000 201 and 170,
     64 at 2000 139 both.  Ten of the uneven steps take 3 to 15% longer, most of them with one key/value head; with whole rounds
-    and three tiles for the adding kernel eighteen did: 80 rows of 2 heads at 1000 44 us, 40 with two runs or three.)"""
+    and three tiles for the adding kernel eighteen did: 80 rows of 2 heads at 1000 44 us, 40 with two runs or three.  These are
+    figures of the kernel with the heads as rows, two blocks per multiprocessor.  Steps of at most eight heads per block run three
+    and gain at every point, but not always the most with these runs, this rule's and the best: 8 rows of 8 heads at 2000 27.6 us both,
+    16 at 4000 66.6 both, 40 at 4000 136 and 126 (four), 64 at 2000 124 and 110 (four), 80 of 2 at 1000 36 and 29 (one).)"""
     tiles, resident = -(-reach // 64), 2 * SM_COUNT
     best, least = 1, None
     for splits in range(1, max(1, min(reach // 192, 64)) + 1):
@@ -1110,8 +1117,9 @@ CHUNK_MODES = (SCAN_DELTA, SCAN_PLAIN, SCAN_HEAD_DECAY, SCAN_FIXED_DECAY)      #
 # are two kernels and less work.  The delta rule with 32 heads of 128 x 128, token by token and by chunks: one portion of 64
 # tokens 27 and 32 us, of 256 80 and 65; eight of 48 tokens 82 and 77, of 64 104 and 91.  Between the lines both take some 40 us,
 # and the second launch costs more than it saves (four portions of 90 tokens, 16 heads of 64 x 128: 29 and 30 us, of the whole
-# op 40 and 48).  The chunks' figures are those of their float32-pipe kernels; on the tensor cores portions of 2048 tokens take three
-# quarters of the time, one portion of 100 tokens as long (37.7 us against 36.9), so the lines stay.
+# op 40 and 48).  The chunks' figures are those of kernels on the float32 pipe; the present ones, on the tensor cores, are faster, so
+# nothing that goes by chunks is slower by them (32 points on that side of the lines, 8 to 69% less time), but some portions on the
+# other side would be faster by chunks now: the delta rule, one portion of 100 tokens 37 and 32 us (eight of 48 not: 80 and 83).
 CHUNK_TOKENS = 64
 
 
@@ -1124,7 +1132,10 @@ def chunks_pay(mode: int, segments: int, tokens: int, heads: int, dk: int, cols:
     of 64 x 16 82 and 112 us, of 64 x 48 (32 heads) 100 and 112, of 64 x 64 101 and 110; of 128 x 16 129 and 147; one decay
     per head, twelve of 64 heads of 64 x 16 96 and 114.  The delta rule's chunks do twice the work of the others', so with keys of
     64 elements they win only while the columns of a step are few: 16 heads of 64 x 128 529 and 169 us for 2048 tokens, three
-    portions of 32 heads up to a fifth faster, four 111 and 126, twelve of 64 heads of 64 x 64 310 and 341."""
+    portions of 32 heads up to a fifth faster, four 111 and 126, twelve of 64 heads of 64 x 64 310 and 341.  (On the float32 pipe;
+    on the tensor cores these lines lie further out: four portions of 32 heads 110 and 95, eight of 32 heads of 64 x 64 with decays
+    per channel 100 and 85, of one decay per head, twelve of 64 heads of 64 x 16, 96 and 87; of 64 x 16 with decays per channel 82 and
+    99, of 128 x 16 with the delta rule 112 and 126 as before.)"""
     if tokens < CHUNK_TOKENS * segments or not (2 * tokens >= 5 * CHUNK_TOKENS * segments or tokens * heads * dk >= CHUNK_TOKENS << 15):
         return False
     pairs = segments * heads * CHUNK_TOKENS / 64
