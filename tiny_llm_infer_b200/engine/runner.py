@@ -457,8 +457,8 @@ class ModelRunner:
     # from the step alone, never from what the runner has done before: the first of a (rows, context, wanted) bucket
     # launches the bucket's kernels one by one, which is the warm-up of the graph that the second captures, and
     # the bits are those of the replays.  (That one capture costs, once per bucket: 4.5 to 7 ms where the general way
-    # takes 3 to 4, at Qwen3-0.6B sizes; 1.7 to 2.3 where it takes 0.8 with four layers of Qwen3-8B sizes.  Sixty requests of 4 to 120 tokens one after the other, four
-    # tokens each, on a new runner: 0.28 s, 0.70 the general way.)
+    # takes 3 to 4, at Qwen3-0.6B sizes; 1.7 to 2.3 where it takes 0.8 with four layers of Qwen3-8B sizes.  Sixty
+    # requests of 4 to 120 tokens one after the other, four tokens each, on a new runner: 0.28 s, 0.70 the general way.)
     # Decode graphs captured after six of these replay no slower (Qwen3-8B sizes, batch 8: 3.24 to 3.28 ms, without 3.25 to 3.29).
     # A row reads its keys by itself, so the line is drawn at rows * context.  Steps at Qwen3-0.6B sizes, row by row
     # (replayed) against the general way, ms: 16 rows of a new request 1.04 against 3.0, 128 rows 1.57 against 3.8; behind
